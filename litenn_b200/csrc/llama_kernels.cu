@@ -762,70 +762,242 @@ __global__ void __launch_bounds__(256) resid_rmsnorm_rows_kernel(float* __restri
     }
 }
 
-// Causal attention over the fp16 cache for rows 0..m-1 at positions pos0+row.  The kernel is bound by the L2
-// reads of K and V (every row streams the whole prefix of its head), so one warp serves ROWS consecutive rows of
-// one head and reuses each loaded batch of eight keys for all of them; a row simply ignores the keys beyond its
-// own position.  Online softmax per row, one rescale per batch; output bf16 ctx[m][n_heads*hd].
-template <int DPL, int ROWS>
+// ---- prefill attention -------------------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p)
+{
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
+// D += A(16x16, fp16) * B(16x8, fp16), fp32 accumulate
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Two fp32 values as a sum of two fp16 pairs: hi + lo holds 22 bits of each.
+__device__ __forceinline__ void split_f16x2(float a, float b, uint32_t& hi, uint32_t& lo)
+{
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 hf = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - hf.x, b - hf.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// Causal attention over the fp16 cache for rows 0..m-1 at positions pos0+row, on the tensor cores.  A CTA owns 64
+// query rows of one head (16 per warp) and walks the keys in tiles of 64, which cp.async brings into shared memory one
+// tile ahead; online softmax per row, output bf16 ctx[m][n_heads*hd].
+// Queries and probabilities are fp32 and stay that precise: each goes through the fp16 MMA as hi + lo, two passes over
+// the same key or value fragment (K and V are fp16, so those are exact).  A power of two per row keeps the split away
+// from fp16's range limits: the row's largest query value is brought to 2^14..2^15, probabilities are taken times 2^14.
+// Masked keys get probability 0, but their V rows do take part in the product: a value that overflowed fp16 reaches the
+// earlier rows of its 64-row group too.  The prompt's last row and every later token see it in any case.
+// Bound: the MMA pipe (twice the flops of a one-pass product).  Four rows per warp with fp32 arithmetic and shuffles were
+// issue-bound: a 1999-token prompt through four blocks of the 7B shape took 19.3 ms with that, 6.0 ms with this; error
+// of the logits against 64 bits the same (1.8e-5 at 300 and 701 tokens).
+template <int HD>
 __global__ void __launch_bounds__(128) attn_prefill_kernel(const float* __restrict__ qkv, int row_stride, int m,
                                                            int pos0, int n_heads, int n_kv, int max_seq,
                                                            const __half* __restrict__ cache_k,
                                                            const __half* __restrict__ cache_v,
                                                            __nv_bfloat16* __restrict__ ctx)
 {
-    constexpr int hd = 32 * DPL;
-    const int lane = threadIdx.x & 31;
-    const int groups = (m + ROWS - 1) / ROWS;
-    const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (wid >= (int64_t)groups * n_heads) {
-        return;
-    }
-    // the longest rows first: the last CTAs to start are the shortest
-    const int row0 = (groups - 1 - (int)(wid / n_heads)) * ROWS, head = (int)(wid % n_heads);
-    const int kvh = head / (n_heads / n_kv);
-    const float scale = rsqrtf((float)hd);
-    float qv[ROWS][DPL], acc[ROWS][DPL], mx[ROWS], l[ROWS];
-    int keys[ROWS];
+    constexpr int KT = 64;                 // keys per tile
+    constexpr int ROW = HD * 2;            // bytes of a key row
+    constexpr int CH = ROW / 16;           // 16-byte pieces of it; piece c of row r sits at c ^ (r & 7)
+    constexpr int TILE = KT * ROW;
+    constexpr float P_SCALE = 16384.0f;
+    extern __shared__ __align__(128) uint8_t att_smem[];  // [2 buffers][K tile | V tile]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int head = blockIdx.y, kvh = head / (n_heads / n_kv);
+    const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 64;  // the longest rows first
+    const int n_keys = pos0 + min(row0 + 64, m);                   // keys the last row of this CTA sees
+    const int tiles = (n_keys + KT - 1) / KT;
+    const __half* kb = cache_k + (int64_t)kvh * max_seq * HD;
+    const __half* vb = cache_v + (int64_t)kvh * max_seq * HD;
+
+    auto fetch = [&](int tile) {
+        const uint32_t dst = smem_addr(att_smem) + (tile & 1) * 2 * TILE;
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        const int row = min(row0 + r, m - 1);  // a ragged last group repeats the last row (stored once)
-        keys[r] = pos0 + row + 1;
-        mx[r] = -INFINITY;
-        l[r] = 0.0f;
+        for (int i = 0; i < KT * CH / 128; ++i) {
+            const int idx = threadIdx.x + i * 128;
+            const int r = idx / CH, c = idx % CH;
+            const int key = min(tile * KT + r, n_keys - 1);  // beyond the last key: any row that exists
+            const uint32_t o = dst + r * ROW + ((c ^ (r & 7)) * 16);
+            cp_async16(o, kb + (int64_t)key * HD + c * 8);
+            cp_async16(o + TILE, vb + (int64_t)key * HD + c * 8);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+
+    // this thread's rows of the warp's 16: g and g + 8
+    int rows[2];
+    uint32_t qh[HD / 16][4], ql[HD / 16][4];
+    float unscale[2];
+    {
+        const float scale = rsqrtf((float)HD);
 #pragma unroll
-        for (int i = 0; i < DPL; ++i) {
-            qv[r][i] = qkv[(int64_t)row * row_stride + head * hd + lane * DPL + i] * scale;
-            acc[r][i] = 0.0f;
+        for (int rs = 0; rs < 2; ++rs) {
+            rows[rs] = row0 + warp * 16 + g + 8 * rs;
+            const float* q = qkv + (int64_t)min(rows[rs], m - 1) * row_stride + head * HD + 2 * t;
+            float2 x[HD / 8];
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < HD / 8; ++i) {
+                x[i] = *reinterpret_cast<const float2*>(q + 8 * i);
+                x[i].x *= scale;
+                x[i].y *= scale;
+                amax = fmaxf(amax, fmaxf(fabsf(x[i].x), fabsf(x[i].y)));
+            }
+            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+            int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127;
+            e = e == 128 ? 14 : max(e, -100);  // infinities and NaN stay what they are
+            const float up = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+            unscale[rs] = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
+#pragma unroll
+            for (int i = 0; i < HD / 16; ++i) {
+                split_f16x2(x[2 * i].x * up, x[2 * i].y * up, qh[i][rs], ql[i][rs]);
+                split_f16x2(x[2 * i + 1].x * up, x[2 * i + 1].y * up, qh[i][2 + rs], ql[i][2 + rs]);
+            }
         }
     }
-    const __half* kb = cache_k + (int64_t)kvh * max_seq * hd + lane * DPL;
-    const __half* vb = cache_v + (int64_t)kvh * max_seq * hd + lane * DPL;
-    const int n_keys = keys[ROWS - 1];
-    KvBatch<DPL> a, b;
-    kv_batch_load<DPL>(a, kb, vb, 0, n_keys);
-    for (int kbase = 0; kbase < n_keys; kbase += 16) {
-        if (kbase + 8 < n_keys) {
-            kv_batch_load<DPL>(b, kb, vb, kbase + 8, n_keys);
-        }
+    float acc[HD / 8][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            kv_batch_apply<DPL>(a, qv[r], kbase, keys[r], mx[r], l[r], acc[r]);
-        }
-        if (kbase + 16 < n_keys) {
-            kv_batch_load<DPL>(a, kb, vb, kbase + 16, n_keys);
-        }
+    for (int j = 0; j < HD / 8; ++j) {
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            kv_batch_apply<DPL>(b, qv[r], kbase + 8, keys[r], mx[r], l[r], acc[r]);
+        for (int i = 0; i < 4; ++i) {
+            acc[j][i] = 0.0f;
         }
     }
+
+    for (int tile = 0; tile < tiles; ++tile) {
+        if (tile + 1 < tiles) {
+            fetch(tile + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const uint32_t ks = smem_addr(att_smem) + (tile & 1) * 2 * TILE, vs = ks + TILE;
+
+        // scores of 16 rows x 64 keys
+        float sc[KT / 8][4];
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        if (row0 + r < m) {
+        for (int j = 0; j < KT / 8; ++j) {
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                ctx[(int64_t)(row0 + r) * n_heads * hd + head * hd + lane * DPL + i] =
-                    __float2bfloat16_rn(acc[r][i] / l[r]);
+            for (int i = 0; i < 4; ++i) {
+                sc[j][i] = 0.0f;
+            }
+            const int r = 8 * j + (lane & 7);
+#pragma unroll
+            for (int k2 = 0; k2 < HD / 32; ++k2) {
+                uint32_t b[4];
+                ldmatrix_x4(b, ks + r * ROW + (((4 * k2 + (lane >> 3)) ^ (r & 7)) * 16));
+                mma_f16(sc[j], qh[2 * k2], b[0], b[1]);
+                mma_f16(sc[j], ql[2 * k2], b[0], b[1]);
+                mma_f16(sc[j], qh[2 * k2 + 1], b[2], b[3]);
+                mma_f16(sc[j], ql[2 * k2 + 1], b[2], b[3]);
+            }
+        }
+        const bool masked = tile * KT + KT - 1 > pos0 + row0 + warp * 16;  // some row of the warp ends inside the tile
+        float corr[2], sum[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int rs = 0; rs < 2; ++rs) {
+            float mb = mx[rs];
+#pragma unroll
+            for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float& s = sc[j][2 * rs + i];
+                    s *= unscale[rs];
+                    if (masked && tile * KT + 8 * j + 2 * t + i > pos0 + rows[rs]) {
+                        s = -INFINITY;
+                    }
+                    mb = fmaxf(mb, s);
+                }
+            }
+            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 1));
+            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 2));
+            corr[rs] = __expf(mx[rs] - mb);
+            mx[rs] = mb;
+#pragma unroll
+            for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float p = __expf(sc[j][2 * rs + i] - mb);
+                    sum[rs] += p;
+                    sc[j][2 * rs + i] = p * P_SCALE;
+                }
+            }
+            l[rs] = l[rs] * corr[rs] + sum[rs];
+        }
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j) {
+            acc[j][0] *= corr[0];
+            acc[j][1] *= corr[0];
+            acc[j][2] *= corr[1];
+            acc[j][3] *= corr[1];
+        }
+        // probabilities times V: the score fragments are the A operand as they lie
+#pragma unroll
+        for (int kk = 0; kk < KT / 16; ++kk) {
+            uint32_t ph[4], pl[4];
+            split_f16x2(sc[2 * kk][0], sc[2 * kk][1], ph[0], pl[0]);
+            split_f16x2(sc[2 * kk][2], sc[2 * kk][3], ph[1], pl[1]);
+            split_f16x2(sc[2 * kk + 1][0], sc[2 * kk + 1][1], ph[2], pl[2]);
+            split_f16x2(sc[2 * kk + 1][2], sc[2 * kk + 1][3], ph[3], pl[3]);
+            const int r = 16 * kk + ((lane >> 3) & 1) * 8 + (lane & 7);
+#pragma unroll
+            for (int j2 = 0; j2 < HD / 16; ++j2) {
+                uint32_t b[4];
+                ldmatrix_x4_trans(b, vs + r * ROW + (((2 * j2 + (lane >> 4)) ^ (r & 7)) * 16));
+                mma_f16(acc[2 * j2], ph, b[0], b[1]);
+                mma_f16(acc[2 * j2 + 1], ph, b[2], b[3]);
+                mma_f16(acc[2 * j2], pl, b[0], b[1]);
+                mma_f16(acc[2 * j2 + 1], pl, b[2], b[3]);
+            }
+        }
+        __syncthreads();  // the buffer is refilled two tiles from now
+    }
+#pragma unroll
+    for (int rs = 0; rs < 2; ++rs) {
+        float tot = l[rs];
+        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 1);
+        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 2);
+        tot *= P_SCALE;
+        if (rows[rs] < m) {
+            __nv_bfloat16* out = ctx + (int64_t)rows[rs] * n_heads * HD + head * HD + 2 * t;
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) {
+                *reinterpret_cast<__nv_bfloat162*>(out + 8 * j) =
+                    __floats2bfloat162_rn(acc[j][2 * rs] / tot, acc[j][2 * rs + 1] / tot);
             }
         }
     }
@@ -1007,22 +1179,18 @@ cudaError_t ll_resid_rmsnorm_rows_f32(float* h, const float* add, const float* w
 cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
                             const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, cudaStream_t st)
 {
-    constexpr int ROWS = 4;
     const int row_stride = (n_heads + 2 * n_kv) * hd;
-    const int64_t warps = (int64_t)((m + ROWS - 1) / ROWS) * n_heads;
-    const unsigned grid = (unsigned)((warps + 3) / 4);
-    switch (hd) {
-    case 64:
-        attn_prefill_kernel<2, ROWS><<<grid, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
-                                                           cache_v, ctx);
-        break;
-    case 128:
-        attn_prefill_kernel<4, ROWS><<<grid, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
-                                                           cache_v, ctx);
-        break;
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    const dim3 grid((unsigned)((m + 63) / 64), (unsigned)n_heads);
+    auto launch = [&](auto kernel) -> cudaError_t {
+        const int smem = 4 * 64 * hd * 2;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        kernel<<<grid, 128, smem, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
+        return cudaGetLastError();
+    };
+    return hd == 64 ? launch(attn_prefill_kernel<64>) : hd == 128 ? launch(attn_prefill_kernel<128>) : cudaErrorInvalidValue;
 }
 
 cudaError_t ll_silu_mul_rows(const float* gu, int64_t m, int ffn, __nv_bfloat16* act, cudaStream_t st)
