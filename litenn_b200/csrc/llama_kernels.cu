@@ -1003,6 +1003,76 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(const float* __restri
     }
 }
 
+// Causal attention for a few rows, with fp32 arithmetic throughout: a 64-row tile of the kernel above would be mostly
+// padding.  Bound by the L2
+// reads of K and V (every row streams the whole prefix of its head), so one warp serves ROWS consecutive rows of
+// one head and reuses each loaded batch of eight keys for all of them; a row simply ignores the keys beyond its
+// own position.  Online softmax per row, one rescale per batch; output bf16 ctx[m][n_heads*hd].
+template <int DPL, int ROWS>
+__global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __restrict__ qkv, int row_stride, int m,
+                                                           int pos0, int n_heads, int n_kv, int max_seq,
+                                                           const __half* __restrict__ cache_k,
+                                                           const __half* __restrict__ cache_v,
+                                                           __nv_bfloat16* __restrict__ ctx)
+{
+    constexpr int hd = 32 * DPL;
+    const int lane = threadIdx.x & 31;
+    const int groups = (m + ROWS - 1) / ROWS;
+    const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (wid >= (int64_t)groups * n_heads) {
+        return;
+    }
+    // the longest rows first: the last CTAs to start are the shortest
+    const int row0 = (groups - 1 - (int)(wid / n_heads)) * ROWS, head = (int)(wid % n_heads);
+    const int kvh = head / (n_heads / n_kv);
+    const float scale = rsqrtf((float)hd);
+    float qv[ROWS][DPL], acc[ROWS][DPL], mx[ROWS], l[ROWS];
+    int keys[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        const int row = min(row0 + r, m - 1);  // a ragged last group repeats the last row (stored once)
+        keys[r] = pos0 + row + 1;
+        mx[r] = -INFINITY;
+        l[r] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) {
+            qv[r][i] = qkv[(int64_t)row * row_stride + head * hd + lane * DPL + i] * scale;
+            acc[r][i] = 0.0f;
+        }
+    }
+    const __half* kb = cache_k + (int64_t)kvh * max_seq * hd + lane * DPL;
+    const __half* vb = cache_v + (int64_t)kvh * max_seq * hd + lane * DPL;
+    const int n_keys = keys[ROWS - 1];
+    KvBatch<DPL> a, b;
+    kv_batch_load<DPL>(a, kb, vb, 0, n_keys);
+    for (int kbase = 0; kbase < n_keys; kbase += 16) {
+        if (kbase + 8 < n_keys) {
+            kv_batch_load<DPL>(b, kb, vb, kbase + 8, n_keys);
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            kv_batch_apply<DPL>(a, qv[r], kbase, keys[r], mx[r], l[r], acc[r]);
+        }
+        if (kbase + 16 < n_keys) {
+            kv_batch_load<DPL>(a, kb, vb, kbase + 16, n_keys);
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            kv_batch_apply<DPL>(b, qv[r], kbase + 8, keys[r], mx[r], l[r], acc[r]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        if (row0 + r < m) {
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                ctx[(int64_t)(row0 + r) * n_heads * hd + head * hd + lane * DPL + i] =
+                    __float2bfloat16_rn(acc[r][i] / l[r]);
+            }
+        }
+    }
+}
+
 // act[m][ffn] = bf16(silu(gate) * up) from gu[m][2*ffn], whose columns are the gate|up weight's rows:
 // groups of 8 gate channels followed by the same 8 channels of up (the matvec's SwiGLU epilogue
 // wants both halves of a channel in one 16-row tile).
@@ -1177,9 +1247,22 @@ cudaError_t ll_resid_rmsnorm_rows_f32(float* h, const float* add, const float* w
 }
 
 cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
-                            const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, cudaStream_t st)
+                            const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, int rows_max,
+                            cudaStream_t st)
 {
     const int row_stride = (n_heads + 2 * n_kv) * hd;
+    if (m <= rows_max && (hd == 64 || hd == 128)) {
+        constexpr int ROWS = 4;
+        const unsigned ctas = (unsigned)(((m + ROWS - 1) / ROWS * n_heads + 3) / 4);
+        if (hd == 64) {
+            attn_prefill_rows_kernel<2, ROWS><<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
+                                                                    cache_v, ctx);
+        } else {
+            attn_prefill_rows_kernel<4, ROWS><<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
+                                                                    cache_v, ctx);
+        }
+        return cudaGetLastError();
+    }
     const dim3 grid((unsigned)((m + 63) / 64), (unsigned)n_heads);
     auto launch = [&](auto kernel) -> cudaError_t {
         const int smem = 4 * 64 * hd * 2;
