@@ -944,25 +944,25 @@ int qmm_llama_prefill(qmm_llama* m, const int32_t* tokens_host, int n, int32_t* 
     const int d = c.d_model, hd = c.head_dim;
     const int pos0 = m->host_pos;
     // Activations are rounded to bf16 between the layers, and in a narrow model one rounding that falls the other way moves
-    // the logits by up to 2e-3 (in a 4096-wide one by 1e-4): up to 2048 wide attention keeps its order of summation up to
-    // 256 rows.  Such prompts are mostly launches.
+    // the logits by up to 2e-3 (in a 4096-wide one by 1e-4): up to 2048 wide every product keeps its order of summation,
+    // and so does attention up to 256 rows.  Such prompts are mostly launches (1536 x 2048, 64 rows: 14 us against 10).
     const bool keep_order = d <= 2048;
     LL_CUDA(cudaMemcpyAsync(m->tokens_dev, tokens_host, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st));
     LL_CUDA(ll_embed_rows(c.embd_fmt, m->embd, m->tokens_dev, n, d, m->hr, st));
     for (int l = 0; l < c.n_layers; ++l) {
         Layer& L = m->layers[l];
         LL_CUDA(ll_resid_rmsnorm_rows(m->hr, l == 0 ? nullptr : m->y2r, L.attn_norm, c.rms_eps, d, n, m->xn, st));
-        LL_QMM(qmm_gemm_bf16(L.w[QMM_LL_QKV], m->xn, m->qkvr, n, QMM_OUT_F32, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_QKV], m->xn, m->qkvr, n, QMM_OUT_F32, keep_order, st));
         LL_CUDA(ll_rope_kv(m->qkvr, m->pos, 0, n, m->hl, m->kvl, hd, c.rope_dim, m->rope_cos, m->rope_sin, c.max_seq,
                            L.cache_k, L.cache_v, st));
         LL_CUDA(ll_attn_prefill(m->qkvr, n, pos0, m->hl, m->kvl, hd, c.max_seq, L.cache_k, L.cache_v, m->ctx,
                                 keep_order ? 256 : 32, st));
-        LL_QMM(qmm_gemm_bf16(L.w[QMM_LL_O], m->ctx, m->yr, n, QMM_OUT_F32, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_O], m->ctx, m->yr, n, QMM_OUT_F32, keep_order, st));
         LL_QMM(all_reduce(m, m->yr, (size_t)n * d, st));
         LL_CUDA(ll_resid_rmsnorm_rows(m->hr, m->yr, L.ffn_norm, c.rms_eps, d, n, m->xn, st));
-        LL_QMM(qmm_gemm_bf16(L.w[QMM_LL_GU], m->xn, m->gur, n, QMM_OUT_F32, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_GU], m->xn, m->gur, n, QMM_OUT_F32, keep_order, st));
         LL_CUDA(ll_silu_mul_rows(m->gur, n, m->ffl, m->act, st));
-        LL_QMM(qmm_gemm_bf16(L.w[QMM_LL_DOWN], m->act, m->y2r, n, QMM_OUT_F32, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_DOWN], m->act, m->y2r, n, QMM_OUT_F32, keep_order, st));
         LL_QMM(all_reduce(m, m->y2r, (size_t)n * d, st));
     }
     // the last prompt position produces the first generated token

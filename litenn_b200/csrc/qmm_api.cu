@@ -776,7 +776,11 @@ int qmm_gemv_f32_host(const qmm_weight* w, const float* x_host, float* y_host, i
     return QMM_OK;
 }
 
-int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, void* stream)
+}  // extern "C"
+
+// For the decoder (llama_decoder.cu) and qmm_gemm_bf16.
+int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, bool keep_order,
+                      void* stream)
 {
     if (int rc = check_weight(w, "qmm_gemm_bf16")) {
         return rc;
@@ -799,8 +803,8 @@ int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int6
         return rc;
     }
     const char* why = nullptr;
-    cudaError_t e = launch_gemm_bf16(view_of(w), x_bf16_dev, y_dev, m, out_dtype == QMM_OUT_BF16 ? 1 : 0, w->sm_count,
-                                     status, static_cast<cudaStream_t>(stream), &why);
+    cudaError_t e = launch_gemm_bf16(view_of(w), x_bf16_dev, y_dev, m, out_dtype == QMM_OUT_BF16 ? 1 : 0, keep_order,
+                                     w->sm_count, status, static_cast<cudaStream_t>(stream), &why);
     if (e != cudaSuccess) {
         if (why) {
             return fail(e == cudaErrorNotSupported ? QMM_E_UNSUPPORTED : QMM_E_INVALID, "qmm_gemm_bf16: %s", why);
@@ -808,6 +812,13 @@ int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int6
         return fail_cuda(e, "qmm_gemm_bf16 launch");
     }
     return QMM_OK;
+}
+
+extern "C" {
+
+int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, void* stream)
+{
+    return qmm_internal_gemm(w, x_bf16_dev, y_dev, m, out_dtype, false, stream);
 }
 
 int qmm_gemm_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int64_t m, void* stream_v)

@@ -1,405 +1,155 @@
-// Prefill GEMM on the 5th-generation tensor cores (sm_100a): Y[M,N] = X[M,K] · Wᵀ with bf16
+// Prefill GEMM on the 5th-generation tensor cores (sm_100a): Y[M,N] = X[M,K] . W^T with bf16
 // activations, block-quantized weights dequantized on the fly, fp32 accumulation in TMEM.
 //
-// One CTA owns up to 256 activation rows (two 128-row UMMA tiles) and a contiguous group
-// of up to 16 row tiles of the weight (n <= 256 output features); its accumulators fill
-// 2 x n <= 512 TMEM columns, so every weight tile is dequantized once per CTA and reused
-// for all its activation rows.  Per 64-wide K step:
-//   warp 0          TMA: two 128x64 bf16 boxes of X -> shared memory (128-byte swizzle)
-//   warps 2..17     read the packed weight tiles (qmm_common.cuh) from global memory,
-//                   rebuild the exact fp32 values ggml's to_float gives, round them to bf16
-//                   and store them as the K-major, 128-byte-swizzled B tile
-//   warp 1, lane 0  tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, M=128, N=n, K=16) x 4 x 2,
-//                   then tcgen05.commit to hand the stage back
-// A 3-stage mbarrier ring decouples the three roles.  At the end warps 2..5 read the
-// accumulators with tcgen05.ld and write Y.  Every wait has an iteration limit; a CTA
-// that gives up sets the status word, still frees its TMEM and returns.
+// The weights are the A operand and live in TMEM, the activation rows ("tokens") are the B operand
+// in shared memory, so D has one weight row per TMEM lane and one token per column.  A CTA owns NB
+// blocks of 128 weight rows, up to 128 tokens and a range of K.  Per 64-wide K step:
+//   dequant warps   read packed tiles (qmm_common.cuh) from global memory, rebuild the exact fp32
+//                   values ggml's to_float gives, round them to bf16 and store them with
+//                   tcgen05.st.16x256b, whose register layout (lane 4g+t: row g and g+8, columns 2t, 2t+1)
+//                   is the packed tiles' own: no shuffle, no shared memory
+//   TMA warp        one 64 x tokens bf16 box of X -> shared memory (128-byte swizzle)
+//   MMA warp        tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, M = 128, N = tokens, K = 16), A from TMEM
+// Weights never pass through shared memory, whose bandwidth (128 bytes per cycle and SM) a B operand of
+// dequantized weights shares with the operand reads and the TMA writes.
+// Bound: the dequant warps' instruction issue.  Q6_K 4096 x 11264, 64 tokens: 27 us here against 125 us of the
+// shared-memory form, whose 16 dequant warps have two row tiles to work on; Q4_0 4096 x 4096, 512 tokens: 34.7 against
+// 51.6.  The MMAs are issued under elect.sync: with a lane comparison in its place the same kernel took a fifth longer
+// (Q4_0 4096 x 11008, 512 tokens: 94 us and 77 us).
+// Every wait has an iteration limit; a CTA that gives up sets the status word, still frees its TMEM and
+// returns.
 #include <cuda.h>
 
-#include <cstdlib>
+#include <algorithm>
+
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
+#include "qmm_gemm_dequant.cuh"
+#include "qmm_gemm_smem.h"
 #include "qmm_kernels.h"
 
 namespace qmm {
 
 namespace {
 
-constexpr int GEMM_STAGES = 3;
-constexpr int GEMM_BK = 64;                    // K per stage: 128 bytes of bf16 = one swizzle row
-constexpr int GEMM_A_TILE_BYTES = 128 * 128;   // 128 rows x 64 bf16
-constexpr int GEMM_A_STAGE_BYTES = 2 * GEMM_A_TILE_BYTES;
-constexpr int GEMM_B_STAGE_BYTES = 256 * 128;  // up to 256 weight rows x 64 bf16
-constexpr int GEMM_STAGE_BYTES = GEMM_A_STAGE_BYTES + GEMM_B_STAGE_BYTES;
-constexpr int GEMM_DEQ_WARPS = 16;
-constexpr int GEMM_THREADS = (2 + GEMM_DEQ_WARPS) * 32;
-constexpr int GEMM_SMEM_BYTES = GEMM_STAGES * GEMM_STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
-constexpr uint32_t GEMM_SPIN_LIMIT = 1u << 22;
+constexpr int GEMM_MAX_TOKENS = 128;     // B columns of one CTA
+constexpr int GEMM_A_STAGES = 4;         // K steps of dequantized weights in TMEM, 32 columns per block each
+constexpr int GEMM_MAX_RING = 8;         // K steps of tokens in shared memory
+constexpr int GEMM_BAR_BYTES = 1024;     // barriers, in front of the ring
 
-__device__ __forceinline__ uint32_t g_smem_u32(const void* p)
-{
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void g_mbar_init(uint64_t* bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(g_smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void g_mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(g_smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void g_mbar_expect_tx(uint64_t* bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(g_smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool g_mbar_wait(uint64_t* bar, uint32_t parity)
-{
-    const uint32_t addr = g_smem_u32(bar);
-    for (uint32_t spin = 0; spin < GEMM_SPIN_LIMIT; ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) {
-            return true;
-        }
-    }
-    return false;
-}
-
-// Same with a non-suspending probe: used by single elected threads that sit on the critical
-// path of the stage hand-over (a suspended try_wait wakes up late).
-__device__ __forceinline__ bool g_mbar_poll(uint64_t* bar, uint32_t parity)
-{
-    const uint32_t addr = g_smem_u32(bar);
-    for (uint32_t spin = 0; spin < (GEMM_SPIN_LIMIT << 4); ++spin) {
-        uint32_t done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) {
-            return true;
-        }
-    }
-    return false;
-}
-
-// 2-D tiled TMA load (no multicast): box {64 k, 128 rows} at element coordinates (k0, row0).
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int k0, int row0, uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            g_smem_u32(dst)),
-        "l"(map), "r"(k0), "r"(row0), "r"(g_smem_u32(bar))
-        : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);   // start address
-    d |= (uint64_t)1 << 16;                          // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                          // descriptor version of this architecture
-    d |= (uint64_t)2 << 61;                          // 128-byte swizzle
-    return d;
-}
-
-// Instruction descriptor: D fp32, A and B bf16, both K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t umma_idesc_bf16(int n)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                          uint32_t accumulate)
+// D[tmem] (+)= A[tmem, 128 x 16 bf16] * B[smem descriptor, 16 x N]
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                             uint32_t accumulate)
 {
     asm volatile(
         "{\n"
         ".reg .pred p;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
         "}\n" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(g_smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)[32])
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16])
 {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Byte offset of element (row, k) of a K-major tile with 128-byte rows and 128-byte swizzle:
-// the 16-byte chunk index is XORed with the row index modulo 8.
-__device__ __forceinline__ uint32_t swz128(int row, int k)
+// 16 rows x 32 columns (64 bf16 of K): registers 4p..4p+3 are K slice p, {row g: k 4t..4t+1, 4t+2..4t+3; row g+8: the
+// same}, in lane 4g+t.
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&r)[16])
 {
-    const uint32_t chunk = (uint32_t)(k >> 3) ^ (uint32_t)(row & 7);
-    return (uint32_t)row * 128u + chunk * 16u + (uint32_t)(k & 7) * 2u;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
-{
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-// Store four consecutive k values (k0 multiple of 4) of one row: 8 bytes inside one 16-byte chunk.
-__device__ __forceinline__ void store_b4(uint8_t* btile, int row, int k0, float v0, float v1, float v2, float v3)
-{
-    *reinterpret_cast<uint2*>(btile + swz128(row, k0)) = make_uint2(pack_bf16x2(v0, v1), pack_bf16x2(v2, v3));
-}
-
-// ---- dequantization of one 16-row x 64-column piece into the B tile --------------------------
-
-// What one lane keeps of a (row tile, 64-wide K step): quant words and scale words.
-struct PackedRegs {
-    uint32_t w[8];
-    uint32_t s[8];
-};
-
-__device__ __forceinline__ uint32_t ldg_u32(const uint8_t* p)
-{
-    return __ldg(reinterpret_cast<const uint32_t*>(p));
-}
-
-// `tile` points at the packed 16x256 tile, q (0..3) selects the 64-wide quarter of it.
-template <int FMT>
-__device__ __forceinline__ void load_packed(PackedRegs& r, const uint8_t* tile, int q, int lane)
-{
-    const int g = lane >> 2;
-    const uint8_t* p1 = tile + tile_p1_offset(FMT);
-    const uint8_t* p2 = tile + tile_p2_offset(FMT);
-    if constexpr (FMT == FMT_Q4_0 || FMT == FMT_Q4_K) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(tile) + q * 32 + lane);
-        r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w;
-        if constexpr (FMT == FMT_Q4_0) {
-            r.s[0] = ldg_u32(p1 + g * 16 + 4 * q);        // fp16 d of blocks 2q, 2q+1, row g
-            r.s[1] = ldg_u32(p1 + (g + 8) * 16 + 4 * q);  // row g+8
-        } else {
-#pragma unroll
-            for (int rs = 0; rs < 2; ++rs) {
-                const uint8_t* sp = p1 + (g + 8 * rs) * 12;
-                r.s[4 * rs + 0] = ldg_u32(sp);
-                r.s[4 * rs + 1] = ldg_u32(sp + 4);
-                r.s[4 * rs + 2] = ldg_u32(sp + 8);
-                r.s[4 * rs + 3] = ldg_u32(p2 + (g + 8 * rs) * 4);  // (d, dmin)
-            }
-        }
-    } else if constexpr (FMT == FMT_Q8_0) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(tile) + (2 * q) * 32 + lane);
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(tile) + (2 * q + 1) * 32 + lane);
-        r.w[0] = a.x; r.w[1] = a.y; r.w[2] = a.z; r.w[3] = a.w;
-        r.w[4] = b.x; r.w[5] = b.y; r.w[6] = b.z; r.w[7] = b.w;
-        r.s[0] = ldg_u32(p1 + g * 16 + 4 * q);
-        r.s[1] = ldg_u32(p1 + (g + 8) * 16 + 4 * q);
-    } else {  // Q6_K: quarter q = sub-blocks 4q..4q+3; words (q*2+rsel)*3 + {0,1,2} of this lane
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const int W = (q * 2 + rs) * 3 + j;
-                r.w[3 * rs + j] = ldg_u32(tile + (((W >> 2) * 32 + lane) * 4 + (W & 3)) * 4);
-            }
-            r.s[rs] = ldg_u32(p1 + (g + 8 * rs) * 16 + 4 * q);  // int8 scales of sub-blocks 4q..4q+3
-            r.s[2 + rs] = __ldg(reinterpret_cast<const unsigned short*>(p2 + (g + 8 * rs) * 2));
-        }
-    }
-}
-
-__device__ __forceinline__ float h2f_bits(uint32_t bits16)
-{
-    return __half2float(__ushort_as_half((unsigned short)(bits16 & 0xFFFFu)));
-}
-
-// Writes rows (16*rl + g) and (16*rl + g + 8), 64 columns, of the B tile.  The fp32 value of
-// every weight is computed with the same roundings as ggml's to_float, then rounded to bf16.
-template <int FMT>
-__device__ __forceinline__ void dequant_to_btile(const PackedRegs& r, uint8_t* btile, int rl, int q, int lane)
-{
-    const int g = lane >> 2;
-    const int t = lane & 3;
-    const int row0 = 16 * rl + g;
-    if constexpr (FMT == FMT_Q4_0) {
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi) {
-            // word wi: block 2q + (wi>>1), weights 16*(wi&1) + 4t.. -> column 32*(wi>>1) + 16*(wi&1) + 4t
-            const int k0 = 32 * (wi >> 1) + 16 * (wi & 1) + 4 * t;
-            const uint32_t w = r.w[wi];
-#pragma unroll
-            for (int rs = 0; rs < 2; ++rs) {
-                const float d = h2f_bits(r.s[rs] >> (16 * (wi >> 1)));
-                float v[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int n = (int)((w >> (8 * i + 4 * rs)) & 15u);
-                    v[i] = __fmul_rn((float)(n - 8), d);
-                }
-                store_b4(btile, row0 + 8 * rs, k0, v[0], v[1], v[2], v[3]);
-            }
-        }
-    } else if constexpr (FMT == FMT_Q8_0) {
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // word j of block b: row g + 8*(j&1), bytes 16*(j>>1) + 4t..
-                const int rs = j & 1;
-                const int k0 = 32 * b + 16 * (j >> 1) + 4 * t;
-                const uint32_t w = r.w[4 * b + j];
-                const float d = h2f_bits(r.s[rs] >> (16 * b));
-                float v[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    v[i] = __fmul_rn((float)(int)(signed char)((w >> (8 * i)) & 0xFFu), d);
-                }
-                store_b4(btile, row0 + 8 * rs, k0, v[0], v[1], v[2], v[3]);
-            }
-        }
-    } else if constexpr (FMT == FMT_Q4_K) {
-        // this quarter holds sub-blocks 2q and 2q+1
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-            const uint32_t w0 = r.s[4 * rs + 0], w1 = r.s[4 * rs + 1], w2 = r.s[4 * rs + 2];
-            const uint32_t scw = q < 2 ? (w0 & 0x3F3F3F3Fu) : ((w2 & 0x0F0F0F0Fu) | ((w0 >> 2) & 0x30303030u));
-            const uint32_t mnw = q < 2 ? (w1 & 0x3F3F3F3Fu) : (((w2 >> 4) & 0x0F0F0F0Fu) | ((w1 >> 2) & 0x30303030u));
-            const float d = h2f_bits(r.s[4 * rs + 3]);
-            const float dmin = h2f_bits(r.s[4 * rs + 3] >> 16);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int byte = (2 * q + h) & 3;
-                const float d1 = __fmul_rn(d, (float)((scw >> (8 * byte)) & 0xFFu));
-                const float m1 = __fmul_rn(dmin, (float)((mnw >> (8 * byte)) & 0xFFu));
-#pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const uint32_t w = r.w[2 * h + half];
-                    const int k0 = 32 * h + 16 * half + 4 * t;
-                    float v[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int n = (int)((w >> (8 * i + 4 * rs)) & 15u);
-                        v[i] = __fsub_rn(__fmul_rn(d1, (float)n), m1);
-                    }
-                    store_b4(btile, row0 + 8 * rs, k0, v[0], v[1], v[2], v[3]);
-                }
-            }
-        }
-    } else {  // Q6_K
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-            const uint32_t X = r.w[3 * rs + 0], Y = r.w[3 * rs + 1], Z = r.w[3 * rs + 2];
-            const float d = h2f_bits(r.s[2 + rs]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float ds = __fmul_rn(d, (float)(int)(signed char)((r.s[rs] >> (8 * j)) & 0xFFu));
-                float v[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint32_t u;
-                    if (j < 3) {
-                        const uint32_t word = j == 0 ? X : (j == 1 ? Y : Z);
-                        u = ((word >> (8 * i)) & 0xFFu) >> 2;
-                    } else {
-                        u = (((X >> (8 * i)) & 3u) << 4) | (((Y >> (8 * i)) & 3u) << 2) | ((Z >> (8 * i)) & 3u);
-                    }
-                    const int qv = (int)(u ^ 32u) - 32;
-                    v[i] = __fmul_rn(ds, (float)qv);
-                }
-                store_b4(btile, row0 + 8 * rs, 16 * j + 4 * t, v[0], v[1], v[2], v[3]);
-            }
-        }
-    }
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // ---- the kernel -----------------------------------------------------------------------------
 
 struct GemmArgs {
     WeightView w;
-    void* y;            // [M, N] row-major, fp32 or bf16
+    void* y;        // [M, N] row-major, fp32 or bf16
     int64_t m;
     int out_bf16;
-    int groups_per_tg;  // CTAs that share one group of 256 activation rows
+    int tokens;     // B columns per CTA, a multiple of 16
+    int t_tiles;    // token tiles
+    int ring;       // K steps of tokens in shared memory
     int* status;
 };
 
-
-template <int FMT>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
-    gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs args)
+__device__ __forceinline__ void store_y(const GemmArgs& a, int64_t token, int64_t row, float v)
 {
+    if (a.out_bf16) {
+        static_cast<__nv_bfloat16*>(a.y)[token * a.w.n + row] = __float2bfloat16_rn(v);
+    } else {
+        static_cast<float*>(a.y)[token * a.w.n + row] = v;
+    }
+}
+
+// grid = blocks x t_tiles x splits; a cluster of `splits` CTAs shares one output tile and cuts K between them.
+template <int FMT, int NB>
+__global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
+    gemm_ts_kernel(const __grid_constant__ CUtensorMap xmap, const GemmArgs args)
+{
+    namespace cg = cooperative_groups;
+    constexpr int DW = 8 * NB;               // dequant warps: one row tile each
+    constexpr uint32_t TMEM_COLS = 256 * NB;
+    constexpr uint32_t D_COL = GEMM_A_STAGES * 32 * NB;  // accumulators behind the A stages
     extern __shared__ uint8_t gemm_smem_raw[];
     // the swizzle pattern is defined on absolute shared-memory addresses: 1024-byte alignment
     uint8_t* smem = gemm_smem_raw + ((1024u - (g_smem_u32(gemm_smem_raw) & 1023u)) & 1023u);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GEMM_STAGES * GEMM_STAGE_BYTES);
-    uint64_t* full_a = bars;                    // [STAGES]  TMA bytes landed
-    uint64_t* full_b = bars + GEMM_STAGES;      // [STAGES]  dequant warps done
-    uint64_t* empty = bars + 2 * GEMM_STAGES;   // [STAGES]  MMAs that read the stage have completed
-    uint64_t* accum = bars + 3 * GEMM_STAGES;   // all MMAs completed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * GEMM_STAGES + 1);
+    uint64_t* full_b = reinterpret_cast<uint64_t*>(smem);  // [MAX_RING]  TMA bytes landed
+    uint64_t* empty_b = full_b + GEMM_MAX_RING;            // [MAX_RING]  MMAs that read the slot have completed
+    uint64_t* full_a = empty_b + GEMM_MAX_RING;            // [A_STAGES]  dequant warps done
+    uint64_t* empty_a = full_a + GEMM_A_STAGES;            // [A_STAGES]  MMAs that read the stage have completed
+    uint64_t* accum = empty_a + GEMM_A_STAGES;             // all MMAs completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+    uint8_t* ring = smem + GEMM_BAR_BYTES;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const WeightView& v = args.w;
-    const int tg = blockIdx.x / args.groups_per_tg;
-    const int gi = blockIdx.x % args.groups_per_tg;
-    const int rt0 = (int)((long long)v.rt * gi / args.groups_per_tg);
-    const int rt1 = (int)((long long)v.rt * (gi + 1) / args.groups_per_tg);
-    const int R = rt1 - rt0;        // row tiles of this CTA, 1..16
-    const int n = R * 16;           // UMMA N
-    const int64_t row_base = (int64_t)tg * 256;
-    const int ntt = (args.m - row_base) > 128 ? 2 : 1;
-    const int n_stages = (int)((v.k + GEMM_BK - 1) / GEMM_BK);
-    // CTAs that share activation rows start at different K offsets (the sum does not care
-    // about the order), so they do not all ask L2 for the same lines at the same moment.
-    const int k_rot = (int)((long long)n_stages * gi / args.groups_per_tg);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int splits = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    const int tile = blockIdx.x / splits;
+    const int block = tile / args.t_tiles;
+    const int64_t token0 = (int64_t)(tile % args.t_tiles) * args.tokens;
+    const int n = args.tokens;
+    const int slot_bytes = n * 128;
+    // this CTA's K: whole 256-wide chunks c0..c1, in steps of 64 up to the last one that holds data
+    const int c0 = (int)((long long)v.kc * rank / splits), c1 = (int)((long long)v.kc * (rank + 1) / splits);
+    const int k_steps = (int)((v.k + GEMM_BK - 1) / GEMM_BK);
+    const int s0 = 4 * c0, n_steps = min(4 * c1, k_steps) - s0;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GEMM_STAGES; ++s) {
-            g_mbar_init(&full_a[s], 1);
-            g_mbar_init(&full_b[s], GEMM_DEQ_WARPS);
-            g_mbar_init(&empty[s], 1);
+        for (int s = 0; s < GEMM_MAX_RING; ++s) {
+            g_mbar_init(&full_b[s], 1);
+            g_mbar_init(&empty_b[s], 1);
+        }
+        for (int s = 0; s < GEMM_A_STAGES; ++s) {
+            g_mbar_init(&full_a[s], DW);
+            g_mbar_init(&empty_a[s], 1);
         }
         g_mbar_init(accum, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
-        // 512 columns: two accumulators of up to 256 columns each
+    if (warp == DW + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem_u32(tmem_slot)),
-                     "r"(512u)
+                     "r"(TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -408,178 +158,161 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        // ---- TMA producer: activations ----
+    if (warp == DW) {
+        // ---- TMA producer: tokens ----
         if (lane == 0) {
-            for (int s = 0; s < n_stages; ++s) {
-                const int slot = s % GEMM_STAGES;
-                if (s >= GEMM_STAGES && !g_mbar_poll(&empty[slot], (uint32_t)(s / GEMM_STAGES - 1) & 1u)) {
+            int slot = 0;
+            uint32_t phase = 1;
+            for (int s = 0; s < n_steps; ++s) {
+                if (s >= args.ring && !g_mbar_wait(&empty_b[slot], phase)) {
                     atomicExch(args.status, 11);
                     break;
                 }
-                uint8_t* a = smem + (size_t)slot * GEMM_STAGE_BYTES;
-                g_mbar_expect_tx(&full_a[slot], (uint32_t)(ntt * GEMM_A_TILE_BYTES));
-                const int ks = (s + k_rot) % n_stages;
-                tma_load_2d(a, &xmap, ks * GEMM_BK, (int)row_base, &full_a[slot]);
-                if (ntt == 2) {
-                    tma_load_2d(a + GEMM_A_TILE_BYTES, &xmap, ks * GEMM_BK, (int)row_base + 128, &full_a[slot]);
+                g_mbar_expect_tx(&full_b[slot], (uint32_t)slot_bytes);
+                tma_load_2d(ring + slot * slot_bytes, &xmap, (s0 + s) * GEMM_BK, (int)token0, &full_b[slot]);
+                if (++slot == args.ring) {
+                    slot = 0;
+                    phase ^= 1u;
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---- MMA issuer ----
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc_bf16(n);
-            bool ok = true;
-            for (int s = 0; s < n_stages && ok; ++s) {
-                const int slot = s % GEMM_STAGES;
-                const uint32_t parity = (uint32_t)(s / GEMM_STAGES) & 1u;
-                if (!g_mbar_poll(&full_a[slot], parity) || !g_mbar_poll(&full_b[slot], parity)) {
+    } else if (warp == DW + 1) {
+        // ---- MMA issuer: the whole warp walks the steps, one lane issues ----
+        const uint32_t idesc = umma_idesc_bf16(n);
+        const uint64_t desc0 = umma_smem_desc(g_smem_u32(ring));
+        int slot = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int s = 0; s < n_steps; ++s) {
+            const int as = s % GEMM_A_STAGES;
+            ok = g_mbar_wait(&full_b[slot], phase) && g_mbar_wait(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) {
+                if (lane == 0) {
                     atomicExch(args.status, 12);
-                    ok = false;
-                    break;
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = g_smem_u32(smem + (size_t)slot * GEMM_STAGE_BYTES);
-                const uint32_t b_addr = a_addr + GEMM_A_STAGE_BYTES;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const uint64_t db = desc0 + (uint64_t)(slot * slot_bytes >> 4);
+                const uint32_t a0 = tmem_base + (uint32_t)(as * 32 * NB);
 #pragma unroll
                 for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
-                    const uint64_t db = umma_smem_desc(b_addr + kk * 32);
-                    for (int tt = 0; tt < ntt; ++tt) {
-                        const uint64_t da = umma_smem_desc(a_addr + tt * GEMM_A_TILE_BYTES + kk * 32);
-                        umma_bf16(tmem_base + (uint32_t)tt * 256u, da, db, idesc, (s > 0 || kk > 0) ? 1u : 0u);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        umma_bf16_ts(tmem_base + D_COL + (uint32_t)(b * GEMM_MAX_TOKENS), a0 + (uint32_t)(32 * b + 8 * kk),
+                                     db + (uint64_t)(2 * kk), idesc, (s > 0 || kk > 0) ? 1u : 0u);
                     }
                 }
-                umma_commit(&empty[slot]);  // arrives when the MMAs above have read their operands
+                umma_commit(&empty_a[as]);  // both arrive when the MMAs above have read their operands
+                umma_commit(&empty_b[slot]);
             }
-            if (ok) {
-                umma_commit(accum);
+            __syncwarp();
+            if (++slot == args.ring) {
+                slot = 0;
+                phase ^= 1u;
             }
         }
+        if (ok && elect_one()) {
+            umma_commit(accum);
+        }
+        __syncwarp();
     } else {
-        // ---- dequant producers: weights -> bf16 B tile ----
-        const int dw = warp - 2;  // 0..15: row tile dw of this CTA
-        const bool has0 = dw < R;
-        // Three register sets rotate: a set is refilled with the packed words of the K step
-        // three ahead as soon as it has been converted, so global-memory latency is covered
-        // by three steps of work.
-        PackedRegs pa0 = {}, pb0 = {}, pc0 = {};
+        // ---- dequant producers: weights -> TMEM ----
+        // a warp reaches the 32 TMEM lanes of its quadrant (warp % 4): two row tiles of a block
+        const int quad = warp & 3;
+        const int sub = (warp >> 2) & 1;
+        const int wb = warp >> 3;
+        const int rt = (block * NB + wb) * 8 + 2 * quad + sub;
+        const bool has = rt < v.rt;  // rows beyond the weight: their lanes are never stored to Y
+        const uint32_t a_addr = tmem_base + ((uint32_t)(32 * quad + 16 * sub) << 16) + (uint32_t)(32 * wb);
         const size_t tile_stride = tile_bytes(FMT);
-        const uint8_t* t0 = v.tiles + ((size_t)(rt0 + dw) * v.kc) * tile_stride;
-        auto fetch = [&](int s, PackedRegs& p0) {
-            if (s < n_stages && has0) {
-                const int ks = (s + k_rot) % n_stages;
-                load_packed<FMT>(p0, t0 + (size_t)(ks >> 2) * tile_stride, ks & 3, lane);
+        const uint8_t* wt = v.tiles + ((size_t)(has ? rt : 0) * v.kc + c0) * tile_stride;
+        Packed<FMT> P;
+        Scales<FMT> S, SN;
+        if (c0 < c1) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                load_quarter<FMT>(P, wt, q, lane);
             }
-        };
+            load_scales<FMT>(S, wt, lane >> 2);
+        }
+        SN = S;
         bool ok = true;
-        auto step = [&](int s, PackedRegs& p0) {
-            if (!ok || s >= n_stages) {
-                return;
+        int s = 0;
+        for (int c = c0; c < c1 && ok; ++c) {
+            const bool more = c + 1 < c1;
+            const uint8_t* next = wt + tile_stride;
+            if (more) {
+                load_scales<FMT>(SN, next, lane >> 2);
             }
-            const int slot = s % GEMM_STAGES;
-            const int ks = (s + k_rot) % n_stages;
-            if ((ks & 3) == 0) {
-                // pull the packed tiles two K chunks ahead into L2, one 128-byte line per lane
-                const int cpre = (ks >> 2) + 2;
-                if (cpre < v.kc && lane * 128 < (int)tile_stride) {
-                    if (has0) {
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(t0 + (size_t)cpre * tile_stride + lane * 128));
+            if (c + 3 < c1 && lane * 128 < (int)tile_stride) {  // three chunks ahead into L2
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(wt + 3 * tile_stride + lane * 128));
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (s < n_steps && ok) {
+                    uint32_t r[16];
+                    dequant_quarter<FMT>(P, S, q, r);
+                    if (more) {  // the registers just read are free: refill them from the next tile
+                        load_quarter<FMT>(P, next, q, lane);
                     }
-                }
-            }
-            if (s >= GEMM_STAGES) {
-                // lane 0 probes, the others wait for it at the warp barrier
-                bool landed = true;
-                if (lane == 0) {
-                    landed = g_mbar_poll(&empty[slot], (uint32_t)(s / GEMM_STAGES - 1) & 1u);
-                }
-                landed = __shfl_sync(0xFFFFFFFFu, landed, 0);
-                if (!landed) {
-                    if (lane == 0) {
-                        atomicExch(args.status, 13);
+                    const int as = s % GEMM_A_STAGES;
+                    if (s >= GEMM_A_STAGES && !g_mbar_wait(&empty_a[as], (uint32_t)(s / GEMM_A_STAGES - 1) & 1u)) {
+                        if (lane == 0) {
+                            atomicExch(args.status, 13);
+                        }
+                        ok = false;
                     }
-                    ok = false;
-                    return;
+                    ok = __all_sync(0xFFFFFFFFu, ok);
+                    if (ok) {
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (has) {
+                            tmem_st_16x256b_x4(a_addr + (uint32_t)(as * 32 * NB), r);
+                        }
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            g_mbar_arrive(&full_a[as]);
+                        }
+                    }
+                    ++s;
                 }
             }
-            uint8_t* btile = smem + (size_t)slot * GEMM_STAGE_BYTES + GEMM_A_STAGE_BYTES;
-            if (has0) {
-                dequant_to_btile<FMT>(p0, btile, dw, ks & 3, lane);
-            }
-            // make the generic-proxy stores visible to the tensor core (async proxy), then signal
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                g_mbar_arrive(&full_b[slot]);
-            }
-            fetch(s + 3, p0);
-        };
-        fetch(0, pa0);
-        fetch(1, pb0);
-        fetch(2, pc0);
-        for (int s = 0; s < n_stages; s += 3) {
-            step(s, pa0);
-            step(s + 1, pb0);
-            step(s + 2, pc0);
+            S = SN;
+            wt = next;
         }
 
-        // ---- epilogue: warps 2..5 own TMEM lanes 32*(warp%4).. ----
-        if (warp < 6) {
-            if (!g_mbar_wait(accum, 0)) {
-                if (lane == 0) {
-                    atomicExch(args.status, 14);
-                }
-            } else {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int quad = warp & 3;
-                for (int tt = 0; tt < ntt; ++tt) {
-                    const int64_t row = row_base + 128 * tt + 32 * quad + lane;
-                    for (int c0 = 0; c0 < n; c0 += 32) {
-                        uint32_t acc[32];
-                        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(tt * 256 + c0), acc);
-                        if (row < args.m) {
-                            const int64_t col0 = (int64_t)rt0 * 16 + c0;
-                            // 8 columns at a time: 16-byte (bf16) or 2 x 16-byte (fp32) stores when
-                            // the row pitch keeps them aligned, scalar stores at ragged edges
-                            if (args.out_bf16) {
-                                __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * v.n + col0;
-                                const bool vec = (v.n & 7) == 0;
+        // ---- epilogue: D has one weight row per lane, one token per column ----
+        if (!g_mbar_wait(accum, 0)) {
+            if (lane == 0) {
+                atomicExch(args.status, 14);
+            }
+        } else {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int units = NB * (n / 16);
+            for (int u = warp >> 2; u < units; u += 2 * NB) {
+                const int b = u / (n / 16), col0 = (u % (n / 16)) * 16;
+                uint32_t acc[16];
+                __syncwarp();
+                tmem_ld_32x32b_x16(tmem_base + ((uint32_t)(32 * quad) << 16) + D_COL + (uint32_t)(b * GEMM_MAX_TOKENS + col0),
+                                   acc);
+                const int row_in = 32 * quad + lane;
+                if (NB == 1 && splits > 1) {  // partial sums [token][128 rows] in the ring, whose last reader is done
+                    float* part = reinterpret_cast<float*>(ring);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    if (vec && c0 + 8 * j + 8 <= n && col0 + 8 * j + 8 <= v.n) {
-                                        uint4 o;
-                                        o.x = pack_bf16x2(__uint_as_float(acc[8 * j + 0]), __uint_as_float(acc[8 * j + 1]));
-                                        o.y = pack_bf16x2(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]));
-                                        o.z = pack_bf16x2(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5]));
-                                        o.w = pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]));
-                                        *reinterpret_cast<uint4*>(yo + 8 * j) = o;
-                                    } else {
+                    for (int i = 0; i < 16; ++i) {
+                        part[(col0 + i) * 128 + row_in] = __uint_as_float(acc[i]);
+                    }
+                } else {
+                    const int64_t row = (int64_t)(block * NB + b) * 128 + row_in;
+                    if (row < v.n) {
 #pragma unroll
-                                        for (int i = 8 * j; i < 8 * j + 8; ++i) {
-                                            if (col0 + i < v.n && c0 + i < n) {
-                                                yo[i] = __float2bfloat16_rn(__uint_as_float(acc[i]));
-                                            }
-                                        }
-                                    }
-                                }
-                            } else {
-                                float* yo = static_cast<float*>(args.y) + row * v.n + col0;
-                                const bool vec = (v.n & 3) == 0;
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    if (vec && c0 + 4 * j + 4 <= n && col0 + 4 * j + 4 <= v.n) {
-                                        *reinterpret_cast<uint4*>(yo + 4 * j) =
-                                            make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-                                    } else {
-#pragma unroll
-                                        for (int i = 4 * j; i < 4 * j + 4; ++i) {
-                                            if (col0 + i < v.n && c0 + i < n) {
-                                                yo[i] = __uint_as_float(acc[i]);
-                                            }
-                                        }
-                                    }
-                                }
+                        for (int i = 0; i < 16; ++i) {
+                            const int64_t token = token0 + col0 + i;
+                            if (token < args.m) {
+                                store_y(args, token, row, __uint_as_float(acc[i]));
                             }
                         }
                     }
@@ -590,8 +323,31 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    if (warp == DW + 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+    if constexpr (NB == 1) {
+        if (splits > 1) {
+            // The TMEM is free before the CTAs wait for one another.  Each sums its share of the tokens over the
+            // ranks' partials, always in rank order.
+            cluster.sync();
+            const int per = n / splits;  // n is a multiple of 16, splits 2, 4 or 8
+            const float* own = reinterpret_cast<const float*>(ring);
+            for (int i = threadIdx.x; i < per * 128; i += (DW + 2) * 32) {
+                const int col = rank * per + (i >> 7), row_in = i & 127;
+                float sum = 0.0f;
+                for (int r = 0; r < splits; ++r) {
+                    sum += cluster.map_shared_rank(own, r)[col * 128 + row_in];
+                }
+                const int64_t token = token0 + col, row = (int64_t)block * 128 + row_in;
+                if (token < args.m && row < v.n) {
+                    store_y(args, token, row, sum);
+                }
+            }
+            cluster.sync();  // a peer may still read this CTA's partials
+        }
     }
 }
 
@@ -615,18 +371,92 @@ EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-template <int FMT>
-cudaError_t launch_gemm_fmt(const CUtensorMap& xmap, const GemmArgs& args, int grid, cudaStream_t stream)
+// How one product is cut: NB blocks of 128 weight rows and `tokens` activation rows per CTA, `splits` CTAs along K; or,
+// with groups > 0, the shared-memory kernel with that many CTAs per 256 tokens.
+struct GemmPlan {
+    int nb, tokens, t_tiles, splits, ring, grid, smem, groups;
+};
+
+// Three shapes of CTA, and the one with the least estimated time wins.
+//   NB = 2    one CTA per SM, each token tile read once for 256 weight rows
+//   NB = 1    two CTAs per SM; cuts finer and can split K over a cluster: few tokens or few weight rows
+//   shared memory (qmm_gemm_smem.cu)   one dequantization per 256 tokens instead of 128: many tokens, where the
+//             dequantization is what the other two spend their time on
+// The estimates are microseconds on a B200: waves of CTAs x steps of 64 columns x time per step, plus a start-up per
+// wave, fitted to 100 (weight, token count) pairs from 512 x 1024 to 8192 x 28672 and 17 to 1999 tokens, over which the
+// choice costs 2 % against the best of all shapes.  Some of them (us): Q4_0 4096 x 4096, 64 tokens: NB = 1 with K split
+// in four 14.7, shared memory 43.3; 1024 tokens: NB = 2 45.2, shared memory 57.4; 1999 tokens: NB = 2 85.6, shared
+// memory 71.8.  Q6_K 8192 x 28672, 128 tokens: NB = 1 90.8, shared memory 327; 1024 tokens: 588 and 444.
+//
+// keep_order asks for the shared-memory form, whose sums run over K in one fixed order per row tile; the other two add the
+// K splits of a tile and start elsewhere, which changes the last bits.
+GemmPlan plan_gemm(const WeightView& w, int64_t m, int sm_count, bool keep_order)
 {
-    auto kernel = gemm_tcgen05_kernel<FMT>;
+    GemmPlan best = {};
+    const int64_t steps = (w.k + GEMM_BK - 1) / GEMM_BK;
+    const auto waves = [](int64_t ctas, int64_t slots) { return (double)((ctas + slots - 1) / slots); };
+    best.groups = gemm_smem_groups(w.rt, m, sm_count);
+    best.grid = (int)((m + 255) / 256) * best.groups;
+    const double tiles_per_cta = (double)((w.rt + best.groups - 1) / best.groups);
+    double best_cost = waves(best.grid, sm_count) * (4.0 * w.kc * (0.57 + 0.026 * tiles_per_cta) + 9.2);
+    if (keep_order) {
+        return best;
+    }
+    const int64_t min_tiles = (m + GEMM_MAX_TOKENS - 1) / GEMM_MAX_TOKENS;
+    for (int64_t tt = min_tiles; tt <= min_tiles + 1; ++tt) {
+        const int64_t tokens = ((m + tt - 1) / tt + 15) / 16 * 16;
+        const int64_t t_tiles = (m + tokens - 1) / tokens;
+        const double fill = (double)tokens / GEMM_MAX_TOKENS;
+        for (int nb = 1; nb <= 2; ++nb) {
+            const int64_t tiles = ((w.rt + 8 * nb - 1) / (8 * nb)) * t_tiles;
+            for (int splits = 1; splits <= (nb == 1 ? 8 : 1) && splits <= w.kc; splits *= 2) {
+                const int64_t ctas = tiles * splits;
+                double cost;
+                if (nb == 2) {
+                    cost = waves(ctas, sm_count) * (steps * (0.481 + 0.15 * fill) + 7.1);
+                } else {
+                    // two CTAs per SM; a last round that leaves most SMs with one runs its steps faster
+                    const double st = (double)((steps + splits - 1) / splits);
+                    const double paired = st * (0.615 + 0.104 * fill) + 6.7, alone = st * (0.385 + 0.034 * fill) + 6.7;
+                    const int64_t rounds = ctas / (2 * sm_count), rest = ctas % (2 * sm_count);
+                    cost = rounds * paired + (rest > sm_count ? paired : rest > 0 ? alone : 0.0) + (splits > 1 ? 4.2 : 0.0);
+                }
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best.groups = 0;
+                    best.nb = nb;
+                    best.tokens = (int)tokens;
+                    best.t_tiles = (int)t_tiles;
+                    best.splits = splits;
+                    best.grid = (int)ctas;
+                }
+            }
+        }
+    }
+    if (best.groups > 0) {
+        return best;
+    }
+    const int room = best.nb == 2 ? 200 * 1024 : 110 * 1024;
+    best.ring = std::min(GEMM_MAX_RING, room / (best.tokens * 128));
+    const int ring_bytes = best.ring * best.tokens * 128;
+    const int part_bytes = best.splits > 1 ? best.tokens * 128 * 4 : 0;
+    best.smem = 1024 /*alignment*/ + GEMM_BAR_BYTES + std::max(ring_bytes, part_bytes);
+    return best;
+}
+
+template <int FMT, int NB>
+cudaError_t launch_gemm_nb(const CUtensorMap& xmap, const GemmArgs& args, const GemmPlan& plan, cudaStream_t stream)
+{
+    auto kernel = gemm_ts_kernel<FMT, NB>;
     static bool configured[64] = {};
+    constexpr int LIMIT = NB == 2 ? 204 * 1024 : 113 * 1024;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
         return e;
     }
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMIT);
         if (e != cudaSuccess) {
             return e;
         }
@@ -634,15 +464,36 @@ cudaError_t launch_gemm_fmt(const CUtensorMap& xmap, const GemmArgs& args, int g
             configured[dev] = true;
         }
     }
-    kernel<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(xmap, args);
-    return cudaGetLastError();
+    if (plan.smem > LIMIT) {
+        return cudaErrorInvalidConfiguration;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)plan.grid);
+    cfg.blockDim = dim3((8 * NB + 2) * 32);
+    cfg.dynamicSmemBytes = (size_t)plan.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)plan.splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, xmap, args);
+}
+
+template <int FMT>
+cudaError_t launch_gemm_fmt(const CUtensorMap& xmap, const GemmArgs& args, const GemmPlan& plan, cudaStream_t stream)
+{
+    return plan.nb == 2 ? launch_gemm_nb<FMT, 2>(xmap, args, plan, stream)
+                        : launch_gemm_nb<FMT, 1>(xmap, args, plan, stream);
 }
 
 }  // namespace
 
 
-cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, int sm_count,
-                             int* status, cudaStream_t stream, const char** why)
+cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, bool keep_order,
+                             int sm_count, int* status, cudaStream_t stream, const char** why)
 {
     *why = nullptr;
     EncodeTiledFn encode = encode_tiled_fn();
@@ -654,10 +505,11 @@ cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, i
         *why = "activations must be 16-byte aligned with a row length that is a multiple of 8";
         return cudaErrorInvalidValue;
     }
+    const GemmPlan plan = plan_gemm(w, m, sm_count, keep_order);
     CUtensorMap xmap;
     const cuuint64_t dims[2] = {(cuuint64_t)w.k, (cuuint64_t)m};
     const cuuint64_t strides[1] = {(cuuint64_t)w.k * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)GEMM_BK, 128u};
+    const cuuint32_t box[2] = {(cuuint32_t)GEMM_BK, (cuuint32_t)(plan.groups > 0 ? GEMM_SMEM_BOX_ROWS : plan.tokens)};
     const cuuint32_t estr[2] = {1u, 1u};
     const CUresult cr = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x_bf16), dims, strides, box,
                                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -666,30 +518,23 @@ cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, i
         *why = "cuTensorMapEncodeTiled rejected the activation tensor";
         return cudaErrorInvalidValue;
     }
-    // Work split: groups of 256 activation rows x groups of <= 16 weight row tiles, sized so that
-    // one wave of CTAs covers the SMs as evenly as whole row tiles allow.
-    const int tgs = (int)((m + 255) / 256);
-    int per_tg = sm_count / tgs;
-    const int min_per_tg = (w.rt + 15) / 16;
-    if (per_tg < min_per_tg) {
-        per_tg = min_per_tg;
-    }
-    if (per_tg > w.rt) {
-        per_tg = w.rt;
+    if (plan.groups > 0) {
+        return launch_gemm_smem(w, xmap, y, m, out_bf16, plan.groups, keep_order, status, stream);
     }
     GemmArgs args;
     args.w = w;
     args.y = y;
     args.m = m;
     args.out_bf16 = out_bf16;
-    args.groups_per_tg = per_tg;
+    args.tokens = plan.tokens;
+    args.t_tiles = plan.t_tiles;
+    args.ring = plan.ring;
     args.status = status;
-    const int grid = tgs * per_tg;
     switch (w.fmt) {
-    case FMT_Q4_0: return launch_gemm_fmt<FMT_Q4_0>(xmap, args, grid, stream);
-    case FMT_Q8_0: return launch_gemm_fmt<FMT_Q8_0>(xmap, args, grid, stream);
-    case FMT_Q4_K: return launch_gemm_fmt<FMT_Q4_K>(xmap, args, grid, stream);
-    case FMT_Q6_K: return launch_gemm_fmt<FMT_Q6_K>(xmap, args, grid, stream);
+    case FMT_Q4_0: return launch_gemm_fmt<FMT_Q4_0>(xmap, args, plan, stream);
+    case FMT_Q8_0: return launch_gemm_fmt<FMT_Q8_0>(xmap, args, plan, stream);
+    case FMT_Q4_K: return launch_gemm_fmt<FMT_Q4_K>(xmap, args, plan, stream);
+    case FMT_Q6_K: return launch_gemm_fmt<FMT_Q6_K>(xmap, args, plan, stream);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -38,8 +38,9 @@ cudaError_t launch_gemv_q6_k(const WeightView& w, const XPackView& xp, float* y,
 cudaError_t launch_f32_to_bf16(const float* x, int64_t count, void* out_bf16, cudaStream_t stream);
 
 // Prefill GEMM on tcgen05: y[m,n] = x_bf16[m,k] · Wᵀ, fp32 or bf16 output.  On a
-// configuration error `*why` explains it.
-cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, int sm_count,
-                             int* status, cudaStream_t stream, const char** why);
+// configuration error `*why` explains it.  keep_order: sums in the shared-memory
+// form's order of K, also where another form is faster.
+cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, bool keep_order,
+                             int sm_count, int* status, cudaStream_t stream, const char** why);
 
 }  // namespace qmm
