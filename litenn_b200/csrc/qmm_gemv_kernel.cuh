@@ -263,9 +263,12 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
     const int g = lane >> 2;
     const int t = lane & 3;
     if constexpr (MC == 1) {
-        // lanes t=0 and t=1 each folded one block of every pair
-        acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1);
-        acc[1] += __shfl_xor_sync(0xFFFFFFFFu, acc[1], 1);
+        // lane t folded one block of every group of four
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], o);
+            acc[1] += __shfl_xor_sync(0xFFFFFFFFu, acc[1], o);
+        }
         if (t == 0) {
             red[warp * 16 + g] = acc[0];
             red[warp * 16 + g + 8] = acc[1];
