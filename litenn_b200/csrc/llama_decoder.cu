@@ -31,6 +31,7 @@
 
 #include "llama_kernels.h"
 #include "qmm_internal.h"
+#include "qmm_kernels.h"
 
 using namespace qmm;
 
@@ -111,7 +112,7 @@ struct qmm_llama {
     float *rope_cos = nullptr, *rope_sin = nullptr;
     int *pos = nullptr, *token = nullptr, *out_tokens = nullptr, *out_count = nullptr, *pair = nullptr, *pairs = nullptr;
     // prefill buffers
-    float *hr = nullptr, *yr = nullptr, *y2r = nullptr, *qkvr = nullptr, *gur = nullptr;
+    float *hr = nullptr, *yr = nullptr, *y2r = nullptr, *qkvr = nullptr;
     __nv_bfloat16 *xn = nullptr, *ctx = nullptr, *act = nullptr;
     int* tokens_dev = nullptr;
     // state
@@ -626,7 +627,6 @@ int qmm_llama_create(int device, const qmm_llama_config* cfg, qmm_llama** out)
         LL_TRY(dev_alloc(m, &m->yr, (size_t)mp * d));
         LL_TRY(dev_alloc(m, &m->y2r, (size_t)mp * d));
         LL_TRY(dev_alloc(m, &m->qkvr, (size_t)mp * qkv_w));
-        LL_TRY(dev_alloc(m, &m->gur, (size_t)mp * 2 * m->ffl));
         LL_TRY(dev_alloc(m, &m->xn, (size_t)mp * d));
         LL_TRY(dev_alloc(m, &m->ctx, (size_t)mp * m->hl * hd));
         LL_TRY(dev_alloc(m, &m->act, (size_t)mp * m->ffl));
@@ -952,17 +952,16 @@ int qmm_llama_prefill(qmm_llama* m, const int32_t* tokens_host, int n, int32_t* 
     for (int l = 0; l < c.n_layers; ++l) {
         Layer& L = m->layers[l];
         LL_CUDA(ll_resid_rmsnorm_rows(m->hr, l == 0 ? nullptr : m->y2r, L.attn_norm, c.rms_eps, d, n, m->xn, st));
-        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_QKV], m->xn, m->qkvr, n, QMM_OUT_F32, keep_order, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_QKV], m->xn, m->qkvr, n, GEMM_OUT_F32, keep_order, st));
         LL_CUDA(ll_rope_kv(m->qkvr, m->pos, 0, n, m->hl, m->kvl, hd, c.rope_dim, m->rope_cos, m->rope_sin, c.max_seq,
                            L.cache_k, L.cache_v, st));
         LL_CUDA(ll_attn_prefill(m->qkvr, n, pos0, m->hl, m->kvl, hd, c.max_seq, L.cache_k, L.cache_v, m->ctx,
                                 keep_order ? 256 : 32, st));
-        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_O], m->ctx, m->yr, n, QMM_OUT_F32, keep_order, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_O], m->ctx, m->yr, n, GEMM_OUT_F32, keep_order, st));
         LL_QMM(all_reduce(m, m->yr, (size_t)n * d, st));
         LL_CUDA(ll_resid_rmsnorm_rows(m->hr, m->yr, L.ffn_norm, c.rms_eps, d, n, m->xn, st));
-        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_GU], m->xn, m->gur, n, QMM_OUT_F32, keep_order, st));
-        LL_CUDA(ll_silu_mul_rows(m->gur, n, m->ffl, m->act, st));
-        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_DOWN], m->act, m->y2r, n, QMM_OUT_F32, keep_order, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_GU], m->xn, m->act, n, GEMM_OUT_SWIGLU, keep_order, st));
+        LL_QMM(qmm_internal_gemm(L.w[QMM_LL_DOWN], m->act, m->y2r, n, GEMM_OUT_F32, keep_order, st));
         LL_QMM(all_reduce(m, m->y2r, (size_t)n * d, st));
     }
     // the last prompt position produces the first generated token

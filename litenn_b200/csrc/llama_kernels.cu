@@ -669,10 +669,6 @@ __global__ void __launch_bounds__(512) commit_batch_kernel(const int* __restrict
 
 // ---- prefill (many tokens) ------------------------------------------------------------------------
 
-__device__ __forceinline__ void store_row_value(__nv_bfloat16* p, float v)
-{
-    *p = __float2bfloat16_rn(v);
-}
 __device__ __forceinline__ void store_row_value(float* p, float v)
 {
     *p = v;
@@ -1274,12 +1270,6 @@ cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int 
         return cudaGetLastError();
     };
     return hd == 64 ? launch(attn_prefill_kernel<64>) : hd == 128 ? launch(attn_prefill_kernel<128>) : cudaErrorInvalidValue;
-}
-
-cudaError_t ll_silu_mul_rows(const float* gu, int64_t m, int ffn, __nv_bfloat16* act, cudaStream_t st)
-{
-    silu_mul_rows_kernel<__nv_bfloat16><<<1024, 256, 0, st>>>(gu, m, ffn, act);
-    return cudaGetLastError();
 }
 
 cudaError_t ll_silu_mul_rows_f32(const float* gu, int64_t m, int ffn, float* act, cudaStream_t st)

@@ -72,7 +72,6 @@ cudaError_t ll_resid_rmsnorm_rows(float* h, const float* add, const float* w, fl
 cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
                             const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, int rows_max,
                             cudaStream_t st);
-cudaError_t ll_silu_mul_rows(const float* gu, int64_t m, int ffn, __nv_bfloat16* act, cudaStream_t st);
 // fp32 outputs of the two row kernels, for the packed matvec at batches 2..16
 cudaError_t ll_resid_rmsnorm_rows_f32(float* h, const float* add, const float* w, float eps, int d, int64_t m, float* xn,
                                       cudaStream_t st);

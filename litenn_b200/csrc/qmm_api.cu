@@ -779,7 +779,7 @@ int qmm_gemv_f32_host(const qmm_weight* w, const float* x_host, float* y_host, i
 }  // extern "C"
 
 // For the decoder (llama_decoder.cu) and qmm_gemm_bf16.
-int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, bool keep_order,
+int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out, bool keep_order,
                       void* stream)
 {
     if (int rc = check_weight(w, "qmm_gemm_bf16")) {
@@ -791,8 +791,8 @@ int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, 
     if (m < 1) {
         return fail(QMM_E_INVALID, "qmm_gemm_bf16: invalid row count %lld", (long long)m);
     }
-    if (out_dtype != QMM_OUT_F32 && out_dtype != QMM_OUT_BF16) {
-        return fail(QMM_E_INVALID, "qmm_gemm_bf16: unknown output type %d", out_dtype);
+    if (out < 0) {
+        return fail(QMM_E_INVALID, "qmm_gemm_bf16: unknown output type");
     }
     DeviceGuard guard(w->device);
     if (!guard.ok) {
@@ -803,8 +803,8 @@ int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, 
         return rc;
     }
     const char* why = nullptr;
-    cudaError_t e = launch_gemm_bf16(view_of(w), x_bf16_dev, y_dev, m, out_dtype == QMM_OUT_BF16 ? 1 : 0, keep_order,
-                                     w->sm_count, status, static_cast<cudaStream_t>(stream), &why);
+    cudaError_t e = launch_gemm_bf16(view_of(w), x_bf16_dev, y_dev, m, out, keep_order, w->sm_count, status,
+                                     static_cast<cudaStream_t>(stream), &why);
     if (e != cudaSuccess) {
         if (why) {
             return fail(e == cudaErrorNotSupported ? QMM_E_UNSUPPORTED : QMM_E_INVALID, "qmm_gemm_bf16: %s", why);
@@ -818,7 +818,8 @@ extern "C" {
 
 int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, void* stream)
 {
-    return qmm_internal_gemm(w, x_bf16_dev, y_dev, m, out_dtype, false, stream);
+    const int out = out_dtype == QMM_OUT_F32 ? GEMM_OUT_F32 : out_dtype == QMM_OUT_BF16 ? GEMM_OUT_BF16 : -1;
+    return qmm_internal_gemm(w, x_bf16_dev, y_dev, m, out, false, stream);
 }
 
 int qmm_gemm_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int64_t m, void* stream_v)

@@ -81,9 +81,9 @@ __device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_
 
 struct GemmArgs {
     WeightView w;
-    void* y;        // [M, N] row-major, fp32 or bf16
+    void* y;        // [M, N] row-major, fp32 or bf16; [M, N / 2] bf16 for GEMM_OUT_SWIGLU
     int64_t m;
-    int out_bf16;
+    int out;        // GEMM_OUT_*
     int tokens;     // B columns per CTA, a multiple of 16
     int t_tiles;    // token tiles
     int ring;       // K steps of tokens in shared memory
@@ -92,7 +92,7 @@ struct GemmArgs {
 
 __device__ __forceinline__ void store_y(const GemmArgs& a, int64_t token, int64_t row, float v)
 {
-    if (a.out_bf16) {
+    if (a.out == GEMM_OUT_BF16) {
         static_cast<__nv_bfloat16*>(a.y)[token * a.w.n + row] = __float2bfloat16_rn(v);
     } else {
         static_cast<float*>(a.y)[token * a.w.n + row] = v;
@@ -305,6 +305,21 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
                     for (int i = 0; i < 16; ++i) {
                         part[(col0 + i) * 128 + row_in] = __uint_as_float(acc[i]);
                     }
+                } else if (args.out == GEMM_OUT_SWIGLU) {
+                    // lanes 8..15 of a row tile hold up for the gates of lanes 0..7: the two swap every other token
+                    const int64_t row = (int64_t)(block * NB + b) * 128 + row_in;
+                    const bool up_lane = (lane & 8) != 0;
+                    const int64_t ch = (row >> 4) * 8 + (row & 7);
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const float mine = __uint_as_float(up_lane ? acc[i + 1] : acc[i]);
+                        const float other = __shfl_xor_sync(0xFFFFFFFFu, __uint_as_float(up_lane ? acc[i] : acc[i + 1]), 8);
+                        const int64_t token = token0 + col0 + i + (up_lane ? 1 : 0);
+                        if (token < args.m && row < v.n) {
+                            static_cast<__nv_bfloat16*>(args.y)[token * (v.n >> 1) + ch] =
+                                __float2bfloat16_rn(up_lane ? silu_mul(other, mine) : silu_mul(mine, other));
+                        }
+                    }
                 } else {
                     const int64_t row = (int64_t)(block * NB + b) * 128 + row_in;
                     if (row < v.n) {
@@ -335,15 +350,29 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
             cluster.sync();
             const int per = n / splits;  // n is a multiple of 16, splits 2, 4 or 8
             const float* own = reinterpret_cast<const float*>(ring);
-            for (int i = threadIdx.x; i < per * 128; i += (DW + 2) * 32) {
-                const int col = rank * per + (i >> 7), row_in = i & 127;
+            auto total = [&](int col, int row_in) {
                 float sum = 0.0f;
                 for (int r = 0; r < splits; ++r) {
                     sum += cluster.map_shared_rank(own, r)[col * 128 + row_in];
                 }
-                const int64_t token = token0 + col, row = (int64_t)block * 128 + row_in;
-                if (token < args.m && row < v.n) {
-                    store_y(args, token, row, sum);
+                return sum;
+            };
+            if (args.out == GEMM_OUT_SWIGLU) {
+                for (int i = threadIdx.x; i < per * 64; i += (DW + 2) * 32) {
+                    const int col = rank * per + (i >> 6), ch = i & 63, row_in = (ch >> 3) * 16 + (ch & 7);
+                    const int64_t token = token0 + col, row = (int64_t)block * 128 + row_in;
+                    if (token < args.m && row < v.n) {
+                        static_cast<__nv_bfloat16*>(args.y)[token * (v.n >> 1) + (int64_t)block * 64 + ch] =
+                            __float2bfloat16_rn(silu_mul(total(col, row_in), total(col, row_in + 8)));
+                    }
+                }
+            } else {
+                for (int i = threadIdx.x; i < per * 128; i += (DW + 2) * 32) {
+                    const int col = rank * per + (i >> 7), row_in = i & 127;
+                    const int64_t token = token0 + col, row = (int64_t)block * 128 + row_in;
+                    if (token < args.m && row < v.n) {
+                        store_y(args, token, row, total(col, row_in));
+                    }
                 }
             }
             cluster.sync();  // a peer may still read this CTA's partials
@@ -492,7 +521,7 @@ cudaError_t launch_gemm_fmt(const CUtensorMap& xmap, const GemmArgs& args, const
 }  // namespace
 
 
-cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, bool keep_order,
+cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out, bool keep_order,
                              int sm_count, int* status, cudaStream_t stream, const char** why)
 {
     *why = nullptr;
@@ -503,6 +532,10 @@ cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, i
     }
     if ((reinterpret_cast<uintptr_t>(x_bf16) & 15u) != 0 || (w.k % 8) != 0) {
         *why = "activations must be 16-byte aligned with a row length that is a multiple of 8";
+        return cudaErrorInvalidValue;
+    }
+    if (out == GEMM_OUT_SWIGLU && (w.n % 16 != 0 || (reinterpret_cast<uintptr_t>(y) & 15u) != 0)) {
+        *why = "a gate|up product needs whole 16-row tiles and a 16-byte aligned result";
         return cudaErrorInvalidValue;
     }
     const GemmPlan plan = plan_gemm(w, m, sm_count, keep_order);
@@ -519,13 +552,13 @@ cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, i
         return cudaErrorInvalidValue;
     }
     if (plan.groups > 0) {
-        return launch_gemm_smem(w, xmap, y, m, out_bf16, plan.groups, keep_order, status, stream);
+        return launch_gemm_smem(w, xmap, y, m, out, plan.groups, keep_order, status, stream);
     }
     GemmArgs args;
     args.w = w;
     args.y = y;
     args.m = m;
-    args.out_bf16 = out_bf16;
+    args.out = out;
     args.tokens = plan.tokens;
     args.t_tiles = plan.t_tiles;
     args.ring = plan.ring;

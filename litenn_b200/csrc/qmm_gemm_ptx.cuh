@@ -118,6 +118,12 @@ __device__ __forceinline__ float h2f_bits(uint32_t bits16)
     return __half2float(__ushort_as_half((unsigned short)(bits16 & 0xFFFFu)));
 }
 
+// sigmoid = 1 / (1 + exp(-x)), SiLU = x * sigmoid(x) (src/LiteNN/Layer/Activation.h:20-33,52-59)
+__device__ __forceinline__ float silu_mul(float g, float u)
+{
+    return (g * (1.0f / (1.0f + expf(-g)))) * u;
+}
+
 }  // namespace
 
 }  // namespace qmm

@@ -11,7 +11,7 @@
 //                   and store them as the K-major, 128-byte-swizzled B tile
 //   warp 1          tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, M=128, N=n, K=16) x 4 x 2,
 //                   then tcgen05.commit to hand the stage back
-// A 3-stage mbarrier ring decouples the three roles.  At the end warps 2..5 read the
+// A 3-stage mbarrier ring decouples the three roles.  At the end warps 2..17 read the
 // accumulators with tcgen05.ld and write Y.  Every wait has an iteration limit; a CTA
 // that gives up sets the status word, still frees its TMEM and returns.
 // Bound: shared-memory bandwidth (operand reads, dequantized stores, TMA writes) and the dequant warps' issue, about
@@ -21,6 +21,7 @@
 
 #include "qmm_gemm_dequant.cuh"
 #include "qmm_gemm_smem.h"
+#include "qmm_kernels.h"
 
 namespace qmm {
 
@@ -118,9 +119,9 @@ __device__ __forceinline__ void store_quarter(const uint32_t (&r)[16], uint8_t* 
 
 struct GemmArgs {
     WeightView w;
-    void* y;            // [M, N] row-major, fp32 or bf16
+    void* y;            // [M, N] row-major, fp32 or bf16; [M, N / 2] bf16 for GEMM_OUT_SWIGLU
     int64_t m;
-    int out_bf16;
+    int out;            // GEMM_OUT_*
     int groups_per_tg;  // CTAs that share one group of 256 activation rows
     int* status;
 };
@@ -302,59 +303,74 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             S = SN;
         }
 
-        // ---- epilogue: warps 2..5 own TMEM lanes 32*(warp%4).. ----
-        if (warp < 6) {
-            if (!g_mbar_wait(accum, 0)) {
-                if (lane == 0) {
-                    atomicExch(args.status, 14);
-                }
-            } else {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int quad = warp & 3;
-                for (int tt = 0; tt < ntt; ++tt) {
-                    const int64_t row = row_base + 128 * tt + 32 * quad + lane;
-                    for (int c0 = 0; c0 < n; c0 += 32) {
-                        uint32_t acc[32];
-                        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(tt * 256 + c0), acc);
-                        if (row < args.m) {
-                            const int64_t col0 = (int64_t)rt0 * 16 + c0;
-                            // 8 columns at a time: 16-byte (bf16) or 2 x 16-byte (fp32) stores when
-                            // the row pitch keeps them aligned, scalar stores at ragged edges
-                            if (args.out_bf16) {
-                                __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * v.n + col0;
-                                const bool vec = (v.n & 7) == 0;
+        // ---- epilogue: a warp reaches TMEM lanes 32*(warp%4).., four warps share them by columns ----
+        if (!g_mbar_wait(accum, 0)) {
+            if (lane == 0) {
+                atomicExch(args.status, 14);
+            }
+        } else {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int quad = warp & 3;
+            for (int tt = 0; tt < ntt; ++tt) {
+                const int64_t row = row_base + 128 * tt + 32 * quad + lane;
+                for (int c0 = 32 * (dw >> 2); c0 < n; c0 += 128) {
+                    uint32_t acc[32];
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(tt * 256 + c0), acc);
+                    if (row < args.m) {
+                        const int64_t col0 = (int64_t)rt0 * 16 + c0;
+                        // 8 columns at a time: 16-byte (bf16) or 2 x 16-byte (fp32) stores when
+                        // the row pitch keeps them aligned, scalar stores at ragged edges
+                        if (args.out == GEMM_OUT_SWIGLU) {
+                            // a row tile's 16 columns are 8 gates and their 8 ups
+                            __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * (v.n >> 1) + (col0 >> 1);
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    if (vec && c0 + 8 * j + 8 <= n && col0 + 8 * j + 8 <= v.n) {
-                                        uint4 o;
-                                        o.x = pack_bf16x2(__uint_as_float(acc[8 * j + 0]), __uint_as_float(acc[8 * j + 1]));
-                                        o.y = pack_bf16x2(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]));
-                                        o.z = pack_bf16x2(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5]));
-                                        o.w = pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]));
-                                        *reinterpret_cast<uint4*>(yo + 8 * j) = o;
-                                    } else {
+                            for (int j = 0; j < 2; ++j) {
+                                if (c0 + 16 * j < n && col0 + 16 * j < v.n) {
+                                    uint32_t o[4];
 #pragma unroll
-                                        for (int i = 8 * j; i < 8 * j + 8; ++i) {
-                                            if (col0 + i < v.n && c0 + i < n) {
-                                                yo[i] = __float2bfloat16_rn(__uint_as_float(acc[i]));
-                                            }
+                                    for (int i = 0; i < 4; ++i) {
+                                        const int e = 16 * j + 2 * i;
+                                        o[i] = pack_bf16x2(
+                                            silu_mul(__uint_as_float(acc[e]), __uint_as_float(acc[e + 8])),
+                                            silu_mul(__uint_as_float(acc[e + 1]), __uint_as_float(acc[e + 9])));
+                                    }
+                                    *reinterpret_cast<uint4*>(yo + 8 * j) = make_uint4(o[0], o[1], o[2], o[3]);
+                                }
+                            }
+                        } else if (args.out == GEMM_OUT_BF16) {
+                            __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * v.n + col0;
+                            const bool vec = (v.n & 7) == 0;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                if (vec && c0 + 8 * j + 8 <= n && col0 + 8 * j + 8 <= v.n) {
+                                    uint4 o;
+                                    o.x = pack_bf16x2(__uint_as_float(acc[8 * j + 0]), __uint_as_float(acc[8 * j + 1]));
+                                    o.y = pack_bf16x2(__uint_as_float(acc[8 * j + 2]), __uint_as_float(acc[8 * j + 3]));
+                                    o.z = pack_bf16x2(__uint_as_float(acc[8 * j + 4]), __uint_as_float(acc[8 * j + 5]));
+                                    o.w = pack_bf16x2(__uint_as_float(acc[8 * j + 6]), __uint_as_float(acc[8 * j + 7]));
+                                    *reinterpret_cast<uint4*>(yo + 8 * j) = o;
+                                } else {
+#pragma unroll
+                                    for (int i = 8 * j; i < 8 * j + 8; ++i) {
+                                        if (col0 + i < v.n && c0 + i < n) {
+                                            yo[i] = __float2bfloat16_rn(__uint_as_float(acc[i]));
                                         }
                                     }
                                 }
-                            } else {
-                                float* yo = static_cast<float*>(args.y) + row * v.n + col0;
-                                const bool vec = (v.n & 3) == 0;
+                            }
+                        } else {
+                            float* yo = static_cast<float*>(args.y) + row * v.n + col0;
+                            const bool vec = (v.n & 3) == 0;
 #pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    if (vec && c0 + 4 * j + 4 <= n && col0 + 4 * j + 4 <= v.n) {
-                                        *reinterpret_cast<uint4*>(yo + 4 * j) =
-                                            make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
-                                    } else {
+                            for (int j = 0; j < 8; ++j) {
+                                if (vec && c0 + 4 * j + 4 <= n && col0 + 4 * j + 4 <= v.n) {
+                                    *reinterpret_cast<uint4*>(yo + 4 * j) =
+                                        make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]);
+                                } else {
 #pragma unroll
-                                        for (int i = 4 * j; i < 4 * j + 4; ++i) {
-                                            if (col0 + i < v.n && c0 + i < n) {
-                                                yo[i] = __uint_as_float(acc[i]);
-                                            }
+                                    for (int i = 4 * j; i < 4 * j + 4; ++i) {
+                                        if (col0 + i < v.n && c0 + i < n) {
+                                            yo[i] = __uint_as_float(acc[i]);
                                         }
                                     }
                                 }
@@ -412,14 +428,14 @@ int gemm_smem_groups(int rt, int64_t m, int sm_count)
     return std::min(std::max(sm_count / tgs, (rt + 15) / 16), rt);
 }
 
-cudaError_t launch_gemm_smem(const WeightView& w, const CUtensorMap& xmap, void* y, int64_t m, int out_bf16, int groups,
+cudaError_t launch_gemm_smem(const WeightView& w, const CUtensorMap& xmap, void* y, int64_t m, int out, int groups,
                              bool keep_order, int* status, cudaStream_t stream)
 {
     GemmArgs args;
     args.w = w;
     args.y = y;
     args.m = m;
-    args.out_bf16 = out_bf16;
+    args.out = out;
     args.groups_per_tg = groups;
     args.status = status;
     const int grid = (int)((m + 255) / 256) * groups;

@@ -16,8 +16,8 @@ int qmm_internal_weight_view(const qmm_weight* w, qmm::WeightView* out);
 // fused prologue/epilogue (qmm_common.cuh); `y_dev` may be null when the epilogue replaces it.
 int qmm_internal_gemv_fused(const qmm_weight* w, const void* packed_dev, float* y_dev, const qmm::PeerScatter* scatter,
                             const qmm::GemvFuse* fuse, void* stream);
-// qmm_gemm_bf16 with the choice of a fixed summation order (launch_gemm_bf16).
-int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, bool keep_order,
+// qmm_gemm_bf16 with every GEMM_OUT_* form and the choice of a fixed summation order (qmm_kernels.h).
+int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out, bool keep_order,
                       void* stream);
 
 namespace qmm {

@@ -37,10 +37,12 @@ cudaError_t launch_gemv_q6_k(const WeightView& w, const XPackView& xp, float* y,
 // fp32 -> bf16, round to nearest even.
 cudaError_t launch_f32_to_bf16(const float* x, int64_t count, void* out_bf16, cudaStream_t stream);
 
-// Prefill GEMM on tcgen05: y[m,n] = x_bf16[m,k] · Wᵀ, fp32 or bf16 output.  On a
-// configuration error `*why` explains it.  keep_order: sums in the shared-memory
-// form's order of K, also where another form is faster.
-cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out_bf16, bool keep_order,
+// Prefill GEMM on tcgen05: y[m,n] = x_bf16[m,k] · Wᵀ.  On a configuration error `*why` explains it.
+//   GEMM_OUT_SWIGLU  the rows are interleaved gate|up (EPI_SWIGLU, qmm_common.cuh): y[m, n / 2] = bf16(silu(gate) * up);
+//                    n a multiple of 16, y 16-byte aligned
+//   keep_order       sums in the shared-memory form's order of K, also where another form is faster
+constexpr int GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2;
+cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out, bool keep_order,
                              int sm_count, int* status, cudaStream_t stream, const char** why);
 
 }  // namespace qmm
