@@ -16,7 +16,7 @@
 // 1/rms commutes with the matvec.)  With tensor parallelism the two K-split matvecs also exchange their
 // partial sums with the peers inside that epilogue (PeerScatter, qmm_common.cuh); with NCCL sums instead,
 // a stand-alone kernel does the residual add and the packing after the all-reduce.
-// Batched decode (enqueue_batch_step) is the unfused row form of the same chain.
+// Batched decode (enqueue_batch_step) is the row form of the same chain.
 #include "../../include/litenn_llama.h"
 
 #include <dlfcn.h>
@@ -131,9 +131,10 @@ struct qmm_llama {
     // batched decode (qmm_llama_batch_*): `batch` independent sequences share the weights
     int batch = 0, batch_max_steps = 0;
     std::vector<__half*> bcache_k, bcache_v;  // per block: [batch][kv heads][max_seq][head_dim]
-    float *bh = nullptr, *bx = nullptr, *bqkv = nullptr, *bctx = nullptr, *by = nullptr, *bgu = nullptr,
-          *blogits = nullptr;
-    uint8_t* bpk = nullptr;                   // packed activations of the batch (general form)
+    float *bh = nullptr, *bqkv = nullptr, *by = nullptr, *bgu = nullptr, *blogits = nullptr;
+    // packed activations of the batch, one buffer per width: rows past the batch and blocks past the width are
+    // never written and stay zero
+    uint8_t *bpk_d = nullptr, *bpk_ctx = nullptr, *bpk_act = nullptr;
     int *btok = nullptr, *bpos = nullptr, *bout = nullptr, *bsteps = nullptr, *bpair = nullptr, *bpairs = nullptr;
     std::vector<int> bpos_host, btok_host;
     int bsteps_host = 0;
@@ -469,38 +470,34 @@ void drop_graph(qmm_llama* m)
 
 // One step of `batch` sequences: every sequence's current token -> its next token.  The linears see the
 // batch as the rows of one skinny product (packed matvec at batch 2..16); attention, position and cache
-// are per sequence.  Unfused on purpose: each stage is the row form of a stage of the batch-1 chain.
+// are per sequence.  Whatever feeds a linear packs its own result, so a block is eight launches (twelve with
+// pack kernels of their own).
 int enqueue_batch_step(qmm_llama* m, cudaStream_t st)
 {
     const qmm_llama_config& c = m->cfg;
     const int B = m->batch, d = c.d_model, hd = c.head_dim;
-    const int qkv_w = (m->hl + 2 * m->kvl) * hd, ctx_w = m->hl * hd;
-    auto linear = [&](const qmm_weight* w, const float* x, int64_t k, float* y) -> int {
-        LL_QMM(qmm_pack_activations(m->device, x, B, k, m->bpk, st));
-        return qmm_gemv_packed(w, m->bpk, y, B, st);
-    };
     LL_CUDA(ll_embed_rows(c.embd_fmt, m->embd, m->btok, B, d, m->bh, st));
     for (int l = 0; l < c.n_layers; ++l) {
         Layer& L = m->layers[l];
-        LL_CUDA(ll_resid_rmsnorm_rows_f32(m->bh, l == 0 ? nullptr : m->by, L.attn_norm, c.rms_eps, d, B, m->bx, st));
-        LL_QMM(linear(L.w[QMM_LL_QKV], m->bx, d, m->bqkv));
+        LL_CUDA(ll_resid_rmsnorm_rows_packed(m->bh, l == 0 ? nullptr : m->by, L.attn_norm, c.rms_eps, d, B, m->bpk_d, st));
+        LL_QMM(qmm_gemv_packed(L.w[QMM_LL_QKV], m->bpk_d, m->bqkv, B, st));
         AttnBatch ab = {};
-        ab.qkv_stride = qkv_w;
+        ab.qkv_stride = (m->hl + 2 * m->kvl) * hd;
         ab.cache_stride = (int64_t)m->kvl * c.max_seq * hd;
-        ab.ctx = m->bctx;
-        ab.ctx_stride = ctx_w;
+        ab.packed = m->bpk_ctx;
+        ab.ncp = B == 1 ? 0 : xpack_ncp(B);
         LL_CUDA(ll_attn_fused(m->bqkv, m->bpos, m->hl, m->kvl, hd, c.rope_dim, m->rope_cos, m->rope_sin, c.max_seq,
                               m->bcache_k[l], m->bcache_v[l], nullptr, B, ab, st));
-        LL_QMM(linear(L.w[QMM_LL_O], m->bctx, ctx_w, m->by));
+        LL_QMM(qmm_gemv_packed(L.w[QMM_LL_O], m->bpk_ctx, m->by, B, st));
         LL_QMM(all_reduce(m, m->by, (size_t)B * d, st));
-        LL_CUDA(ll_resid_rmsnorm_rows_f32(m->bh, m->by, L.ffn_norm, c.rms_eps, d, B, m->bx, st));
-        LL_QMM(linear(L.w[QMM_LL_GU], m->bx, d, m->bgu));
-        LL_CUDA(ll_silu_mul_rows_f32(m->bgu, B, m->ffl, m->bx, st));
-        LL_QMM(linear(L.w[QMM_LL_DOWN], m->bx, m->ffl, m->by));
+        LL_CUDA(ll_resid_rmsnorm_rows_packed(m->bh, m->by, L.ffn_norm, c.rms_eps, d, B, m->bpk_d, st));
+        LL_QMM(qmm_gemv_packed(L.w[QMM_LL_GU], m->bpk_d, m->bgu, B, st));
+        LL_CUDA(ll_silu_mul_rows_packed(m->bgu, B, m->ffl, m->bpk_act, st));
+        LL_QMM(qmm_gemv_packed(L.w[QMM_LL_DOWN], m->bpk_act, m->by, B, st));
         LL_QMM(all_reduce(m, m->by, (size_t)B * d, st));
     }
-    LL_CUDA(ll_resid_rmsnorm_rows_f32(m->bh, m->by, m->final_norm, c.rms_eps, d, B, m->bx, st));
-    LL_QMM(linear(m->head, m->bx, d, m->blogits));
+    LL_CUDA(ll_resid_rmsnorm_rows_packed(m->bh, m->by, m->final_norm, c.rms_eps, d, B, m->bpk_d, st));
+    LL_QMM(qmm_gemv_packed(m->head, m->bpk_d, m->blogits, B, st));
     LL_CUDA(ll_argmax(m->blogits, m->vl, m->vl * c.tp_rank, ARGMAX_CTAS, m->bpair, B, m->vl, st));
     const int* pairs = m->bpair;
     if (c.tp_size > 1) {
@@ -1089,17 +1086,19 @@ int qmm_llama_batch_create(qmm_llama* m, int batch, int max_steps)
     const qmm_llama_config& c = m->cfg;
     const size_t B = (size_t)batch, d = (size_t)c.d_model, hd = (size_t)c.head_dim;
     const size_t qkv_w = (size_t)(m->hl + 2 * m->kvl) * hd, ctx_w = (size_t)m->hl * hd;
-    const size_t widest = std::max(std::max(d, ctx_w), (size_t)m->ffl);
-    size_t pk = 0;
-    LL_QMM(qmm_packed_activation_bytes((int64_t)widest, batch, &pk));
+    auto alloc_packed = [&](uint8_t** p, size_t width) -> int {
+        size_t bytes = 0;
+        LL_QMM(qmm_packed_activation_bytes((int64_t)width, batch, &bytes));
+        return dev_alloc(m, p, bytes);
+    };
     LL_QMM(dev_alloc(m, &m->bh, B * d));
-    LL_QMM(dev_alloc(m, &m->bx, B * widest));
     LL_QMM(dev_alloc(m, &m->bqkv, B * qkv_w));
-    LL_QMM(dev_alloc(m, &m->bctx, B * ctx_w));
     LL_QMM(dev_alloc(m, &m->by, B * d));
     LL_QMM(dev_alloc(m, &m->bgu, B * 2 * (size_t)m->ffl));
     LL_QMM(dev_alloc(m, &m->blogits, B * (size_t)m->vl));
-    LL_QMM(dev_alloc(m, &m->bpk, pk));
+    LL_QMM(alloc_packed(&m->bpk_d, d));
+    LL_QMM(alloc_packed(&m->bpk_ctx, ctx_w));
+    LL_QMM(alloc_packed(&m->bpk_act, (size_t)m->ffl));
     LL_QMM(dev_alloc(m, &m->btok, B));
     LL_QMM(dev_alloc(m, &m->bpos, B));
     LL_QMM(dev_alloc(m, &m->bout, B * (size_t)max_steps));

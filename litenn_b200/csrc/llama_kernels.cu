@@ -468,14 +468,16 @@ __global__ void __launch_bounds__(256) attn_fused_kernel(const float* __restrict
             L += parts[r][h2][hd + 1] * f;
         }
         vals[threadIdx.x] = L > 0.0f ? a / L : 0.0f;
-        if (ab.ctx) {  // batched decode keeps fp32 rows; the rows are packed together afterwards
-            if (chunk * 256 + (int)threadIdx.x < n_heads * hd) {
-                ab.ctx[(int64_t)blockIdx.y * ab.ctx_stride + chunk * 256 + threadIdx.x] = vals[threadIdx.x];
-            }
-            return;
-        }
     }
     __syncthreads();
+    if (ab.packed) {  // batched decode: this sequence's row of the chunk's record
+        if (threadIdx.x < 64) {
+            const int e = 4 * threadIdx.x;  // two warps, 128 activations each
+            const float4 v = make_float4(vals[e], vals[e + 1], vals[e + 2], vals[e + 3]);
+            pack_row_block4(v, ab.packed + (size_t)chunk * xpack_row_rec_bytes(ab.ncp), ab.ncp, blockIdx.y, e >> 5, true);
+        }
+        return;
+    }
     if (threadIdx.x < 32) {
         float r8[8];
 #pragma unroll
@@ -669,33 +671,43 @@ __global__ void __launch_bounds__(512) commit_batch_kernel(const int* __restrict
 
 // ---- prefill (many tokens) ------------------------------------------------------------------------
 
-__device__ __forceinline__ void store_row_value(float* p, float v)
-{
-    *p = v;
-}
+// Where a row kernel puts four neighbouring values of its row.  All threads of a warp call it; `ok` marks the ones that
+// hold values.
+struct RowOutBf16 {  // bf16 rows for the GEMM
+    __nv_bfloat16* p;
+    int64_t width;
+    __device__ __forceinline__ void put(int64_t row, int i4, const float4& v, bool ok) const
+    {
+        if (ok) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(p + row * width + 4 * (int64_t)i4) =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+    }
+};
+struct RowOutPacked {  // the row's part of the matvec's packed activations; rows are a multiple of 32 wide
+    uint8_t* p;
+    int ncp;
+    __device__ __forceinline__ void put(int64_t row, int i4, const float4& v, bool ok) const
+    {
+        pack_row_block4(v, p + (size_t)(i4 >> 6) * xpack_row_rec_bytes(ncp), ncp, (int)row, (i4 >> 3) & 7, ok);
+    }
+};
 
-__device__ __forceinline__ void store_row_values(__nv_bfloat16* p, float a, float b, float c, float d4)
-{
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d4);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-}
-__device__ __forceinline__ void store_row_values(float* p, float a, float b, float c, float d4)
-{
-    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d4);
-}
-
-// Per row: h += add (optional); xn = rmsnorm(h) * w, as bf16 for the GEMM or as fp32 for the packed matvec.
+// Per row: h += add (optional); rmsnorm(h) * w, as bf16 for the GEMM or packed for the matvec of a batch.
 // One CTA per row (d a multiple of 4); a thread keeps its float4 pieces of the row in registers between the
 // two passes (up to 8 pieces = d <= 8192 with 256 threads; longer rows re-read h), and all of a pass's loads
 // are issued before the first is used: with scalar loads in a 16-trip loop the kernel took 18 us for 16 rows.
 // Statistics and the scale by the weight in double, one cast (ComputePrimitives.h:755-816); one double
 // reciprocal per row instead of a division per element (within one unit in the last place of the double
 // quotient, so the fp32 result is the reference's).
-template <typename OutT>
+template <typename Out>
 __global__ void __launch_bounds__(256) resid_rmsnorm_rows_kernel(float* __restrict__ h, const float* __restrict__ add,
                                                                  const float* __restrict__ w, float eps, int d,
-                                                                 OutT* __restrict__ xn)
+                                                                 Out out)
 {
+    pdl_trigger();
+    pdl_sync();
     constexpr int KEEP = 8;
     __shared__ double red[32];
     const int64_t row = blockIdx.x;
@@ -741,20 +753,24 @@ __global__ void __launch_bounds__(256) resid_rmsnorm_rows_kernel(float* __restri
     const double inv = 1.0 / sqrt(ss / (double)d + (double)eps);
     const float4* wr = reinterpret_cast<const float4*>(w);
     auto emit = [&](int i, const float4& v) {
-        const float4 ww = wr[i];
-        store_row_values(xn + row * d + 4 * (int64_t)i, (float)(((double)v.x * inv) * (double)ww.x),
-                         (float)(((double)v.y * inv) * (double)ww.y), (float)(((double)v.z * inv) * (double)ww.z),
-                         (float)(((double)v.w * inv) * (double)ww.w));
+        const bool ok = i < n4;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (ok) {
+            const float4 ww = wr[i];
+            o = make_float4((float)(((double)v.x * inv) * (double)ww.x), (float)(((double)v.y * inv) * (double)ww.y),
+                            (float)(((double)v.z * inv) * (double)ww.z), (float)(((double)v.w * inv) * (double)ww.w));
+        }
+        out.put(row, i, o, ok);
     };
 #pragma unroll
     for (int j = 0; j < KEEP; ++j) {
-        const int i = threadIdx.x + j * 256;
-        if (i < n4) {
-            emit(i, keep[j]);
+        if (j * 256 < n4) {
+            emit(threadIdx.x + j * 256, keep[j]);
         }
     }
-    for (int i = threadIdx.x + KEEP * 256; i < n4; i += 256) {
-        emit(i, hr[i]);
+    for (int i0 = KEEP * 256; i0 < n4; i0 += 256) {
+        const int i = i0 + threadIdx.x;
+        emit(i, i < n4 ? hr[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f));
     }
 }
 
@@ -1069,27 +1085,23 @@ __global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __r
     }
 }
 
-// act[m][ffn] = bf16(silu(gate) * up) from gu[m][2*ffn], whose columns are the gate|up weight's rows:
-// groups of 8 gate channels followed by the same 8 channels of up (the matvec's SwiGLU epilogue
-// wants both halves of a channel in one 16-row tile).
-template <typename OutT>
-__global__ void silu_mul_rows_kernel(const float* __restrict__ gu, int64_t m, int ffn, OutT* __restrict__ act)
+// silu(gate) * up, packed for ffn_down, from gu[m][2*ffn], whose columns are the gate|up weight's rows: groups of 8 gate
+// channels followed by the same 8 channels of up (the matvec's SwiGLU epilogue wants both halves of a channel in one
+// 16-row tile).  A thread takes four neighbouring channels; grid (channels / 1024, rows).
+__global__ void __launch_bounds__(256) silu_mul_rows_kernel(const float* __restrict__ gu, int ffn, RowOutPacked out)
 {
-    const int64_t total = m * ffn;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / ffn;
-        const int c = (int)(i % ffn);
-        const int col = (c >> 3) * 16 + (c & 7);
-        const float g = gu[r * 2 * ffn + col], u = gu[r * 2 * ffn + col + 8];
-        store_row_value(&act[i], (g * (1.0f / (1.0f + expf(-g)))) * u);
+    pdl_trigger();
+    pdl_sync();
+    const int i4 = blockIdx.x * 256 + threadIdx.x;
+    const bool ok = 4 * i4 < ffn;
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (ok) {
+        const float* p = gu + (int64_t)blockIdx.y * 2 * ffn + (i4 >> 1) * 16 + (i4 & 1) * 4;
+        const float4 g = *reinterpret_cast<const float4*>(p), u = *reinterpret_cast<const float4*>(p + 8);
+        o = make_float4((g.x * (1.0f / (1.0f + expf(-g.x)))) * u.x, (g.y * (1.0f / (1.0f + expf(-g.y)))) * u.y,
+                        (g.z * (1.0f / (1.0f + expf(-g.z)))) * u.z, (g.w * (1.0f / (1.0f + expf(-g.w)))) * u.w);
     }
-}
-
-__global__ void add_rows_kernel(float* __restrict__ h, const float* __restrict__ add, int64_t total)
-{
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        h[i] += add[i];
-    }
+    out.put(blockIdx.y, i4, o, ok);
 }
 
 template <typename... KArgs, typename... Args>
@@ -1231,15 +1243,15 @@ cudaError_t ll_commit_token(const int* pairs, int n_local, const ArgmaxExchange&
 cudaError_t ll_resid_rmsnorm_rows(float* h, const float* add, const float* w, float eps, int d, int64_t m,
                                   __nv_bfloat16* xn, cudaStream_t st)
 {
-    resid_rmsnorm_rows_kernel<__nv_bfloat16><<<(unsigned)m, 256, 0, st>>>(h, add, w, eps, d, xn);
-    return cudaGetLastError();
+    return launch_pdl(resid_rmsnorm_rows_kernel<RowOutBf16>, dim3((unsigned)m), dim3(256), 0, st, h, add, w, eps, d,
+                      RowOutBf16{xn, d});
 }
 
-cudaError_t ll_resid_rmsnorm_rows_f32(float* h, const float* add, const float* w, float eps, int d, int64_t m, float* xn,
-                                      cudaStream_t st)
+cudaError_t ll_resid_rmsnorm_rows_packed(float* h, const float* add, const float* w, float eps, int d, int m,
+                                         uint8_t* packed, cudaStream_t st)
 {
-    resid_rmsnorm_rows_kernel<float><<<(unsigned)m, 256, 0, st>>>(h, add, w, eps, d, xn);
-    return cudaGetLastError();
+    return launch_pdl(resid_rmsnorm_rows_kernel<RowOutPacked>, dim3((unsigned)m), dim3(256), 0, st, h, add, w, eps, d,
+                      RowOutPacked{packed, m == 1 ? 0 : xpack_ncp(m)});
 }
 
 cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
@@ -1272,16 +1284,11 @@ cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int 
     return hd == 64 ? launch(attn_prefill_kernel<64>) : hd == 128 ? launch(attn_prefill_kernel<128>) : cudaErrorInvalidValue;
 }
 
-cudaError_t ll_silu_mul_rows_f32(const float* gu, int64_t m, int ffn, float* act, cudaStream_t st)
+cudaError_t ll_silu_mul_rows_packed(const float* gu, int m, int ffn, uint8_t* packed, cudaStream_t st)
 {
-    silu_mul_rows_kernel<float><<<(unsigned)std::min<int64_t>(1024, (m * ffn + 255) / 256), 256, 0, st>>>(gu, m, ffn, act);
-    return cudaGetLastError();
-}
-
-cudaError_t ll_add_rows(float* h, const float* add, int64_t total, cudaStream_t st)
-{
-    add_rows_kernel<<<1024, 256, 0, st>>>(h, add, total);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)((ffn / 4 + 255) / 256), (unsigned)m);
+    return launch_pdl(silu_mul_rows_kernel, grid, dim3(256), 0, st, gu, ffn,
+                      RowOutPacked{packed, m == 1 ? 0 : xpack_ncp(m)});
 }
 
 }  // namespace qmm

@@ -39,12 +39,12 @@ cudaError_t ll_rope_kv(float* qkv, const int* pos, int pos_add, int rows, int n_
                        const float* rope_cos, const float* rope_sin, int max_seq, __half* cache_k, __half* cache_v,
                        cudaStream_t st);
 // Batched decode attention (grid.y = sequence): every sequence has its own qkv row, position and cache.
-// All zero = one sequence whose context is packed for the attn_output matvec.
+// All zero = one sequence whose context is packed as compact records.
 struct AttnBatch {
     int qkv_stride;        // floats between the sequences' qkv rows
     int64_t cache_stride;  // halves between the sequences' caches of one block
-    float* ctx;            // not null: the context is stored as fp32 rows [batch][ctx_stride] instead of packed
-    int ctx_stride;
+    uint8_t* packed;       // not null: each sequence's context becomes its row of these packed activations
+    int ncp;               // their column groups; 0 = compact (a batch of one)
 };
 // RoPE of q and the new key, KV append, attention over the cache, for `batch` sequences (pos[batch]).
 cudaError_t ll_attn_fused(const float* qkv, const int* pos, int n_heads, int n_kv, int hd, int rope_dim,
@@ -72,12 +72,9 @@ cudaError_t ll_resid_rmsnorm_rows(float* h, const float* add, const float* w, fl
 cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
                             const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, int rows_max,
                             cudaStream_t st);
-// fp32 outputs of the two row kernels, for the packed matvec at batches 2..16
-cudaError_t ll_resid_rmsnorm_rows_f32(float* h, const float* add, const float* w, float eps, int d, int64_t m, float* xn,
-                                      cudaStream_t st);
-cudaError_t ll_silu_mul_rows_f32(const float* gu, int64_t m, int ffn, float* act, cudaStream_t st);
-cudaError_t ll_add_rows(float* h, const float* add, int64_t total, cudaStream_t st);
-
-
+// The two row kernels of a batch of m rows (1..16), with their result packed for its matvec.
+cudaError_t ll_resid_rmsnorm_rows_packed(float* h, const float* add, const float* w, float eps, int d, int m,
+                                         uint8_t* packed, cudaStream_t st);
+cudaError_t ll_silu_mul_rows_packed(const float* gu, int m, int ffn, uint8_t* packed, cudaStream_t st);
 
 }  // namespace qmm

@@ -1,6 +1,7 @@
-// Writers of the compact (batch 1) packed-activation records of qmm_common.cuh, for every
-// kernel that produces the input of a matvec: the stand-alone pack kernel, the matvec's own
-// fused epilogues, the embedding row kernel, decode attention and the tensor-parallel gather.
+// Writers of the packed-activation records of qmm_common.cuh, for every kernel that produces the
+// input of a matvec: the stand-alone pack kernel, the matvec's own fused epilogues, the embedding
+// row kernel, decode attention and the tensor-parallel gather (compact records), and the row kernels
+// of batched decode (one row of a general record at a time).
 // A 32-wide block is quantized on its own (scale = max|x| / 32639), so a producer that owns
 // 32 consecutive activations can write its block of the record without seeing the others.
 #pragma once
@@ -126,6 +127,59 @@ __device__ __forceinline__ void warp_pack_chunk(const float (&v)[8], uint8_t* re
     if (part == 0) {
         reinterpret_cast<int4*>(rec + XPK1_META)[b] =
             make_int4(8 * bsum, 128 * bsum, __float_as_int(amax / 32639.0f), 0);
+    }
+}
+
+// Row `row` of a record with ncp column groups (0: the compact record of a single row): the fragment word of
+// activations half*16 + 4t .. +3 of block b, and the block's meta entry.
+__device__ __forceinline__ uint32_t* xpack_word(uint8_t* rec, int ncp, int row, int b, int digit, int t, int half)
+{
+    const int lane = ncp == 0 ? b * 8 + 4 * digit + t : (b * ncp + (row >> 2)) * 32 + 4 * (2 * (row & 3) + digit) + t;
+    return reinterpret_cast<uint32_t*>(rec) + (lane * 2 + half);
+}
+
+__device__ __forceinline__ void xpack_meta(uint8_t* rec, int ncp, int row, int b, int q, float amax)
+{
+    int4* meta = reinterpret_cast<int4*>(rec + (ncp == 0 ? XPK1_META : xpack_xq_bytes(ncp)));
+    meta[ncp == 0 ? b : b * 16 + row] = make_int4(8 * q, 128 * q, __float_as_int(amax / 32639.0f), 0);
+}
+
+__device__ __forceinline__ size_t xpack_row_rec_bytes(int ncp)
+{
+    return ncp == 0 ? (size_t)XPK1_REC : (size_t)xpack_rec_bytes(ncp);
+}
+
+// Eight neighbouring lanes hold one 32-wide block, lane l8 of them its activations 4*l8 .. +3.  All lanes of the warp
+// take part; a group whose block does not exist passes store = false.
+__device__ __forceinline__ void pack_row_block4(const float4& v, uint8_t* rec, int ncp, int row, int b, bool store)
+{
+    const int l8 = threadIdx.x & 7;
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+    }
+    const float inv = amax > 0.0f ? 32639.0f / amax : 0.0f;
+    int hi[4], lo[4];
+    int q = quant16(v.x, inv, hi[0], lo[0]) + quant16(v.y, inv, hi[1], lo[1]) + quant16(v.z, inv, hi[2], lo[2]) +
+            quant16(v.w, inv, hi[3], lo[3]);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        q += __shfl_xor_sync(0xFFFFFFFFu, q, o);
+    }
+    if (!store) {
+        return;
+    }
+    uint32_t hw = 0u, lw = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        hw |= (uint32_t)(hi[i] & 0xFF) << (8 * i);
+        lw |= (uint32_t)(lo[i] & 0xFF) << (8 * i);
+    }
+    *xpack_word(rec, ncp, row, b, 0, l8 & 3, l8 >> 2) = hw;
+    *xpack_word(rec, ncp, row, b, 1, l8 & 3, l8 >> 2) = lw;
+    if (l8 == 0) {
+        xpack_meta(rec, ncp, row, b, q, amax);
     }
 }
 
