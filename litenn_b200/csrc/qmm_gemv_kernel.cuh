@@ -66,7 +66,7 @@ struct SmemPlan {
 template <int MC, int THREADS, int EPI>
 constexpr int gemv_min_blocks()
 {
-    return EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : MC > 1 ? 7 : (THREADS <= 256 ? 6 : 3);
+    return EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : MC > 1 ? 7 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
 }
 
 template <int FMT, int MC, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
     if constexpr (MC == 1) {
         // zero page for the lanes that carry no activation row
         uint32_t* z = reinterpret_cast<uint32_t*>(smem + Plan::X_OFF + xpack1_bytes(kc));
-        if (threadIdx.x < 128) {
-            z[threadIdx.x] = 0u;
+        for (int i = threadIdx.x; i < 128; i += NW * 32) {
+            z[i] = 0u;
         }
     }
     pdl_launch_dependents();
@@ -499,7 +499,10 @@ cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float*
 // Batch 1: warps x ring slots by row length.
 //   K of 2304..4096: eight warps with one slot each (the whole row tile is requested by the first
 //   instruction, 18 KB per CTA) measured faster than four warps with three slots for every format but
-//   Q8_0, whose larger tiles would leave fewer CTAs per SM.
+//   Q8_0, whose larger tiles would leave fewer CTAs per SM.  Inside a chain (ss_in: the input's norm factor
+//   comes from the kernel before) 4-bit rows take four warps with two slots: half the warps' prologues and
+//   reductions, 7B-shape token with eight blocks 309.7 -> 304.9 us; on its own that form gains nothing
+//   (11008 x 4096, twelve weights in turn: 92 us and 92..99).
 //   K > 4096: with four warps a warp would walk 6-28 tiles one after the other, and in a chain of
 //   dependent matvecs that walk starts only when the activations arrive; more warps per row tile
 //   shorten it, as long as two CTAs still fit on an SM.
@@ -523,6 +526,11 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         const int ctas = w.rt / 2;
         const int per_sm = (ctas + sms - 1) / sms;
         const int budget = 232448 / per_sm - 1280;
+        // 4-bit rows of up to 16 chunks: four warps with four slots, every tile requested at once (7B-shape step with eight
+        // blocks 304.9 -> 302.5 us against eight warps with one slot)
+        if (tile_bytes(FMT) == 2304 && w.kc > 8 && w.kc <= 16 && SmemPlan<FMT, 1, 4, 4, 2>::total(w.kc, 1) <= budget) {
+            return launch_gemv_variant<FMT, 1, 4, 4, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        }
         if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0 && SmemPlan<FMT, 1, 8, 1, 2>::total(w.kc, 1) <= budget) {
             return launch_gemv_variant<FMT, 1, 8, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
         }
@@ -538,6 +546,9 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         // more than one CTA per SM wanted and nothing deeper fits: one slot per warp, the number of CTAs keeps
         // the bytes in flight up
         return launch_gemv_variant<FMT, 1, 4, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
+    }
+    if (tile_bytes(FMT) == 2304 && EPI == EPI_STORE && fu.ss_in != nullptr && w.kc > 8 && w.kc <= 16) {
+        return launch_gemv_variant<FMT, 1, 4, 2, EPI>(w, xp, y, 1, status, ps, fu, stream);
     }
     if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0) {
         return launch_gemv_variant<FMT, 1, 8, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
@@ -570,9 +581,10 @@ cudaError_t launch_gemv_fmt(const WeightView& w, const XPackView& xp, float* y, 
         case EPI_STORE: return launch_gemv_m1<FMT, EPI_STORE>(w, xp, y, status, ps, fu, stream);
         case EPI_RESID_PACK: return launch_gemv_m1<FMT, EPI_RESID_PACK>(w, xp, y, status, ps, fu, stream);
         case EPI_SWIGLU: return launch_gemv_m1<FMT, EPI_SWIGLU>(w, xp, y, status, ps, fu, stream);
-        // four row tiles per CTA, two warps per tile with three slots each: 8 warps walk kc / 2 tiles apiece
-        // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together
-        case EPI_SWIGLU_PACK: return launch_gemv_variant<FMT, 1, 2, 3, EPI_SWIGLU_PACK>(w, xp, y, 1, status, ps, fu, stream);
+        // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
+        // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
+        // 7B-shape step slower)
+        case EPI_SWIGLU_PACK: return launch_gemv_variant<FMT, 1, 2, 2, EPI_SWIGLU_PACK>(w, xp, y, 1, status, ps, fu, stream);
         default: return cudaErrorInvalidValue;
         }
     }
