@@ -100,13 +100,29 @@ __global__ void unpack_x_kernel(const uint8_t* __restrict__ packed, int64_t k, f
     }
 }
 
-// fp32 -> bf16 (round to nearest even), for fp32 callers of the prefill GEMM
-__global__ void f32_to_bf16_kernel(const float* __restrict__ x, int64_t count, unsigned short* __restrict__ out)
+__device__ __forceinline__ uint32_t bf16_bits(float x)  // round to nearest even; keeps infinities and NaN
 {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t u = __float_as_uint(x[i]);
-        const uint32_t r = (u & 0x7F800000u) == 0x7F800000u ? u : u + 0x7FFFu + ((u >> 16) & 1u);  // keeps inf/nan
-        out[i] = (unsigned short)(r >> 16);
+    const uint32_t u = __float_as_uint(x);
+    return ((u & 0x7F800000u) == 0x7F800000u ? u : u + 0x7FFFu + ((u >> 16) & 1u)) >> 16;
+}
+
+// fp32 -> bf16, for fp32 callers of the prefill GEMM.  Bound by memory latency: VEC takes sixteen bytes per load, which
+// needs an aligned x (77 rows of 11008 with the product that follows: 32.8 us with single elements, 30.7 with four).
+template <bool VEC>
+__global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ x, int64_t count,
+                                                          unsigned short* __restrict__ out)
+{
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if constexpr (VEC) {
+        for (int64_t i = first; i < count / 4; i += step) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(x) + i);
+            reinterpret_cast<uint2*>(out)[i] =
+                make_uint2(bf16_bits(v.x) | (bf16_bits(v.y) << 16), bf16_bits(v.z) | (bf16_bits(v.w) << 16));
+        }
+    } else {
+        for (int64_t i = first; i < count; i += step) {
+            out[i] = (unsigned short)bf16_bits(x[i]);
+        }
     }
 }
 
@@ -114,9 +130,16 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ x, int64_t count, u
 
 cudaError_t launch_f32_to_bf16(const float* x, int64_t count, void* out_bf16, cudaStream_t stream)
 {
-    const int64_t blocks = (count + 255) / 256;
-    f32_to_bf16_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, stream>>>(x, count,
-                                                                                      static_cast<unsigned short*>(out_bf16));
+    unsigned short* out = static_cast<unsigned short*>(out_bf16);
+    const bool vec = count % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
+                     (reinterpret_cast<uintptr_t>(out_bf16) & 7u) == 0;
+    const int64_t blocks = ((vec ? count / 4 : count) + 255) / 256;
+    const unsigned grid = (unsigned)(blocks < 4096 ? blocks : 4096);
+    if (vec) {
+        f32_to_bf16_kernel<true><<<grid, 256, 0, stream>>>(x, count, out);
+    } else {
+        f32_to_bf16_kernel<false><<<grid, 256, 0, stream>>>(x, count, out);
+    }
     return cudaGetLastError();
 }
 
