@@ -227,8 +227,9 @@ int qmm_gemv_f32_static(const qmm_weight* w, const float* x_dev, float* y_dev, i
 
 /*
  * y[m,n] = x[m,k] · Wᵀ for prefill: bf16 activations, weights dequantized tile by
- * tile to bf16 in shared memory and multiplied on the tcgen05 tensor cores with
+ * tile to bf16 on the chip and multiplied on the tcgen05 tensor cores with
  * fp32 accumulation in tensor memory.  out_dtype is QMM_OUT_F32 or QMM_OUT_BF16.
+ * x must be 16-byte aligned and k a multiple of 8; y needs its elements' alignment only.
  */
 int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype,
                   void* stream);

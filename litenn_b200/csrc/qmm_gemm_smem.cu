@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         } else {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int quad = warp & 3;
+            const bool y_aligned = (reinterpret_cast<uintptr_t>(args.y) & 15u) == 0;  // a caller's y may be any element
             for (int tt = 0; tt < ntt; ++tt) {
                 const int64_t row = row_base + 128 * tt + 32 * quad + lane;
                 for (int c0 = 32 * (dw >> 2); c0 < n; c0 += 128) {
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     if (row < args.m) {
                         const int64_t col0 = (int64_t)rt0 * 16 + c0;
                         // 8 columns at a time: 16-byte (bf16) or 2 x 16-byte (fp32) stores when
-                        // the row pitch keeps them aligned, scalar stores at ragged edges
+                        // base and row pitch keep them aligned, scalar stores elsewhere and at ragged edges
                         if (args.out == GEMM_OUT_SWIGLU) {
                             // a row tile's 16 columns are 8 gates and their 8 ups
                             __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * (v.n >> 1) + (col0 >> 1);
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             }
                         } else if (args.out == GEMM_OUT_BF16) {
                             __nv_bfloat16* yo = static_cast<__nv_bfloat16*>(args.y) + row * v.n + col0;
-                            const bool vec = (v.n & 7) == 0;
+                            const bool vec = y_aligned && (v.n & 7) == 0;
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
                                 if (vec && c0 + 8 * j + 8 <= n && col0 + 8 * j + 8 <= v.n) {
@@ -360,7 +361,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                             }
                         } else {
                             float* yo = static_cast<float*>(args.y) + row * v.n + col0;
-                            const bool vec = (v.n & 3) == 0;
+                            const bool vec = y_aligned && (v.n & 3) == 0;
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
                                 if (vec && c0 + 4 * j + 4 <= n && col0 + 4 * j + 4 <= v.n) {
