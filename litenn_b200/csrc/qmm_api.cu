@@ -778,9 +778,7 @@ int qmm_gemv_f32_host(const qmm_weight* w, const float* x_host, float* y_host, i
 
 }  // extern "C"
 
-// For the decoder (llama_decoder.cu) and qmm_gemm_bf16.
-int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out, bool keep_order,
-                      void* stream)
+static int check_gemm(const qmm_weight* w, const void* x_bf16_dev, const void* y_dev, int64_t m)
 {
     if (int rc = check_weight(w, "qmm_gemm_bf16")) {
         return rc;
@@ -791,8 +789,18 @@ int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, 
     if (m < 1) {
         return fail(QMM_E_INVALID, "qmm_gemm_bf16: invalid row count %lld", (long long)m);
     }
-    if (out < 0) {
-        return fail(QMM_E_INVALID, "qmm_gemm_bf16: unknown output type");
+    return QMM_OK;
+}
+
+// For the decoder (llama_decoder.cu) and qmm_gemm_bf16.
+int qmm_internal_gemm(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out, bool keep_order,
+                      void* stream)
+{
+    if (int rc = check_gemm(w, x_bf16_dev, y_dev, m)) {
+        return rc;
+    }
+    if (out != GEMM_OUT_F32 && out != GEMM_OUT_BF16 && out != GEMM_OUT_SWIGLU) {
+        return fail(QMM_E_INVALID, "qmm_gemm_bf16: unknown output form %d", out);
     }
     DeviceGuard guard(w->device);
     if (!guard.ok) {
@@ -818,8 +826,13 @@ extern "C" {
 
 int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int64_t m, int out_dtype, void* stream)
 {
-    const int out = out_dtype == QMM_OUT_F32 ? GEMM_OUT_F32 : out_dtype == QMM_OUT_BF16 ? GEMM_OUT_BF16 : -1;
-    return qmm_internal_gemm(w, x_bf16_dev, y_dev, m, out, false, stream);
+    if (int rc = check_gemm(w, x_bf16_dev, y_dev, m)) {
+        return rc;
+    }
+    if (out_dtype != QMM_OUT_F32 && out_dtype != QMM_OUT_BF16) {
+        return fail(QMM_E_INVALID, "qmm_gemm_bf16: unknown output type %d", out_dtype);
+    }
+    return qmm_internal_gemm(w, x_bf16_dev, y_dev, m, out_dtype == QMM_OUT_BF16 ? GEMM_OUT_BF16 : GEMM_OUT_F32, false, stream);
 }
 
 int qmm_gemm_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int64_t m, void* stream_v)
