@@ -185,8 +185,7 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         bool ok = true;
         for (int s = 0; s < n_steps; ++s) {
             const int as = s % GEMM_A_STAGES;
-            ok = g_mbar_wait(&full_b[slot], phase) && g_mbar_wait(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
-            ok = __all_sync(0xFFFFFFFFu, ok);
+            ok = g_mbar_wait_warp(&full_b[slot], phase) && g_mbar_wait_warp(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
             if (!ok) {
                 if (lane == 0) {
                     atomicExch(args.status, 12);
@@ -259,13 +258,12 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
                         load_quarter<FMT>(P, next, q, lane);
                     }
                     const int as = s % GEMM_A_STAGES;
-                    if (s >= GEMM_A_STAGES && !g_mbar_wait(&empty_a[as], (uint32_t)(s / GEMM_A_STAGES - 1) & 1u)) {
+                    if (s >= GEMM_A_STAGES && !g_mbar_wait_warp(&empty_a[as], (uint32_t)(s / GEMM_A_STAGES - 1) & 1u)) {
                         if (lane == 0) {
                             atomicExch(args.status, 13);
                         }
                         ok = false;
                     }
-                    ok = __all_sync(0xFFFFFFFFu, ok);
                     if (ok) {
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         if (has) {
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         }
 
         // ---- epilogue: D has one weight row per lane, one token per column ----
-        if (!g_mbar_wait(accum, 0)) {
+        if (!g_mbar_wait_warp(accum, 0)) {
             if (lane == 0) {
                 atomicExch(args.status, 14);
             }

@@ -59,6 +59,13 @@ __device__ __forceinline__ bool g_mbar_wait(uint64_t* bar, uint32_t parity)
     return false;
 }
 
+// The same for a whole converged warp, which goes on together: what follows may be a warp-wide tcgen05 instruction, and
+// lanes that gave up on their own would leave the others without them.
+__device__ __forceinline__ bool g_mbar_wait_warp(uint64_t* bar, uint32_t parity)
+{
+    return __all_sync(0xFFFFFFFFu, g_mbar_wait(bar, parity));
+}
+
 // True in one lane of a converged warp.  MMAs are issued under this and not under a lane comparison: the compiler then
 // knows that their operands are uniform.
 __device__ __forceinline__ bool elect_one()

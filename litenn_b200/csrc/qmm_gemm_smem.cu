@@ -208,8 +208,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         for (int s = 0; s < n_stages; ++s) {
             const int slot = s % GEMM_STAGES;
             const uint32_t parity = (uint32_t)(s / GEMM_STAGES) & 1u;
-            ok = g_mbar_wait(&full_a[slot], parity) && g_mbar_wait(&full_b[slot], parity);
-            ok = __all_sync(0xFFFFFFFFu, ok);
+            ok = g_mbar_wait_warp(&full_a[slot], parity) && g_mbar_wait_warp(&full_b[slot], parity);
             if (!ok) {
                 if (lane == 0) {
                     atomicExch(args.status, 12);
@@ -304,7 +303,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
 
         // ---- epilogue: a warp reaches TMEM lanes 32*(warp%4).., four warps share them by columns ----
-        if (!g_mbar_wait(accum, 0)) {
+        if (!g_mbar_wait_warp(accum, 0)) {
             if (lane == 0) {
                 atomicExch(args.status, 14);
             }
