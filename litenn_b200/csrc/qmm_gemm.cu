@@ -398,79 +398,6 @@ EncodeTiledFn encode_tiled_fn()
     return fn;
 }
 
-// How one product is cut: NB blocks of 128 weight rows and `tokens` activation rows per CTA, `splits` CTAs along K; or,
-// with groups > 0, the shared-memory kernel with that many CTAs per 256 tokens.
-struct GemmPlan {
-    int nb, tokens, t_tiles, splits, ring, grid, smem, groups;
-};
-
-// Three shapes of CTA, and the one with the least estimated time wins.
-//   NB = 2    one CTA per SM, each token tile read once for 256 weight rows
-//   NB = 1    two CTAs per SM; cuts finer and can split K over a cluster: few tokens or few weight rows
-//   shared memory (qmm_gemm_smem.cu)   one dequantization per 256 tokens instead of 128: many tokens, where the
-//             dequantization is what the other two spend their time on
-// The estimates are microseconds on a B200: waves of CTAs x steps of 64 columns x time per step, plus a start-up per
-// wave, fitted to 100 (weight, token count) pairs from 512 x 1024 to 8192 x 28672 and 17 to 1999 tokens, over which the
-// choice costs 2 % against the best of all shapes.  Some of them (us): Q4_0 4096 x 4096, 64 tokens: NB = 1 with K split
-// in four 14.7, shared memory 43.3; 1024 tokens: NB = 2 45.2, shared memory 57.4; 1999 tokens: NB = 2 85.6, shared
-// memory 71.8.  Q6_K 8192 x 28672, 128 tokens: NB = 1 90.8, shared memory 327; 1024 tokens: 588 and 444.
-//
-// keep_order asks for the shared-memory form, whose sums run over K in one fixed order per row tile; the other two add the
-// K splits of a tile and start elsewhere, which changes the last bits.
-GemmPlan plan_gemm(const WeightView& w, int64_t m, int sm_count, bool keep_order)
-{
-    GemmPlan best = {};
-    const int64_t steps = (w.k + GEMM_BK - 1) / GEMM_BK;
-    const auto waves = [](int64_t ctas, int64_t slots) { return (double)((ctas + slots - 1) / slots); };
-    best.groups = gemm_smem_groups(w.rt, m, sm_count);
-    best.grid = (int)((m + 255) / 256) * best.groups;
-    const double tiles_per_cta = (double)((w.rt + best.groups - 1) / best.groups);
-    double best_cost = waves(best.grid, sm_count) * (4.0 * w.kc * (0.57 + 0.026 * tiles_per_cta) + 9.2);
-    if (keep_order) {
-        return best;
-    }
-    const int64_t min_tiles = (m + GEMM_MAX_TOKENS - 1) / GEMM_MAX_TOKENS;
-    for (int64_t tt = min_tiles; tt <= min_tiles + 1; ++tt) {
-        const int64_t tokens = ((m + tt - 1) / tt + 15) / 16 * 16;
-        const int64_t t_tiles = (m + tokens - 1) / tokens;
-        const double fill = (double)tokens / GEMM_MAX_TOKENS;
-        for (int nb = 1; nb <= 2; ++nb) {
-            const int64_t tiles = ((w.rt + 8 * nb - 1) / (8 * nb)) * t_tiles;
-            for (int splits = 1; splits <= (nb == 1 ? 8 : 1) && splits <= w.kc; splits *= 2) {
-                const int64_t ctas = tiles * splits;
-                double cost;
-                if (nb == 2) {
-                    cost = waves(ctas, sm_count) * (steps * (0.481 + 0.15 * fill) + 7.1);
-                } else {
-                    // two CTAs per SM; a last round that leaves most SMs with one runs its steps faster
-                    const double st = (double)((steps + splits - 1) / splits);
-                    const double paired = st * (0.615 + 0.104 * fill) + 6.7, alone = st * (0.385 + 0.034 * fill) + 6.7;
-                    const int64_t rounds = ctas / (2 * sm_count), rest = ctas % (2 * sm_count);
-                    cost = rounds * paired + (rest > sm_count ? paired : rest > 0 ? alone : 0.0) + (splits > 1 ? 4.2 : 0.0);
-                }
-                if (cost < best_cost) {
-                    best_cost = cost;
-                    best.groups = 0;
-                    best.nb = nb;
-                    best.tokens = (int)tokens;
-                    best.t_tiles = (int)t_tiles;
-                    best.splits = splits;
-                    best.grid = (int)ctas;
-                }
-            }
-        }
-    }
-    if (best.groups > 0) {
-        return best;
-    }
-    const int room = best.nb == 2 ? 200 * 1024 : 110 * 1024;
-    best.ring = std::min(GEMM_MAX_RING, room / (best.tokens * 128));
-    const int ring_bytes = best.ring * best.tokens * 128;
-    const int part_bytes = best.splits > 1 ? best.tokens * 128 * 4 : 0;
-    best.smem = 1024 /*alignment*/ + GEMM_BAR_BYTES + std::max(ring_bytes, part_bytes);
-    return best;
-}
-
 template <int FMT, int NB>
 cudaError_t launch_gemm_nb(const CUtensorMap& xmap, const GemmArgs& args, const GemmPlan& plan, cudaStream_t stream)
 {
@@ -518,9 +445,86 @@ cudaError_t launch_gemm_fmt(const CUtensorMap& xmap, const GemmArgs& args, const
 
 }  // namespace
 
+GemmPlan gemm_form(const WeightView& w, int64_t m, int sm_count, int nb, int tokens, int splits)
+{
+    GemmPlan p = {};
+    if (nb == 0) {
+        p.groups = gemm_smem_groups(w.rt, m, sm_count);
+        p.grid = (int)((m + 255) / 256) * p.groups;
+        return p;
+    }
+    p.nb = nb;
+    p.tokens = tokens;
+    p.t_tiles = (int)((m + tokens - 1) / tokens);
+    p.splits = splits;
+    p.grid = (w.rt + 8 * nb - 1) / (8 * nb) * p.t_tiles * splits;
+    const int room = nb == 2 ? 200 * 1024 : 110 * 1024;
+    p.ring = std::min(GEMM_MAX_RING, room / (tokens * 128));
+    const int part_bytes = splits > 1 ? tokens * 128 * 4 : 0;
+    p.smem = 1024 /*alignment*/ + GEMM_BAR_BYTES + std::max(p.ring * tokens * 128, part_bytes);
+    return p;
+}
+
+// Three shapes of CTA, and the one with the least estimated time wins.
+//   NB = 2    one CTA per SM, each token tile read once for 256 weight rows
+//   NB = 1    two CTAs per SM; cuts finer and can split K over a cluster: few tokens or few weight rows
+//   shared memory (qmm_gemm_smem.cu)   one dequantization per 256 tokens instead of 128: many tokens, where the
+//             dequantization is what the other two spend their time on
+// The estimates are microseconds on a B200: waves of CTAs x steps of 64 columns x time per step, plus a start-up per
+// wave, fitted to 100 (weight, token count) pairs from 512 x 1024 to 8192 x 28672 and 17 to 1999 tokens, over which the
+// choice costs 2 % against the best of all shapes.  Some of them (us): Q4_0 4096 x 4096, 64 tokens: NB = 1 with K split
+// in four 14.7, shared memory 43.3; 1024 tokens: NB = 2 45.2, shared memory 57.4; 1999 tokens: NB = 2 85.6, shared
+// memory 71.8.  Q6_K 8192 x 28672, 128 tokens: NB = 1 90.8, shared memory 327; 1024 tokens: 588 and 444.
+//
+// keep_order asks for the shared-memory form, whose sums run over K in one fixed order per row tile; the other two add the
+// K splits of a tile and start elsewhere, which changes the last bits.
+GemmPlan plan_gemm(const WeightView& w, int64_t m, int sm_count, bool keep_order)
+{
+    GemmPlan best = gemm_form(w, m, sm_count, 0, 0, 1);
+    const int64_t steps = (w.k + GEMM_BK - 1) / GEMM_BK;
+    const auto waves = [](int64_t ctas, int64_t slots) { return (double)((ctas + slots - 1) / slots); };
+    const double tiles_per_cta = (double)((w.rt + best.groups - 1) / best.groups);
+    double best_cost = waves(best.grid, sm_count) * (4.0 * w.kc * (0.57 + 0.026 * tiles_per_cta) + 9.2);
+    if (keep_order) {
+        return best;
+    }
+    const int64_t min_tiles = (m + GEMM_MAX_TOKENS - 1) / GEMM_MAX_TOKENS;
+    for (int64_t tt = min_tiles; tt <= min_tiles + 1; ++tt) {
+        const int64_t tokens = ((m + tt - 1) / tt + 15) / 16 * 16;
+        const int64_t t_tiles = (m + tokens - 1) / tokens;
+        const double fill = (double)tokens / GEMM_MAX_TOKENS;
+        for (int nb = 1; nb <= 2; ++nb) {
+            const int64_t tiles = ((w.rt + 8 * nb - 1) / (8 * nb)) * t_tiles;
+            for (int splits = 1; splits <= (nb == 1 ? 8 : 1) && splits <= w.kc; splits *= 2) {
+                const int64_t ctas = tiles * splits;
+                double cost;
+                if (nb == 2) {
+                    cost = waves(ctas, sm_count) * (steps * (0.481 + 0.15 * fill) + 7.1);
+                } else {
+                    // two CTAs per SM; a last round that leaves most SMs with one runs its steps faster
+                    const double st = (double)((steps + splits - 1) / splits);
+                    const double paired = st * (0.615 + 0.104 * fill) + 6.7, alone = st * (0.385 + 0.034 * fill) + 6.7;
+                    const int64_t rounds = ctas / (2 * sm_count), rest = ctas % (2 * sm_count);
+                    cost = rounds * paired + (rest > sm_count ? paired : rest > 0 ? alone : 0.0) + (splits > 1 ? 4.2 : 0.0);
+                }
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = gemm_form(w, m, sm_count, nb, (int)tokens, splits);
+                }
+            }
+        }
+    }
+    return best;
+}
 
 cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out, bool keep_order,
                              int sm_count, int* status, cudaStream_t stream, const char** why)
+{
+    return launch_gemm_plan(plan_gemm(w, m, sm_count, keep_order), w, x_bf16, y, m, out, keep_order, status, stream, why);
+}
+
+cudaError_t launch_gemm_plan(const GemmPlan& plan, const WeightView& w, const void* x_bf16, void* y, int64_t m, int out,
+                             bool keep_order, int* status, cudaStream_t stream, const char** why)
 {
     *why = nullptr;
     EncodeTiledFn encode = encode_tiled_fn();
@@ -536,7 +540,6 @@ cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, i
         *why = "a gate|up product needs whole 16-row tiles and a 16-byte aligned result";
         return cudaErrorInvalidValue;
     }
-    const GemmPlan plan = plan_gemm(w, m, sm_count, keep_order);
     CUtensorMap xmap;
     const cuuint64_t dims[2] = {(cuuint64_t)w.k, (cuuint64_t)m};
     const cuuint64_t strides[1] = {(cuuint64_t)w.k * 2};

@@ -45,4 +45,16 @@ constexpr int GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2;
 cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out, bool keep_order,
                              int sm_count, int* status, cudaStream_t stream, const char** why);
 
+// How launch_gemm_bf16 cuts one product: NB blocks of 128 weight rows and `tokens` activation rows per CTA, `splits` CTAs
+// along K; or, with groups > 0, the shared-memory kernel with that many CTAs per 256 tokens.
+struct GemmPlan {
+    int nb, tokens, t_tiles, splits, ring, grid, smem, groups;
+};
+GemmPlan plan_gemm(const WeightView& w, int64_t m, int sm_count, bool keep_order);
+// The plan of one form, for plan_gemm and for tests that walk every form: nb 1 or 2 with `tokens` a multiple of 16 up to
+// 128 and splits 1, 2, 4 or 8 up to the weight's K chunks (nb 2: 1); nb 0 is the shared-memory form.
+GemmPlan gemm_form(const WeightView& w, int64_t m, int sm_count, int nb, int tokens, int splits);
+cudaError_t launch_gemm_plan(const GemmPlan& plan, const WeightView& w, const void* x_bf16, void* y, int64_t m, int out,
+                             bool keep_order, int* status, cudaStream_t stream, const char** why);
+
 }  // namespace qmm

@@ -1,7 +1,8 @@
 """The prefill GEMM's CTA shapes at their edges: K split over a cluster of 2, 4 or 8, one or two blocks of 128 weight rows
 per CTA, and the shared-memory form; row counts around the 16-token granule and the 128- and 256-token tiles, weight
 rows that end inside a 16-row tile, K that ends inside a 256-wide chunk.  The shapes are sized so that the dispatch
-reaches the named form on a 148-SM part; on another part they still have to be right."""
+reaches the named form on a 148-SM part (test_gemm_plan.py holds it to that); on another part they still have to be
+right."""
 import numpy as np
 import pytest
 
@@ -15,7 +16,7 @@ CASES = [
     # form, m, n, k (k is rounded to whole super-blocks for the K-quants)
     ("one CTA per tile", 17, 3, 32),
     ("split", 16, 40, 1056), ("split", 33, 129, 1024), ("split", 128, 1000, 2080), ("split", 129, 250, 2048),
-    ("split, two token tiles", 250, 520, 1312),
+    ("split, several token tiles", 250, 520, 1312),
     ("two blocks", 131, 12291, 288), ("two blocks", 145, 14344, 256),
     ("shared memory", 257, 14347, 288), ("shared memory", 700, 8193, 256), ("shared memory", 2050, 2305, 544),
 ]
