@@ -810,232 +810,40 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// Two fp32 values as a sum of two fp16 pairs: hi + lo holds 22 bits of each.
-__device__ __forceinline__ void split_f16x2(float a, float b, uint32_t& hi, uint32_t& lo)
+// Two fp32 values as sums of N fp16 parts, the largest first.  fp16 ends at 2^-24: three parts hold every bit of a value
+// of at least 1/2, of smaller ones what lies above that.
+template <int N>
+__device__ __forceinline__ void split_f16x2(float a, float b, uint32_t (&o)[N])
 {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 hf = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - hf.x, b - hf.y);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
-
-// Causal attention over the fp16 cache for rows 0..m-1 at positions pos0+row, on the tensor cores.  A CTA owns 64
-// query rows of one head (16 per warp) and walks the keys in tiles of 64, which cp.async brings into shared memory one
-// tile ahead; online softmax per row, output bf16 ctx[m][n_heads*hd].
-// Queries and probabilities are fp32 and stay that precise: each goes through the fp16 MMA as hi + lo, two passes over
-// the same key or value fragment (K and V are fp16, so those are exact).  A power of two per row keeps the split away
-// from fp16's range limits: the row's largest query value is brought to 2^14..2^15, probabilities are taken times 2^14.
-// Masked keys get probability 0, but their V rows do take part in the product: a value that overflowed fp16 reaches the
-// earlier rows of its 64-row group too.  The prompt's last row and every later token see it in any case.
-// Bound: the MMA pipe (twice the flops of a one-pass product).  Four rows per warp with fp32 arithmetic and shuffles were
-// issue-bound: a 1999-token prompt through four blocks of the 7B shape took 19.3 ms with that, 6.0 ms with this; error
-// of the logits against 64 bits the same (1.8e-5 at 300 and 701 tokens).
-template <int HD>
-__global__ void __launch_bounds__(128) attn_prefill_kernel(const float* __restrict__ qkv, int row_stride, int m,
-                                                           int pos0, int n_heads, int n_kv, int max_seq,
-                                                           const __half* __restrict__ cache_k,
-                                                           const __half* __restrict__ cache_v,
-                                                           __nv_bfloat16* __restrict__ ctx)
-{
-    constexpr int KT = 64;                 // keys per tile
-    constexpr int ROW = HD * 2;            // bytes of a key row
-    constexpr int CH = ROW / 16;           // 16-byte pieces of it; piece c of row r sits at c ^ (r & 7)
-    constexpr int TILE = KT * ROW;
-    constexpr float P_SCALE = 16384.0f;
-    extern __shared__ __align__(128) uint8_t att_smem[];  // [2 buffers][K tile | V tile]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int head = blockIdx.y, kvh = head / (n_heads / n_kv);
-    const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 64;  // the longest rows first
-    const int n_keys = pos0 + min(row0 + 64, m);                   // keys the last row of this CTA sees
-    const int tiles = (n_keys + KT - 1) / KT;
-    const __half* kb = cache_k + (int64_t)kvh * max_seq * HD;
-    const __half* vb = cache_v + (int64_t)kvh * max_seq * HD;
-
-    auto fetch = [&](int tile) {
-        const uint32_t dst = smem_addr(att_smem) + (tile & 1) * 2 * TILE;
 #pragma unroll
-        for (int i = 0; i < KT * CH / 128; ++i) {
-            const int idx = threadIdx.x + i * 128;
-            const int r = idx / CH, c = idx % CH;
-            const int key = min(tile * KT + r, n_keys - 1);  // beyond the last key: any row that exists
-            const uint32_t o = dst + r * ROW + ((c ^ (r & 7)) * 16);
-            cp_async16(o, kb + (int64_t)key * HD + c * 8);
-            cp_async16(o + TILE, vb + (int64_t)key * HD + c * 8);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch(0);
-
-    // this thread's rows of the warp's 16: g and g + 8
-    int rows[2];
-    uint32_t qh[HD / 16][4], ql[HD / 16][4];
-    float unscale[2];
-    {
-        const float scale = rsqrtf((float)HD);
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-            rows[rs] = row0 + warp * 16 + g + 8 * rs;
-            const float* q = qkv + (int64_t)min(rows[rs], m - 1) * row_stride + head * HD + 2 * t;
-            float2 x[HD / 8];
-            float amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < HD / 8; ++i) {
-                x[i] = *reinterpret_cast<const float2*>(q + 8 * i);
-                x[i].x *= scale;
-                x[i].y *= scale;
-                amax = fmaxf(amax, fmaxf(fabsf(x[i].x), fabsf(x[i].y)));
-            }
-            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
-            int e = (int)((__float_as_uint(amax) >> 23) & 255u) - 127;
-            e = e == 128 ? 14 : max(e, -100);  // infinities and NaN stay what they are
-            const float up = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
-            unscale[rs] = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
-#pragma unroll
-            for (int i = 0; i < HD / 16; ++i) {
-                split_f16x2(x[2 * i].x * up, x[2 * i].y * up, qh[i][rs], ql[i][rs]);
-                split_f16x2(x[2 * i + 1].x * up, x[2 * i + 1].y * up, qh[i][2 + rs], ql[i][2 + rs]);
-            }
-        }
-    }
-    float acc[HD / 8][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int j = 0; j < HD / 8; ++j) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            acc[j][i] = 0.0f;
-        }
-    }
-
-    for (int tile = 0; tile < tiles; ++tile) {
-        if (tile + 1 < tiles) {
-            fetch(tile + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const uint32_t ks = smem_addr(att_smem) + (tile & 1) * 2 * TILE, vs = ks + TILE;
-
-        // scores of 16 rows x 64 keys
-        float sc[KT / 8][4];
-#pragma unroll
-        for (int j = 0; j < KT / 8; ++j) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                sc[j][i] = 0.0f;
-            }
-            const int r = 8 * j + (lane & 7);
-#pragma unroll
-            for (int k2 = 0; k2 < HD / 32; ++k2) {
-                uint32_t b[4];
-                ldmatrix_x4(b, ks + r * ROW + (((4 * k2 + (lane >> 3)) ^ (r & 7)) * 16));
-                mma_f16(sc[j], qh[2 * k2], b[0], b[1]);
-                mma_f16(sc[j], ql[2 * k2], b[0], b[1]);
-                mma_f16(sc[j], qh[2 * k2 + 1], b[2], b[3]);
-                mma_f16(sc[j], ql[2 * k2 + 1], b[2], b[3]);
-            }
-        }
-        const bool masked = tile * KT + KT - 1 > pos0 + row0 + warp * 16;  // some row of the warp ends inside the tile
-        float corr[2], sum[2] = {0.0f, 0.0f};
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-            float mb = mx[rs];
-#pragma unroll
-            for (int j = 0; j < KT / 8; ++j) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    float& s = sc[j][2 * rs + i];
-                    s *= unscale[rs];
-                    if (masked && tile * KT + 8 * j + 2 * t + i > pos0 + rows[rs]) {
-                        s = -INFINITY;
-                    }
-                    mb = fmaxf(mb, s);
-                }
-            }
-            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 1));
-            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 2));
-            corr[rs] = __expf(mx[rs] - mb);
-            mx[rs] = mb;
-#pragma unroll
-            for (int j = 0; j < KT / 8; ++j) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const float p = __expf(sc[j][2 * rs + i] - mb);
-                    sum[rs] += p;
-                    sc[j][2 * rs + i] = p * P_SCALE;
-                }
-            }
-            l[rs] = l[rs] * corr[rs] + sum[rs];
-        }
-#pragma unroll
-        for (int j = 0; j < HD / 8; ++j) {
-            acc[j][0] *= corr[0];
-            acc[j][1] *= corr[0];
-            acc[j][2] *= corr[1];
-            acc[j][3] *= corr[1];
-        }
-        // probabilities times V: the score fragments are the A operand as they lie
-#pragma unroll
-        for (int kk = 0; kk < KT / 16; ++kk) {
-            uint32_t ph[4], pl[4];
-            split_f16x2(sc[2 * kk][0], sc[2 * kk][1], ph[0], pl[0]);
-            split_f16x2(sc[2 * kk][2], sc[2 * kk][3], ph[1], pl[1]);
-            split_f16x2(sc[2 * kk + 1][0], sc[2 * kk + 1][1], ph[2], pl[2]);
-            split_f16x2(sc[2 * kk + 1][2], sc[2 * kk + 1][3], ph[3], pl[3]);
-            const int r = 16 * kk + ((lane >> 3) & 1) * 8 + (lane & 7);
-#pragma unroll
-            for (int j2 = 0; j2 < HD / 16; ++j2) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, vs + r * ROW + (((2 * j2 + (lane >> 4)) ^ (r & 7)) * 16));
-                mma_f16(acc[2 * j2], ph, b[0], b[1]);
-                mma_f16(acc[2 * j2 + 1], ph, b[2], b[3]);
-                mma_f16(acc[2 * j2], pl, b[0], b[1]);
-                mma_f16(acc[2 * j2 + 1], pl, b[2], b[3]);
-            }
-        }
-        __syncthreads();  // the buffer is refilled two tiles from now
-    }
-#pragma unroll
-    for (int rs = 0; rs < 2; ++rs) {
-        float tot = l[rs];
-        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 1);
-        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 2);
-        tot *= P_SCALE;
-        if (rows[rs] < m) {
-            __nv_bfloat16* out = ctx + (int64_t)rows[rs] * n_heads * HD + head * HD + 2 * t;
-#pragma unroll
-            for (int j = 0; j < HD / 8; ++j) {
-                *reinterpret_cast<__nv_bfloat162*>(out + 8 * j) =
-                    __floats2bfloat162_rn(acc[j][2 * rs] / tot, acc[j][2 * rs + 1] / tot);
-            }
-        }
+    for (int i = 0; i < N; ++i) {
+        const __half2 h = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(h);
+        a -= f.x;
+        b -= f.y;
+        o[i] = *reinterpret_cast<const uint32_t*>(&h);
     }
 }
 
-// Causal attention for a few rows, with fp32 arithmetic throughout: a 64-row tile of the kernel above would be mostly
-// padding.  Bound by the L2
-// reads of K and V (every row streams the whole prefix of its head), so one warp serves ROWS consecutive rows of
-// one head and reuses each loaded batch of eight keys for all of them; a row simply ignores the keys beyond its
-// own position.  Online softmax per row, one rescale per batch; output bf16 ctx[m][n_heads*hd].
-template <int DPL, int ROWS>
-__global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __restrict__ qkv, int row_stride, int m,
-                                                           int pos0, int n_heads, int n_kv, int max_seq,
-                                                           const __half* __restrict__ cache_k,
-                                                           const __half* __restrict__ cache_v,
-                                                           __nv_bfloat16* __restrict__ ctx)
+__device__ __forceinline__ void store_ctx(__nv_bfloat16* p, float a, float b)
+{
+    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
+}
+__device__ __forceinline__ void store_ctx(float* p, float a, float b)  // tests look at the sums before they are rounded
+{
+    *reinterpret_cast<float2*>(p) = make_float2(a, b);
+}
+
+// Causal attention for rows row0..row0+ROWS-1 of one head (those below m) by one warp, fp32 arithmetic throughout: it
+// reuses each loaded batch of eight keys for all of its rows; a row simply ignores the keys beyond its own position.
+// Online softmax per row, one rescale per batch.
+template <int DPL, int ROWS, typename OutT>
+__device__ __forceinline__ void attn_rows(const float* __restrict__ qkv, int row_stride, int m, int pos0, int n_heads,
+                                          int n_kv, int max_seq, const __half* __restrict__ cache_k,
+                                          const __half* __restrict__ cache_v, OutT* __restrict__ ctx, int row0, int head)
 {
     constexpr int hd = 32 * DPL;
     const int lane = threadIdx.x & 31;
-    const int groups = (m + ROWS - 1) / ROWS;
-    const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (wid >= (int64_t)groups * n_heads) {
-        return;
-    }
-    // the longest rows first: the last CTAs to start are the shortest
-    const int row0 = (groups - 1 - (int)(wid / n_heads)) * ROWS, head = (int)(wid % n_heads);
     const int kvh = head / (n_heads / n_kv);
     const float scale = rsqrtf((float)hd);
     float qv[ROWS][DPL], acc[ROWS][DPL], mx[ROWS], l[ROWS];
@@ -1077,12 +885,335 @@ __global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __r
     for (int r = 0; r < ROWS; ++r) {
         if (row0 + r < m) {
 #pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                ctx[(int64_t)(row0 + r) * n_heads * hd + head * hd + lane * DPL + i] =
-                    __float2bfloat16_rn(acc[r][i] / l[r]);
+            for (int i = 0; i < DPL; i += 2) {
+                store_ctx(ctx + (int64_t)(row0 + r) * n_heads * hd + head * hd + lane * DPL + i, acc[r][i] / l[r],
+                          acc[r][i + 1] / l[r]);
             }
         }
     }
+}
+
+// Sixteen rows again, for attn_prefill_kernel; kept out of line, so that its registers are not that kernel's.
+template <int HD, typename OutT>
+__device__ __noinline__ void attn_rows_again(const float* qkv, int row_stride, int m, int pos0, int n_heads, int n_kv,
+                                             int max_seq, const __half* cache_k, const __half* cache_v, OutT* ctx, int row0,
+                                             int head)
+{
+    for (int r = row0; r < min(row0 + 16, m); r += 4) {
+        attn_rows<HD / 32, 4>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx, r, head);
+    }
+}
+
+// Causal attention over the fp16 cache for rows 0..m-1 at positions pos0+row, on the tensor cores.  A CTA owns 64
+// query rows of one head (16 per warp) and walks the keys in tiles of 64, which cp.async brings into shared memory one
+// tile ahead; online softmax per row, output bf16 ctx[m][n_heads*hd].
+// Queries and probabilities are fp32 and go through the fp16 MMA in parts (K and V are fp16, so those are exact): a query
+// as three parts, which hold all of its bits, a probability as two, which hold 23.  A power of two per row keeps the
+// split away from fp16's range limits: the row's largest query value is brought to 2^14..2^15, probabilities are taken
+// times 2^14.  The MMA truncates what it adds, so its chains are kept short and start with the smallest parts: 32
+// dimensions of a score, one tile of keys of a context value; fp32 additions, which round, put these together.
+// Error against 64 bits before the rounding to bf16 (2-norm, 300 / 1999 tokens, HD 128, scores of about 1): 1.6e-7 /
+// 1.4e-7 here, 2.1e-7 / 6.2e-7 in the fp32 row kernel below; two parts and one chain for everything had 5.5e-7 / 2.9e-6.
+// Scores of about 16: 4.1e-7 / 5.3e-7, 4.2e-7 / 5.4e-7 and 1.3e-6 / 1.6e-6.
+// Bound: the MMA pipe, 16 cycles per m16n8k16 and scheduler, five MMAs where plain fp16 takes two.  1999 rows, 32 heads,
+// HD 128: 309 us, 272 with two parts of a query, 247 with two parts and long chains.  Four rows per warp with fp32
+// arithmetic and shuffles are issue-bound: 512 rows 250 us against 40.
+// A masked key's V row takes part in the product with probability 0, and a query or a key that overflowed fp16 meets the
+// parts one by one, so infinities and NaN spread further here than they should.  They always leave a mark on the row's own
+// sums, and a warp that finds one does its rows again in fp32, key by key.
+template <int HD, typename OutT>
+__global__ void __launch_bounds__(128, HD == 128 ? 2 : 3)  // what its shared memory lets an SM hold at HD = 128
+    attn_prefill_kernel(const float* __restrict__ qkv, int row_stride, int m,
+                                                           int pos0, int n_heads, int n_kv, int max_seq,
+                                                           const __half* __restrict__ cache_k,
+                                                           const __half* __restrict__ cache_v, OutT* __restrict__ ctx)
+{
+    constexpr int KT = 64;                 // keys per tile
+    constexpr int ROW = HD * 2;            // bytes of a key row
+    constexpr int CH = ROW / 16;           // 16-byte pieces of it; piece c of row r sits at c ^ (r & 7)
+    constexpr int TILE = KT * ROW;
+    constexpr int KS = HD / 16;            // k steps of a score
+    constexpr int QP = 3, PP = 2;          // parts of a query and of a probability
+    constexpr int KG = 2, JG = 2;          // k steps of one MMA chain, 16-wide column groups of V at a time
+    constexpr float P_SCALE = 16384.0f;
+    extern __shared__ __align__(128) uint8_t att_smem[];  // [2 buffers][K tile | V tile], query fragments
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int head = blockIdx.y, kvh = head / (n_heads / n_kv);
+    const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 64;  // the longest rows first
+    const int n_keys = pos0 + min(row0 + 64, m);                   // keys the last row of this CTA sees
+    const int tiles = (n_keys + KT - 1) / KT;
+    const __half* kb = cache_k + (int64_t)kvh * max_seq * HD;
+    const __half* vb = cache_v + (int64_t)kvh * max_seq * HD;
+
+    auto fetch = [&](int tile) {
+        const uint32_t dst = smem_addr(att_smem) + (tile & 1) * 2 * TILE;
+#pragma unroll
+        for (int i = 0; i < KT * CH / 128; ++i) {
+            const int idx = threadIdx.x + i * 128;
+            const int r = idx / CH, c = idx % CH;
+            const int key = min(tile * KT + r, n_keys - 1);  // beyond the last key: any row that exists
+            const uint32_t o = dst + r * ROW + ((c ^ (r & 7)) * 16);
+            cp_async16(o, kb + (int64_t)key * HD + c * 8);
+            cp_async16(o + TILE, vb + (int64_t)key * HD + c * 8);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+
+    // this thread's rows of the warp's 16: g and g + 8; their A fragments wait in shared memory, where only this thread
+    // reads them: [part][k step][lane]
+    int rows[2];
+    uint4* qfrag = reinterpret_cast<uint4*>(att_smem + 4 * TILE) + warp * (QP * KS * 32) + lane;
+    float unscale[2];
+    {
+        const float scale = rsqrtf((float)HD);
+        float2 x[2][HD / 8];
+#pragma unroll
+        for (int rs = 0; rs < 2; ++rs) {
+            rows[rs] = row0 + warp * 16 + g + 8 * rs;
+            const float* q = qkv + (int64_t)min(rows[rs], m - 1) * row_stride + head * HD + 2 * t;
+            float amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < HD / 8; ++i) {
+                x[rs][i] = *reinterpret_cast<const float2*>(q + 8 * i);
+                x[rs][i].x *= scale;
+                x[rs][i].y *= scale;
+                amax = fmaxf(amax, fmaxf(fabsf(x[rs][i].x), fabsf(x[rs][i].y)));
+            }
+            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
+            const int e = max((int)((__float_as_uint(amax) >> 23) & 255u) - 127, -100);
+            const float up = __uint_as_float((uint32_t)(127 + 14 - e) << 23);
+            unscale[rs] = __uint_as_float((uint32_t)(127 - 14 + e) << 23);
+#pragma unroll
+            for (int i = 0; i < HD / 8; ++i) {
+                x[rs][i].x *= up;
+                x[rs][i].y *= up;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            uint32_t a[4][QP];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 v = x[i & 1][2 * k + (i >> 1)];
+                split_f16x2<QP>(v.x, v.y, a[i]);
+            }
+#pragma unroll
+            for (int p = 0; p < QP; ++p) {
+                qfrag[(p * KS + k) * 32] = make_uint4(a[0][p], a[1][p], a[2][p], a[3][p]);
+            }
+        }
+    }
+    float acc[HD / 8][4], mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < HD / 8; ++j) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            acc[j][i] = 0.0f;
+        }
+    }
+
+    for (int tile = 0; tile < tiles; ++tile) {
+        if (tile + 1 < tiles) {
+            fetch(tile + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const uint32_t ks = smem_addr(att_smem) + (tile & 1) * 2 * TILE, vs = ks + TILE;
+
+        // scores of 16 rows x 64 keys
+        float sc[KT / 8][4];
+#pragma unroll
+        for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                sc[j][i] = 0.0f;
+            }
+        }
+#pragma unroll
+        for (int k0 = 0; k0 < KS; k0 += KG) {
+            uint32_t b[KG][KT / 16][4];
+#pragma unroll
+            for (int kg = 0; kg < KG; ++kg) {
+#pragma unroll
+                for (int j2 = 0; j2 < KT / 16; ++j2) {
+                    const int r = 16 * j2 + (lane >> 4) * 8 + (lane & 7);
+                    ldmatrix_x4(b[kg][j2], ks + r * ROW + (((2 * (k0 + kg) + ((lane >> 3) & 1)) ^ (r & 7)) * 16));
+                }
+            }
+            float d[KT / 8][4] = {};
+#pragma unroll
+            for (int p = QP - 1; p >= 0; --p) {
+#pragma unroll
+                for (int kg = 0; kg < KG; ++kg) {
+                    const uint4 v = qfrag[(p * KS + k0 + kg) * 32];
+                    const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int j = 0; j < KT / 8; ++j) {
+                        mma_f16(d[j], q, b[kg][j >> 1][2 * (j & 1)], b[kg][j >> 1][2 * (j & 1) + 1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    sc[j][i] += d[j][i];
+                }
+            }
+        }
+        const bool masked = tile * KT + KT - 1 > pos0 + row0 + warp * 16;  // some row of the warp ends inside the tile
+        float corr[2], sum[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int rs = 0; rs < 2; ++rs) {
+            float mb = mx[rs];
+#pragma unroll
+            for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float& s = sc[j][2 * rs + i];
+                    s *= unscale[rs];
+                    if (masked && tile * KT + 8 * j + 2 * t + i > pos0 + rows[rs]) {
+                        s = -INFINITY;
+                    }
+                    mb = fmaxf(mb, s);
+                }
+            }
+            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 1));
+            mb = fmaxf(mb, __shfl_xor_sync(0xFFFFFFFFu, mb, 2));
+            corr[rs] = __expf(mx[rs] - mb);
+            mx[rs] = mb;
+#pragma unroll
+            for (int j = 0; j < KT / 8; ++j) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float p = __expf(sc[j][2 * rs + i] - mb);
+                    sum[rs] += p;
+                    sc[j][2 * rs + i] = p * P_SCALE;
+                }
+            }
+            l[rs] = l[rs] * corr[rs] + sum[rs];
+        }
+        // probabilities times V: the score fragments are the A operand as they lie
+        uint32_t pf[KT / 16][4][PP];
+#pragma unroll
+        for (int kk = 0; kk < KT / 16; ++kk) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                split_f16x2<PP>(sc[2 * kk + (i >> 1)][2 * (i & 1)], sc[2 * kk + (i >> 1)][2 * (i & 1) + 1], pf[kk][i]);
+            }
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < HD / 16; j0 += JG) {
+            uint32_t b[JG][KT / 16][4];
+#pragma unroll
+            for (int jg = 0; jg < JG; ++jg) {
+#pragma unroll
+                for (int kk = 0; kk < KT / 16; ++kk) {
+                    const int r = 16 * kk + ((lane >> 3) & 1) * 8 + (lane & 7);
+                    ldmatrix_x4_trans(b[jg][kk], vs + r * ROW + (((2 * (j0 + jg) + (lane >> 4)) ^ (r & 7)) * 16));
+                }
+            }
+            float d[JG][2][4] = {};
+#pragma unroll
+            for (int p = PP - 1; p >= 0; --p) {
+#pragma unroll
+                for (int kk = 0; kk < KT / 16; ++kk) {
+                    const uint32_t a[4] = {pf[kk][0][p], pf[kk][1][p], pf[kk][2][p], pf[kk][3][p]};
+#pragma unroll
+                    for (int jg = 0; jg < JG; ++jg) {
+                        mma_f16(d[jg][0], a, b[jg][kk][0], b[jg][kk][1]);
+                        mma_f16(d[jg][1], a, b[jg][kk][2], b[jg][kk][3]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int jg = 0; jg < JG; ++jg) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float& o = acc[2 * (j0 + jg) + h][i];
+                        o = fmaf(o, corr[i >> 1], d[jg][h][i]);
+                    }
+                }
+            }
+        }
+        __syncthreads();  // the buffer is refilled two tiles from now
+    }
+    bool finite = true;
+#pragma unroll
+    for (int rs = 0; rs < 2; ++rs) {
+        float tot = l[rs];
+        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 1);
+        tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 2);
+        tot *= P_SCALE;
+        finite = finite && isfinite(tot);
+#pragma unroll
+        for (int j = 0; j < HD / 8; ++j) {
+            finite = finite && isfinite(acc[j][2 * rs]) && isfinite(acc[j][2 * rs + 1]);
+        }
+        if (rows[rs] < m) {
+            OutT* out = ctx + (int64_t)rows[rs] * n_heads * HD + head * HD + 2 * t;
+#pragma unroll
+            for (int j = 0; j < HD / 8; ++j) {
+                store_ctx(out + 8 * j, acc[j][2 * rs] / tot, acc[j][2 * rs + 1] / tot);
+            }
+        }
+    }
+    if (!__all_sync(0xFFFFFFFFu, finite)) {
+        __syncwarp();  // the lanes' own stores of these rows come first
+        attn_rows_again<HD>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx, row0 + 16 * warp, head);
+    }
+}
+
+// A few rows at a time, where a 64-row tile of the kernel above would be mostly padding: one warp per four rows of a
+// head.  Bound by the L2 reads of K and V (every row streams the whole prefix of its head).
+template <int DPL, int ROWS, typename OutT>
+__global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __restrict__ qkv, int row_stride, int m,
+                                                                int pos0, int n_heads, int n_kv, int max_seq,
+                                                                const __half* __restrict__ cache_k,
+                                                                const __half* __restrict__ cache_v,
+                                                                OutT* __restrict__ ctx)
+{
+    const int groups = (m + ROWS - 1) / ROWS;
+    const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (wid < (int64_t)groups * n_heads) {
+        // the longest rows first: the last CTAs to start are the shortest
+        attn_rows<DPL, ROWS>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx,
+                             (groups - 1 - (int)(wid / n_heads)) * ROWS, (int)(wid % n_heads));
+    }
+}
+
+template <typename OutT>
+cudaError_t attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_kv, int hd, int max_seq,
+                         const __half* cache_k, const __half* cache_v, OutT* ctx, int rows_max, cudaStream_t st)
+{
+    const int row_stride = (n_heads + 2 * n_kv) * hd;
+    if (m <= rows_max && (hd == 64 || hd == 128)) {
+        constexpr int ROWS = 4;
+        const unsigned ctas = (unsigned)(((m + ROWS - 1) / ROWS * n_heads + 3) / 4);
+        auto kernel = hd == 64 ? attn_prefill_rows_kernel<2, ROWS, OutT> : attn_prefill_rows_kernel<4, ROWS, OutT>;
+        kernel<<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
+        return cudaGetLastError();
+    }
+    const dim3 grid((unsigned)((m + 63) / 64), (unsigned)n_heads);
+    auto launch = [&](auto kernel) -> cudaError_t {
+        const int smem = (4 * 64 + 3 * 64) * hd * 2;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        kernel<<<grid, 128, smem, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
+        return cudaGetLastError();
+    };
+    return hd == 64    ? launch(attn_prefill_kernel<64, OutT>)
+           : hd == 128 ? launch(attn_prefill_kernel<128, OutT>)
+                       : cudaErrorInvalidValue;
 }
 
 // silu(gate) * up, packed for ffn_down, from gu[m][2*ffn], whose columns are the gate|up weight's rows: groups of 8 gate
@@ -1258,30 +1389,7 @@ cudaError_t ll_attn_prefill(const float* qkv, int m, int pos0, int n_heads, int 
                             const __half* cache_k, const __half* cache_v, __nv_bfloat16* ctx, int rows_max,
                             cudaStream_t st)
 {
-    const int row_stride = (n_heads + 2 * n_kv) * hd;
-    if (m <= rows_max && (hd == 64 || hd == 128)) {
-        constexpr int ROWS = 4;
-        const unsigned ctas = (unsigned)(((m + ROWS - 1) / ROWS * n_heads + 3) / 4);
-        if (hd == 64) {
-            attn_prefill_rows_kernel<2, ROWS><<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
-                                                                    cache_v, ctx);
-        } else {
-            attn_prefill_rows_kernel<4, ROWS><<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k,
-                                                                    cache_v, ctx);
-        }
-        return cudaGetLastError();
-    }
-    const dim3 grid((unsigned)((m + 63) / 64), (unsigned)n_heads);
-    auto launch = [&](auto kernel) -> cudaError_t {
-        const int smem = 4 * 64 * hd * 2;
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        kernel<<<grid, 128, smem, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
-        return cudaGetLastError();
-    };
-    return hd == 64 ? launch(attn_prefill_kernel<64>) : hd == 128 ? launch(attn_prefill_kernel<128>) : cudaErrorInvalidValue;
+    return attn_prefill(qkv, m, pos0, n_heads, n_kv, hd, max_seq, cache_k, cache_v, ctx, rows_max, st);
 }
 
 cudaError_t ll_silu_mul_rows_packed(const float* gu, int m, int ffn, uint8_t* packed, cudaStream_t st)
