@@ -170,7 +170,7 @@ struct Cols {
 // Batch 1: all compact records (qmm_common.cuh) staged in shared memory.
 struct XShared {
     const uint8_t* base;   // [kc] records of XPK1_REC bytes
-    const uint8_t* zeros;  // 512 zero bytes for the lanes that carry no activation row
+    const uint8_t* zeros;  // Q6_K: 512 zero bytes for the lanes that carry no activation row
 };
 
 // Batches 2..16: the record of one chunk travels with the weight tile into the warp's ring
@@ -351,8 +351,9 @@ __device__ __forceinline__ void compute_chunk(const uint8_t* slot, const XSrc<MC
 // k-slots 16..31 from the next (for a fragment that is only a choice of registers) and its B
 // operand is zero outside those blocks' columns; four MMAs, two per pair of blocks, add up in
 // the same accumulators.  Lane t then folds block t of the group: one fold per four blocks, with
-// every lane at work.  (Two blocks per fold left half of the lanes repeating the other half: 70B-shape layers, a
-// 1024-token prompt and 64 steps, 50.4 ms against 47.9; a 7B-shape answer of 128 tokens 2 % slower.)
+// every lane at work.  (Two blocks per fold left half of the lanes repeating the other half; otherwise the same
+// code: 70B-shape layers, a 1024-token prompt and 64 steps, 48.1 ms against 45.7; a 7B shape, 512 tokens and 128 steps,
+// 161.8 against 157.8.)
 
 template <int FMT>
 __device__ __forceinline__ void compute_chunk_m1(const uint8_t* slot, const XShared& xs, int c, int lane, float* acc)
@@ -362,7 +363,10 @@ __device__ __forceinline__ void compute_chunk_m1(const uint8_t* slot, const XSha
     const int role = g >> 1;  // the block of a group whose activations this lane supplies
     const uint8_t* rec = xs.base + (size_t)c * XPK1_REC;
     // Per-lane sources of the B registers: lane (g, t) feeds column g = digit g & 1 of block g >> 1; every register
-    // that belongs to another block comes from the zero page.  Entry = uint2 {weights 4t.., weights 16+4t..}.
+    // that belongs to another block is zero.  Entry = uint2 {weights 4t.., weights 16+4t..}.  The lane loads its own entry and
+    // selects; with a pointer per register, three of them to a page of zeros (as Q6_K still has them, whose entries are half
+    // as large), the 40-register variants spill: pack + matvec of one row, us, Q4_0 11008 x 2304 6.04 against 5.86, 4096 x
+    // 4096 5.28 and 5.15, 4096 x 14336 9.73 and 9.11; Q8_0 11008 x 2048 6.86 and 6.54; Q4_K 11008 x 8192 15.7 and 15.2.
     const uint8_t* xrow = rec + ((g & 1) * 4 + t) * 8;
     const int4* meta = reinterpret_cast<const int4*>(rec + XPK1_META);
     const uint4* qs = reinterpret_cast<const uint4*>(slot) + lane;
@@ -414,10 +418,7 @@ __device__ __forceinline__ void compute_chunk_m1(const uint8_t* slot, const XSha
         acc[0] = fmaf(a0, 0.25f, acc[0]);
         acc[1] = fmaf(a1, 0.25f, acc[1]);
     } else {
-        const uint8_t* x0p = role == 0 ? xrow : xs.zeros;
-        const uint8_t* x1p = role == 1 ? xrow + 64 : xs.zeros;
-        const uint8_t* x2p = role == 2 ? xrow + 128 : xs.zeros;
-        const uint8_t* x3p = role == 3 ? xrow + 192 : xs.zeros;
+        const uint8_t* mine = xrow + 64 * role;
         // this lane's block of group P is 4P + t
         const __half* dg_p = reinterpret_cast<const __half*>(p1 + g * 16) + t;
         const __half* dg8_p = reinterpret_cast<const __half*>(p1 + (g + 8) * 16) + t;
@@ -440,10 +441,9 @@ __device__ __forceinline__ void compute_chunk_m1(const uint8_t* slot, const XSha
         float m0 = 0.0f, m1 = 0.0f;
 #pragma unroll
         for (int P = 0; P < 2; ++P) {
-            const uint2 x0 = *reinterpret_cast<const uint2*>(x0p + P * 256);
-            const uint2 x1 = *reinterpret_cast<const uint2*>(x1p + P * 256);
-            const uint2 x2 = *reinterpret_cast<const uint2*>(x2p + P * 256);
-            const uint2 x3 = *reinterpret_cast<const uint2*>(x3p + P * 256);
+            const uint2 xv = *reinterpret_cast<const uint2*>(mine + P * 256), none = make_uint2(0u, 0u);
+            const uint2 x0 = role == 0 ? xv : none, x1 = role == 1 ? xv : none, x2 = role == 2 ? xv : none,
+                        x3 = role == 3 ? xv : none;
             const int4 mm = meta[4 * P + t];
             const float xsb = __int_as_float(mm.z);
             if constexpr (FMT == FMT_Q8_0) {

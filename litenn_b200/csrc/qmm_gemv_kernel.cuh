@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
                           &my_bars[s]);
         }
     }
-    if constexpr (MC == 1) {
+    if constexpr (MC == 1 && FMT == FMT_Q6_K) {
         // zero page for the lanes that carry no activation row
         uint32_t* z = reinterpret_cast<uint32_t*>(smem + Plan::X_OFF + xpack1_bytes(kc));
         for (int i = threadIdx.x; i < 128; i += NW * 32) {
