@@ -24,8 +24,10 @@ def load(name, device_code, link_library=None):
                "-gencode", "arch=compute_100a,code=sm_100a"]
         if os.path.exists("/usr/bin/g++"):
             cmd[1:1] = ["-ccbin", "/usr/bin/g++"]
+        env = dict(os.environ)
         if link_library:
             d, f = os.path.split(os.path.abspath(link_library))
-            cmd += ["-L", d, "-l:" + f, "-Xlinker", "-rpath=" + d]
-        subprocess.run(cmd, check=True)
+            cmd += ["-L", d, "-l:" + f]
+            env["LD_RUN_PATH"] = "$ORIGIN/" + os.path.relpath(d, os.path.dirname(out))
+        subprocess.run(cmd, check=True, env=env)
     return ctypes.CDLL(out)
