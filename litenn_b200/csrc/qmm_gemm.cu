@@ -185,7 +185,8 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         bool ok = true;
         for (int s = 0; s < n_steps; ++s) {
             const int as = s % GEMM_A_STAGES;
-            ok = g_mbar_wait_warp(&full_b[slot], phase) && g_mbar_wait_warp(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
+            ok = g_mbar_wait(&full_b[slot], phase) && g_mbar_wait(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
+            ok = __all_sync(0xFFFFFFFFu, ok);
             if (!ok) {
                 if (lane == 0) {
                     atomicExch(args.status, 12);

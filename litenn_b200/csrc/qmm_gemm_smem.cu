@@ -208,7 +208,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         for (int s = 0; s < n_stages; ++s) {
             const int slot = s % GEMM_STAGES;
             const uint32_t parity = (uint32_t)(s / GEMM_STAGES) & 1u;
-            ok = g_mbar_wait_warp(&full_a[slot], parity) && g_mbar_wait_warp(&full_b[slot], parity);
+            ok = g_mbar_wait(&full_a[slot], parity) && g_mbar_wait(&full_b[slot], parity);
+            ok = __all_sync(0xFFFFFFFFu, ok);
             if (!ok) {
                 if (lane == 0) {
                     atomicExch(args.status, 12);
