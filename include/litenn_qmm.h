@@ -240,7 +240,7 @@ int qmm_gemm_bf16(const qmm_weight* w, const void* x_bf16_dev, void* y_dev, int6
  * rounded to bf16 on the device (round to nearest even, into a per-(device, stream) workspace the
  * library allocates on first use), multiplied as above, and the result is fp32.  Against the
  * reference's fp32 product this adds the two bf16 roundings (activations and dequantized weights,
- * 2^-9 relative each); use qmm_gemv_f32 where m <= QMM_GEMV_MAX_BATCH and that matters.
+ * up to 2^-8 relative each); use qmm_gemv_f32 where m <= QMM_GEMV_MAX_BATCH and that matters.
  */
 int qmm_gemm_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int64_t m, void* stream);
 

@@ -940,9 +940,12 @@ int qmm_llama_prefill(qmm_llama* m, const int32_t* tokens_host, int n, int32_t* 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int d = c.d_model, hd = c.head_dim;
     const int pos0 = m->host_pos;
-    // Activations are rounded to bf16 between the layers, and in a narrow model one rounding that falls the other way moves
-    // the logits by up to 2e-3 (in a 4096-wide one by 1e-4): up to 2048 wide every product keeps its order of summation,
-    // and so does attention up to 256 rows.  Such prompts are mostly launches (1536 x 2048, 64 rows: 14 us against 10).
+    // Activations are rounded to bf16 between the layers, and a sum taken in another order flips some of those roundings.
+    // Up to 2048 wide the products keep the shared-memory form's order and attention the row kernel's up to 256 rows: that
+    // keeps the logits of narrow models within 1e-5 (2-norm) of the earlier ones, which free choice moves by up to 2.4e-4,
+    // without being less accurate.  The price, four blocks and four steps: 512 wide, 200 tokens 1019 us against 744; 2048
+    // wide, 200 tokens 1678 against 1092.  Above 256 rows attention's own order changes with the kernel, and keeping the
+    // products' is worth nothing there (2048 wide, 300 tokens: 1e-5 either way, 1532 us against 1188).
     const bool keep_order = d <= 2048;
     LL_CUDA(cudaMemcpyAsync(m->tokens_dev, tokens_host, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st));
     LL_CUDA(ll_embed_rows(c.embd_fmt, m->embd, m->tokens_dev, n, d, m->hr, st));

@@ -915,9 +915,9 @@ __device__ __noinline__ void attn_rows_again(const float* qkv, int row_stride, i
 // Error against 64 bits before the rounding to bf16 (2-norm, 300 / 1999 tokens, HD 128, scores of about 1): 1.6e-7 /
 // 1.4e-7 here, 2.1e-7 / 6.2e-7 in the fp32 row kernel below; two parts and one chain for everything had 5.5e-7 / 2.9e-6.
 // Scores of about 16: 4.1e-7 / 5.3e-7, 4.2e-7 / 5.4e-7 and 1.3e-6 / 1.6e-6.
-// Bound: the MMA pipe, 16 cycles per m16n8k16 and scheduler, five MMAs where plain fp16 takes two.  1999 rows, 32 heads,
-// HD 128: 309 us, 272 with two parts of a query, 247 with two parts and long chains.  Four rows per warp with fp32
-// arithmetic and shuffles are issue-bound: 512 rows 250 us against 40.
+// Bound: the MMA pipe (65 % of all cycles at 1999 rows), about 16 cycles per m16n8k16 and scheduler, five MMAs where plain
+// fp16 takes two.  1999 rows, 32 heads, HD 128: 309 us, 272 with two parts of a query, 247 with two parts and long chains.
+// Four rows per warp with fp32 arithmetic and shuffles are issue-bound: 512 rows 250 us against 40.
 // A masked key's V row takes part in the product with probability 0, and a query or a key that overflowed fp16 meets the
 // parts one by one, so infinities and NaN spread further here than they should.  They always leave a mark on the row's own
 // sums, and a warp that finds one does its rows again in fp32, key by key.

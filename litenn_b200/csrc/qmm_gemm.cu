@@ -12,9 +12,9 @@
 //   MMA warp        tcgen05.mma (kind::f16, bf16 x bf16 -> fp32, M = 128, N = tokens, K = 16), A from TMEM
 // Weights never pass through shared memory, whose bandwidth (128 bytes per cycle and SM) a B operand of
 // dequantized weights shares with the operand reads and the TMA writes.
-// Bound: the dequant warps' instruction issue.  Q6_K 4096 x 11264, 64 tokens: 27 us here against 125 us of the
-// shared-memory form, whose 16 dequant warps have two row tiles to work on; Q4_0 4096 x 4096, 512 tokens: 34.7 against
-// 51.6.  The MMAs are issued under elect.sync: with a lane comparison in its place the same kernel took a fifth longer
+// Bound: the dequant warps' instruction issue (ncu, Q4_0 22016 x 4096, 512 tokens: 65 % of the issue slots, ALU pipe 58 %,
+// tensor pipe 36 %).  Q6_K 4096 x 11264, 64 tokens: 27 us here against 125 us of the shared-memory form, whose 16 dequant
+// warps have two row tiles to work on; Q4_0 4096 x 4096, 512 tokens: 34.7 against 51.6.  The MMAs are issued under elect.sync: with a lane comparison in its place the same kernel took a fifth longer
 // (Q4_0 4096 x 11008, 512 tokens: 94 us and 77 us).
 // Every wait has an iteration limit; a CTA that gives up sets the status word, still frees its TMEM and
 // returns.
@@ -477,8 +477,9 @@ GemmPlan gemm_form(const WeightView& w, int64_t m, int sm_count, int nb, int tok
 // in four 14.7, shared memory 43.3; 1024 tokens: NB = 2 45.2, shared memory 57.4; 1999 tokens: NB = 2 85.6, shared
 // memory 71.8.  Q6_K 8192 x 28672, 128 tokens: NB = 1 90.8, shared memory 327; 1024 tokens: 588 and 444.
 //
-// keep_order asks for the shared-memory form, whose sums run over K in one fixed order per row tile; the other two add the
-// K splits of a tile and start elsewhere, which changes the last bits.
+// keep_order asks for the shared-memory form with the K offsets it has always started from.  They follow from the weight,
+// the number of 256-token groups and the SM count, so the order of a row's sums is fixed for a given product on a given
+// GPU, not for a weight; the other two forms start elsewhere and add the K splits of a tile, which changes the last bits.
 GemmPlan plan_gemm(const WeightView& w, int64_t m, int sm_count, bool keep_order)
 {
     GemmPlan best = gemm_form(w, m, sm_count, 0, 0, 1);

@@ -14,9 +14,10 @@
 // A 3-stage mbarrier ring decouples the three roles.  At the end warps 2..17 read the
 // accumulators with tcgen05.ld and write Y.  Every wait has an iteration limit; a CTA
 // that gives up sets the status word, still frees its TMEM and returns.
-// Bound: shared-memory bandwidth (operand reads, dequantized stores, TMA writes) and the dequant warps' issue, about
-// evenly: Q4_K 14336 x 4096, 512 tokens takes 71 us (850 TFLOP/s).  It took 94 us when every value went through an
-// integer conversion of its own and the MMAs were issued under a lane comparison instead of elect.sync.
+// Bound: latency.  No unit is near its limit (ncu, Q4_0 12288 x 4096, 1999 tokens: tensor pipe 51 %, memory pipes 50 %,
+// issue 41 %); the dequant warps wait for packed words and scales, and three stages do not hide it.  Q4_K 14336 x 4096,
+// 512 tokens takes 71 us (850 TFLOP/s).  It took 94 us when every value went through an integer conversion of its own and
+// the MMAs were issued under a lane comparison instead of elect.sync.
 #include <algorithm>
 
 #include "qmm_gemm_dequant.cuh"

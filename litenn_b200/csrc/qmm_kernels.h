@@ -40,7 +40,7 @@ cudaError_t launch_f32_to_bf16(const float* x, int64_t count, void* out_bf16, cu
 // Prefill GEMM on tcgen05: y[m,n] = x_bf16[m,k] · Wᵀ.  On a configuration error `*why` explains it.
 //   GEMM_OUT_SWIGLU  the rows are interleaved gate|up (EPI_SWIGLU, qmm_common.cuh): y[m, n / 2] = bf16(silu(gate) * up);
 //                    n a multiple of 16, y 16-byte aligned
-//   keep_order       sums in the shared-memory form's order of K, also where another form is faster
+//   keep_order       sums in the shared-memory form's order of K for this m, also where another form is faster
 constexpr int GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2;
 cudaError_t launch_gemm_bf16(const WeightView& w, const void* x_bf16, void* y, int64_t m, int out, bool keep_order,
                              int sm_count, int* status, cudaStream_t stream, const char** why);
