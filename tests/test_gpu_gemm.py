@@ -41,8 +41,8 @@ def run_gemm(torch, w, x_f32, out_bf16=False):
 @pytest.mark.parametrize("fmt", FORMATS)
 @pytest.mark.parametrize("shape", [(128, 16, 256), (128, 256, 512), (1, 48, 256), (100, 200, 1024), (300, 528, 768),
                                    (512, 1000, 512),
-                                   # more than 256 rows: CTA pairs share each dequantized tile; a second CTA with one
-                                   # row, an odd number of 256-row groups (partner without rows), five groups
+                                   # more than 256 rows: a second 256-row group with one
+                                   # row, an odd number of groups, five groups
                                    (257, 272, 512), (600, 96, 512), (1100, 320, 768)])
 def test_gemm_matches_oracle(torch_cuda, fmt, shape):
     m, n, k = shape
