@@ -130,9 +130,12 @@ struct WeightView {
 // 2r carries the high bytes and column 2r+1 the low bytes of row 4*j + r.
 // The buffer is an array of per-chunk records (one 256-wide K chunk each), so whoever produces
 // 32 consecutive activations can write their block without knowing the rest:
-//   general (m > 1), ncp = ceil(m / 4) column groups; record of XPK_XQ(ncp) + 2048 bytes:
-//     xq   [8 blocks][ncp][32 lanes] uint2 {k-slots 4t..4t+3, 16+4t..16+4t+3} of column g
-//     meta [8 blocks][16 rows] int4 {8*Q, 128*Q, float bits of xs, 0}
+//   general (m > 1), ncp = ceil(m / 4) MMAs per block; record of xpack_rec_bytes(ncp), of which xpack_copy_bytes are used.
+//   Pairs of MMAs serve eight rows each (octet o: column g of MMA 2o is the high byte of row 8o + g, of MMA 2o + 1 the low
+//   byte), so that neighbouring rows of one digit sit in neighbouring accumulators; an odd last MMA serves four rows as above:
+//     xq   [8 blocks] of octets [32 lanes] uint4 {MMA 2o k-slots 4t.., 16+4t.., MMA 2o+1 4t.., 16+4t..}, then the odd
+//          MMA's [32 lanes] uint2
+//     meta [2][8 blocks][16] float: xs, then 8*Q*xs; row r at xpack_meta_pos: a lane's values are one load
 //   compact (m == 1): only lanes 0..7 (columns 0 and 1) exist; record of 640 bytes:
 //     xq   [8 blocks][8 lanes] uint2        (lane = 4*digit + t, digit 0 = high byte)
 //     meta [8 blocks] int4 {8*Q, 128*Q, float bits of xs, 0}
@@ -146,6 +149,7 @@ struct XPackView {
 
 constexpr int XPK1_REC = 640;        // compact record
 constexpr int XPK1_META = 512;       // offset of its meta part
+constexpr int XPK_META_PLANE = 512;  // general record: bytes of one of the two planes of its meta part
 
 __host__ __device__ inline int xpack_ncp(int m)
 {
@@ -158,6 +162,27 @@ __host__ __device__ constexpr int xpack_xq_bytes(int ncp)
 __host__ __device__ constexpr int xpack_rec_bytes(int ncp)
 {
     return xpack_xq_bytes(ncp) + 8 * 16 * 16;
+}
+// what a kernel reads of a record: the rest pads it to the size that qmm_packed_activation_bytes has always named
+__host__ __device__ constexpr int xpack_copy_bytes(int ncp)
+{
+    return xpack_xq_bytes(ncp) + 2 * XPK_META_PLANE;
+}
+// place of row r among a block's 16 meta values: lane t of a quad reads rows 2t, 2t+1 (and 8+2t, 8+2t+1), or row t of the odd
+// MMA's four
+__host__ __device__ inline int xpack_meta_pos(int ncp, int row)
+{
+    const int o = row >> 3 < ncp / 2 ? row >> 3 : ncp / 2, r = row - 8 * o;
+    return (r >> 1) * 4 + o * 2 + (r & 1);
+}
+// word of row r's activations half*16 + 4t .. +3 of block b, digit 0 high, 1 low; in 4-byte units from the start of the record
+__host__ __device__ inline int xpack_word_at(int ncp, int row, int b, int digit, int t, int half)
+{
+    const int o = row >> 3;
+    if (o < ncp / 2) {
+        return b * ncp * 64 + o * 128 + (4 * (row & 7) + t) * 4 + 2 * digit + half;
+    }
+    return b * ncp * 64 + (ncp - 1) * 64 + (4 * (2 * (row - 8 * (ncp / 2)) + digit) + t) * 2 + half;
 }
 __host__ __device__ inline size_t xpack_bytes(int kc, int ncp)
 {

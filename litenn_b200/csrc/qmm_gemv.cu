@@ -14,7 +14,6 @@ namespace {
 __global__ void __launch_bounds__(128) pack_x_kernel(const float* __restrict__ x, int m, int64_t k, int ncp,
                                                      int compact, uint8_t* __restrict__ out)
 {
-    __shared__ short q[4][256];
     pdl_launch_dependents();  // the matvec that follows may start fetching its weights
     pdl_wait();               // x may come from the previous kernel; the buffer may still be read by it
     const int c = blockIdx.x;
@@ -35,6 +34,7 @@ __global__ void __launch_bounds__(128) pack_x_kernel(const float* __restrict__ x
         }
         return;
     }
+    // lane L holds one fragment word of each digit twice: activations 8L..8L+3 and 8L+4..8L+7 of block L >> 2
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -43,45 +43,27 @@ __global__ void __launch_bounds__(128) pack_x_kernel(const float* __restrict__ x
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
     const float inv = amax > 0.0f ? 32639.0f / amax : 0.0f;
+    uint32_t hw[2] = {0u, 0u}, lw[2] = {0u, 0u};
     int bsum = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         int hi, lo;
-        const int qi = quant16(v[i], inv, hi, lo);
-        q[warp][8 * lane + i] = (short)qi;
-        bsum += qi;
+        bsum += quant16(v[i], inv, hi, lo);
+        hw[i >> 2] |= (uint32_t)(hi & 0xFF) << (8 * (i & 3));
+        lw[i >> 2] |= (uint32_t)(lo & 0xFF) << (8 * (i & 3));
     }
     bsum += __shfl_xor_sync(0xFFFFFFFFu, bsum, 1);
     bsum += __shfl_xor_sync(0xFFFFFFFFu, bsum, 2);
     uint8_t* rec = out + (size_t)c * xpack_rec_bytes(ncp);
-    if ((lane & 3) == 0) {
-        reinterpret_cast<int4*>(rec + xpack_xq_bytes(ncp))[(lane >> 2) * 16 + row] =
-            make_int4(8 * bsum, 128 * bsum, __float_as_int(amax / 32639.0f), 0);
-    }
-    __syncthreads();
-
-    // fragment lane (g,t) of block b: activation row g>>1 of this group, digit g&1 (0 = high byte)
-    uint2* xq = reinterpret_cast<uint2*>(rec);
-    for (int i = threadIdx.x; i < 8 * 32; i += 128) {
-        const int b = i >> 5;
-        const int fl = i & 31;
-        const int g = fl >> 2;
-        const int t = fl & 3;
-        const int r = g >> 1;
-        const int lo_digit = g & 1;
-        uint32_t w0 = 0, w1 = 0;
+    const int b = lane >> 2, part = lane & 3;
+    const int t0 = 2 * (part & 1), half = part >> 1;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int q0 = q[r][32 * b + 4 * t + e];
-            const int q1 = q[r][32 * b + 16 + 4 * t + e];
-            const int l0 = ((q0 + 128) & 0xFF) - 128;
-            const int l1 = ((q1 + 128) & 0xFF) - 128;
-            const int d0 = lo_digit ? l0 : ((q0 - l0) >> 8);
-            const int d1 = lo_digit ? l1 : ((q1 - l1) >> 8);
-            w0 |= (uint32_t)(d0 & 0xFF) << (8 * e);
-            w1 |= (uint32_t)(d1 & 0xFF) << (8 * e);
-        }
-        xq[(size_t)(b * ncp + j) * 32 + fl] = make_uint2(w0, w1);
+    for (int i = 0; i < 2; ++i) {
+        *xpack_word(rec, ncp, row, b, 0, t0 + i, half) = hw[i];
+        *xpack_word(rec, ncp, row, b, 1, t0 + i, half) = lw[i];
+    }
+    if (part == 0) {
+        xpack_meta(rec, ncp, row, b, bsum, amax);
     }
 }
 

@@ -1,14 +1,11 @@
-// Device-side building blocks of the dequant-fused matvec, shared by the stand-alone GEMV
-// kernels (qmm_gemv.cu) and the persistent decoder kernel (llama_mega.cu): mbarrier / bulk-copy
-// PTX wrappers, the integer MMA wrappers, the packed-activation views and the per-chunk
-// multiply routines for every block format.
+// Device-side building blocks of the dequant-fused matvec kernels (qmm_gemv_kernel.cuh, qmm_gemv_batch.cuh): mbarrier /
+// bulk-copy PTX wrappers, the integer MMA wrappers and the batch-1 multiply routine for every block format.
 #pragma once
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <type_traits>
 
 #include "qmm_common.cuh"
 
@@ -36,6 +33,11 @@ __device__ __forceinline__ void fence_barrier_init()
 __device__ __forceinline__ void fence_proxy_async()
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
@@ -105,15 +107,6 @@ __device__ __forceinline__ void mma_k32(int (&d)[4], uint32_t a0, uint32_t a1, u
     }
 }
 
-// D = A(16x16, row, s8) * B(16x8, col, s8) with a zero C operand.
-__device__ __forceinline__ void mma_k16(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0)
-{
-    const int z = 0;
-    asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
-                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-                 : "r"(a0), "r"(a1), "r"(b0), "r"(z));
-}
-
 // D = A * B + D  (k32, B s8): second half of a two-MMA block pair.
 template <bool A_SIGNED>
 __device__ __forceinline__ void mma_k32_acc(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -153,194 +146,11 @@ __device__ __forceinline__ uint32_t byte_of_word(uint32_t w, int i)
     return (w >> (8 * i)) & 0xFFu;
 }
 
-// ---- activation sources -------------------------------------------------------------------
-//
-// B-fragment of one MMA (k32 x 8 columns): column 2r holds the high bytes and column
-// 2r+1 the low bytes of activation row 4*j + r of column group j, so lane (g,t) keeps
-// in d[0],d[1] the (high, low) sums of weight row g and in d[2],d[3] those of row g+8,
-// all for activation row 4*j + t.
-
-// MC = activation rows handled: 1 (only row 0 is live) or a multiple of 4 up to 16.
-template <int MC>
-struct Cols {
-    static constexpr int NCP = MC == 1 ? 1 : MC / 4;  // MMAs (column groups of 4 rows) per block
-    static constexpr int NOUT = 2 * NCP;              // accumulators per lane
-};
-
 // Batch 1: all compact records (qmm_common.cuh) staged in shared memory.
 struct XShared {
     const uint8_t* base;   // [kc] records of XPK1_REC bytes
     const uint8_t* zeros;  // Q6_K: 512 zero bytes for the lanes that carry no activation row
 };
-
-// Batches 2..16: the record of one chunk travels with the weight tile into the warp's ring
-// slot, behind the tile:  xq [8 blocks][NCP][32 lanes] uint2 | meta [8 blocks][16 rows] int4
-template <int NCP>
-struct XSlot {
-    static constexpr int XQ_BYTES = xpack_xq_bytes(NCP);
-    static constexpr int BYTES = xpack_rec_bytes(NCP);
-    const uint8_t* base;  // the chunk's record in the current slot
-    __device__ __forceinline__ void attach(const uint8_t* p) { base = p; }
-    __device__ __forceinline__ uint2 frag(int b, int j, int lane) const
-    {
-        return *reinterpret_cast<const uint2*>(base + ((b * NCP + j) * 32 + lane) * 8);
-    }
-    // {8*Q, 128*Q, scale bits, 0} of block b for this lane's activation row 4*j + t
-    __device__ __forceinline__ int4 meta(int b, int j, int lane) const
-    {
-        return *reinterpret_cast<const int4*>(base + XQ_BYTES + (b * 16 + 4 * j + (lane & 3)) * 16);
-    }
-};
-
-template <int MC>
-using XSrc = typename std::conditional<MC == 1, XShared, XSlot<Cols<MC>::NCP>>::type;
-
-// One 16x256 tile, resident in shared memory at `slot`, times the activations of its chunk
-// (batches 2..16).  acc[2j], acc[2j+1]: rows g, g+8 for activation row 4j + t.
-template <int FMT, int MC>
-__device__ __forceinline__ void compute_chunk(const uint8_t* slot, const XSrc<MC>& xs, int lane, float* acc)
-{
-    constexpr int NCP = Cols<MC>::NCP;
-    const int g = lane >> 2;
-    int d[4];
-    const uint4* qs = reinterpret_cast<const uint4*>(slot) + lane;
-    const uint8_t* p1 = slot + tile_p1_offset(FMT);
-    const uint8_t* p2 = slot + tile_p2_offset(FMT);
-
-    if constexpr (FMT == FMT_Q4_0) {
-        // d[0],d[1]: digit sums of row g over unsigned nibbles n; d[2],d[3]: those of row g+8 over the
-        // bytes 16*n(g+8) + n(g), so row g+8 comes out in units of 1/16 after row g's part is removed.
-        const uint4 s0 = *reinterpret_cast<const uint4*>(p1 + g * 16);
-        const uint4 s1 = *reinterpret_cast<const uint4*>(p1 + (g + 8) * 16);
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const uint4 q = qs[p * 32];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t w1 = h ? q.z : q.x;  // weights 4t..   rows g | g+8
-                const uint32_t w2 = h ? q.w : q.y;  // weights 16+4t..
-                const int b = 2 * p + h;
-                const float dg = half_of(s0, b);
-                const float dg8 = half_of(s1, b) * 0.0625f;
-#pragma unroll
-                for (int j = 0; j < NCP; ++j) {
-                    const uint2 xf = xs.frag(b, j, lane);
-                    mma_k32<false>(d, w1 & 0x0F0F0F0Fu, w1, w2 & 0x0F0F0F0Fu, w2, xf.x, xf.y);
-                    const int4 mm = xs.meta(b, j, lane);
-                    const float xsb = __int_as_float(mm.z);
-                    const int vg = d[0] * 256 + d[1];
-                    const int vg8 = d[2] * 256 + d[3] - vg;
-                    acc[2 * j + 0] = fmaf((float)(vg - mm.x), dg * xsb, acc[2 * j + 0]);
-                    acc[2 * j + 1] = fmaf((float)(vg8 - mm.y), dg8 * xsb, acc[2 * j + 1]);
-                }
-            }
-        }
-    } else if constexpr (FMT == FMT_Q8_0) {
-        const uint4 s0 = *reinterpret_cast<const uint4*>(p1 + g * 16);
-        const uint4 s1 = *reinterpret_cast<const uint4*>(p1 + (g + 8) * 16);
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const uint4 q = qs[b * 32];
-            const float dg = half_of(s0, b);
-            const float dg8 = half_of(s1, b);
-#pragma unroll
-            for (int j = 0; j < NCP; ++j) {
-                const uint2 xf = xs.frag(b, j, lane);
-                mma_k32<true>(d, q.x, q.y, q.z, q.w, xf.x, xf.y);
-                const float xsb = __int_as_float(xs.meta(b, j, lane).z);
-                acc[2 * j + 0] = fmaf((float)(d[0] * 256 + d[1]), dg * xsb, acc[2 * j + 0]);
-                acc[2 * j + 1] = fmaf((float)(d[2] * 256 + d[3]), dg8 * xsb, acc[2 * j + 1]);
-            }
-        }
-    } else if constexpr (FMT == FMT_Q4_K) {
-        // 12 packed bytes per row -> eight 6-bit scales and eight 6-bit mins, four per word
-        uint32_t scw[2][2], mnw[2][2];
-        float dd[2], dmin[2];
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs) {
-            const uint32_t* sp = reinterpret_cast<const uint32_t*>(p1 + (g + 8 * rs) * 12);
-            const uint32_t w0 = sp[0], w1 = sp[1], w2 = sp[2];
-            scw[rs][0] = w0 & 0x3F3F3F3Fu;
-            mnw[rs][0] = w1 & 0x3F3F3F3Fu;
-            scw[rs][1] = (w2 & 0x0F0F0F0Fu) | ((w0 >> 2) & 0x30303030u);
-            mnw[rs][1] = ((w2 >> 4) & 0x0F0F0F0Fu) | ((w1 >> 2) & 0x30303030u);
-            const uint32_t dm = *reinterpret_cast<const uint32_t*>(p2 + (g + 8 * rs) * 4);
-            dd[rs] = __half2float(__ushort_as_half((unsigned short)(dm & 0xFFFFu)));
-            dmin[rs] = __half2float(__ushort_as_half((unsigned short)(dm >> 16)));
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const uint4 q = qs[p * 32];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int sb = 2 * p + h;
-                const uint32_t w1 = h ? q.z : q.x;
-                const uint32_t w2 = h ? q.w : q.y;
-                const float sg = dd[0] * (float)byte_of_word(scw[0][sb >> 2], sb & 3);
-                const float sg8 = dd[1] * (float)byte_of_word(scw[1][sb >> 2], sb & 3) * 0.0625f;
-                // "- dmin*m": the same offset on every weight of the sub-block, so it multiplies the
-                // sum of the block's quantized activations, (8*Q) / 8
-                const float mg = dmin[0] * (float)byte_of_word(mnw[0][sb >> 2], sb & 3) * 0.125f;
-                const float mg8 = dmin[1] * (float)byte_of_word(mnw[1][sb >> 2], sb & 3) * 0.125f;
-#pragma unroll
-                for (int j = 0; j < NCP; ++j) {
-                    const uint2 xf = xs.frag(sb, j, lane);
-                    mma_k32<false>(d, w1 & 0x0F0F0F0Fu, w1, w2 & 0x0F0F0F0Fu, w2, xf.x, xf.y);
-                    const int4 mm = xs.meta(sb, j, lane);
-                    const float xsb = __int_as_float(mm.z);
-                    const int vg = d[0] * 256 + d[1];
-                    const int vg8 = d[2] * 256 + d[3] - vg;
-                    const float q8 = (float)mm.x * xsb;
-                    acc[2 * j + 0] = fmaf((float)vg, sg * xsb, fmaf(-mg, q8, acc[2 * j + 0]));
-                    acc[2 * j + 1] = fmaf((float)vg8, sg8 * xsb, fmaf(-mg8, q8, acc[2 * j + 1]));
-                }
-            }
-        }
-    } else {  // Q6_K: A byte = 4 * (q - 32) as int8, one k16 MMA per 16-wide sub-block
-        const uint4 s0 = *reinterpret_cast<const uint4*>(p1 + g * 16);
-        const uint4 s1 = *reinterpret_cast<const uint4*>(p1 + (g + 8) * 16);
-        const float dg = __half2float(*reinterpret_cast<const __half*>(p2 + g * 2)) * 0.25f;
-        const float dg8 = __half2float(*reinterpret_cast<const __half*>(p2 + (g + 8) * 2)) * 0.25f;
-        uint4 qv[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            qv[i] = qs[i * 32];
-        }
-#pragma unroll
-        for (int quad = 0; quad < 4; ++quad) {
-            uint32_t out[2][4];
-#pragma unroll
-            for (int rsel = 0; rsel < 2; ++rsel) {
-                const int base = (quad * 2 + rsel) * 3;
-                const uint32_t X = word_of(qv[(base + 0) >> 2], (base + 0) & 3);
-                const uint32_t Y = word_of(qv[(base + 1) >> 2], (base + 1) & 3);
-                const uint32_t Z = word_of(qv[(base + 2) >> 2], (base + 2) & 3);
-                out[rsel][0] = X & 0xFCFCFCFCu;
-                out[rsel][1] = Y & 0xFCFCFCFCu;
-                out[rsel][2] = Z & 0xFCFCFCFCu;
-                out[rsel][3] = ((X & 0x03030303u) << 6) | ((Y & 0x03030303u) << 4) | ((Z & 0x03030303u) << 2);
-            }
-#pragma unroll
-            for (int j = 0; j < NCP; ++j) {
-                const uint2 xf0 = xs.frag(2 * quad, j, lane);
-                const uint2 xf1 = xs.frag(2 * quad + 1, j, lane);
-                const float xsb0 = __int_as_float(xs.meta(2 * quad, j, lane).z);
-                const float xsb1 = __int_as_float(xs.meta(2 * quad + 1, j, lane).z);
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int sb = 4 * quad + jj;
-                    const uint2& xf = (jj >> 1) ? xf1 : xf0;
-                    const float xsb = (jj >> 1) ? xsb1 : xsb0;
-                    mma_k16(d, out[0][jj], out[1][jj], (jj & 1) ? xf.y : xf.x);
-                    const float sg = dg * (float)(int)(signed char)byte_of(s0, sb);
-                    const float sg8 = dg8 * (float)(int)(signed char)byte_of(s1, sb);
-                    acc[2 * j + 0] = fmaf((float)(d[0] * 256 + d[1]), sg * xsb, acc[2 * j + 0]);
-                    acc[2 * j + 1] = fmaf((float)(d[2] * 256 + d[3]), sg8 * xsb, acc[2 * j + 1]);
-                }
-            }
-        }
-    }
-}
 
 // ---- batch 1 ---------------------------------------------------------------------------------
 //

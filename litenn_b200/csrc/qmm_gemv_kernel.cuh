@@ -1,6 +1,6 @@
-// Dequant-fused GEMV / skinny GEMM for decode (1..16 activation rows) on sm_100a: the kernel
-// template and its per-format launcher.  Each block format instantiates it in a translation
-// unit of its own (qmm_gemv_q4_0.cu, ...), so the formats compile in parallel.
+// Dequant-fused GEMV for decode (one activation row) on sm_100a: the kernel template, and the per-format launcher of a
+// matvec of any row count.  Each block format instantiates it in a translation
+// unit of its own (qmm_gemv_q4_0.cu, ...), so the formats compile in parallel.  2..16 rows are qmm_gemv_batch.cuh.
 //
 // The weights never become floats in memory.  One CTA owns one 16-row tile of the
 // output; its warps take the 256-column K chunks of that row tile round-robin.
@@ -10,7 +10,7 @@
 // consumed it, so the copies of a whole CTA are in flight from the first instruction
 // on and HBM latency is paid once, not per chunk.  From shared memory the quants become
 // int8 MMA A-fragments with two or three logic ops per word and are multiplied on the
-// integer tensor-core path (mma.sync m16n8k32 / m16n8k16, s32 accumulate) with the
+// integer tensor-core path (mma.sync m16n8k32, s32 accumulate) with the
 // activations, quantized to 16 bits per 32-wide block and split into a signed high and a
 // signed low byte.  The int32 block sums are exact; they are folded into fp32 accumulators
 // with the block's fp16 weight scale and the block's activation scale, so the accumulation
@@ -20,11 +20,10 @@
 //
 // Kernels are launched with programmatic dependent launch: the weight copies are issued
 // before griddepcontrol.wait, so in a chain of dependent matvecs the next kernel's weights
-// stream while the previous kernel drains.  Batch 1 brings all packed activations into
-// shared memory with one more bulk copy; batches 2..16 bring each chunk's record into the
-// ring slot behind the tile.
+// stream while the previous kernel drains.  All packed activations come into
+// shared memory with one more bulk copy.
 //
-// Fused forms (batch 1, GemvFuse in qmm_common.cuh) let a chain of matvecs run without glue
+// Fused forms (GemvFuse in qmm_common.cuh) let a chain of matvecs run without glue
 // kernels between them: a matvec can pack its own fp32 input, apply the scalar 1/rms of an
 // RMSNorm to its row sums, and write the NEXT matvec's packed input (with the residual add and the
 // norm weights folded in) or silu(gate) * up from its epilogue.
@@ -33,6 +32,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "qmm_gemv_batch.cuh"
 #include "qmm_gemv_device.cuh"
 #include "qmm_kernels.h"
 #include "qmm_pack.cuh"
@@ -42,20 +42,18 @@ namespace qmm {
 namespace {
 
 // Shared memory of one CTA, carved from the dynamic allocation:
-//   slots  TILES*WARPS*DEPTH x (tile [+ batches 2..16: that chunk's activation record]) | mbarriers
-//   (+1 for the activations) | (batch 1) all activation records + 512 zero bytes | cross-warp reduction
-template <int FMT, int MC, int WARPS, int DEPTH, int TILES>
+//   slots  TILES*WARPS*DEPTH x tile | mbarriers (+1 for the activations) | all activation records + 512 zero bytes |
+//   cross-warp reduction
+template <int FMT, int WARPS, int DEPTH, int TILES>
 struct SmemPlan {
     static constexpr int NW = WARPS * TILES;
-    static constexpr int XCHUNK = MC == 1 ? 0 : XSlot<Cols<MC>::NCP>::BYTES;
-    static constexpr int SLOT = tile_bytes(FMT) + XCHUNK;
+    static constexpr int SLOT = tile_bytes(FMT);
     static constexpr int SLOTS_BYTES = NW * DEPTH * SLOT;
     static constexpr int BAR_OFF = SLOTS_BYTES;
     static constexpr int BAR_BYTES = (((NW * DEPTH + 1) * 8 + 15) / 16) * 16;
     static constexpr int X_OFF = BAR_OFF + BAR_BYTES;
-    __host__ __device__ static int x_bytes(int kc, int mc) { return mc == 1 ? (int)xpack1_bytes(kc) + 512 : 0; }
-    __host__ __device__ static int red_off(int kc, int mc) { return X_OFF + x_bytes(kc, mc); }
-    __host__ __device__ static int total(int kc, int mc) { return red_off(kc, mc) + NW * 16 * mc * 4; }
+    __host__ __device__ static int red_off(int kc) { return X_OFF + (int)xpack1_bytes(kc) + 512; }
+    __host__ __device__ static int total(int kc) { return red_off(kc) + NW * 16 * 4; }
 };
 
 // WARPS warps share one row tile; a CTA holds TILES row tiles (2 for EPI_RESID_PACK: the 32 rows of
@@ -64,22 +62,20 @@ struct SmemPlan {
 // 256 threads on every SM at once (42 registers at most): the bound keeps the fp32-packing prologue
 // and the fused epilogues from costing a second wave.  Plain CTAs of 128 threads are held to 64 registers, eight to an SM:
 // one row of Q6_K 11008 x 2048 takes 7.29 us, 7.70 with six to an SM; Q4_0 and Q8_0 differ by 1 % at most, either way.
-template <int MC, int THREADS, int EPI>
+template <int THREADS, int EPI>
 constexpr int gemv_min_blocks()
 {
-    return EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : MC > 1 ? 7 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
+    return EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
 }
 
-template <int FMT, int MC, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
-__global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS * TILES * 32, EPI>())
-    gemv_kernel(WeightView v, XPackView xp, float* __restrict__ y, int m, int* __restrict__ status, PeerScatter ps,
+template <int FMT, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
+__global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TILES * 32, EPI>())
+    gemv_kernel(WeightView v, XPackView xp, float* __restrict__ y, int* __restrict__ status, PeerScatter ps,
                 GemvFuse fu)
 {
-    using Plan = SmemPlan<FMT, MC, WARPS, DEPTH, TILES>;
+    using Plan = SmemPlan<FMT, WARPS, DEPTH, TILES>;
     constexpr int NW = WARPS * TILES;
-    constexpr int NOUT = Cols<MC>::NOUT;
     constexpr uint32_t TILE = tile_bytes(FMT);
-    static_assert(EPI == EPI_STORE || MC == 1, "fused epilogues exist for batch 1 only");
     static_assert(TILES == epi_tiles(EPI), "row tiles per CTA follow from the fused form");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float s_in_sh;  // 1/rms factor of the input activations
@@ -97,11 +93,9 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
     const int n_my = (wl < kc && tile_row < v.rt) ? (kc - wl + WARPS - 1) / WARPS : 0;
 
     // 1. start the weight stream: the first DEPTH tiles of this warp
-    // (batches 2..16: a slot's phase takes two arrivals, one with the tile's bytes, issued here, and
-    // one with the chunk's activation bytes, which can only be issued after the dependency wait)
     if (lane == 0) {
         for (int s = 0; s < DEPTH; ++s) {
-            mbar_init(&my_bars[s], MC == 1 ? 1 : 2);
+            mbar_init(&my_bars[s], 1);
         }
         if (warp == 0) {
             mbar_init(xbar, 1);
@@ -113,7 +107,7 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
                           &my_bars[s]);
         }
     }
-    if constexpr (MC == 1 && FMT == FMT_Q6_K) {
+    if constexpr (FMT == FMT_Q6_K) {
         // zero page for the lanes that carry no activation row
         uint32_t* z = reinterpret_cast<uint32_t*>(smem + Plan::X_OFF + xpack1_bytes(kc));
         for (int i = threadIdx.x; i < 128; i += NW * 32) {
@@ -125,107 +119,88 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
     pdl_wait();
 
     unsigned int epoch = 0;
-    if constexpr (MC == 1 && (EPI == EPI_STORE || EPI == EPI_RESID_PACK)) {
+    if constexpr (EPI == EPI_STORE || EPI == EPI_RESID_PACK) {
         if (ps.n_peers > 0) {
             epoch = (unsigned int)(*ps.pos * ps.sites + ps.site + 1);
         }
     }
-    XSrc<MC> xsrc;
+    XShared xsrc;
     bool ok = true;
     float h_pre = 0.0f, w_pre = 0.0f;  // EPI_RESID_PACK: residual and norm weight of this thread's row
-    if constexpr (MC == 1) {
-        uint8_t* xbase = smem + Plan::X_OFF;
-        const uint32_t xbytes = (uint32_t)xpack1_bytes(kc);
-        if (!XF32 && threadIdx.x == 0) {  // the thread that initialised xbar
-            mbar_expect_tx(xbar, xbytes);
-            bulk_copy_g2s(xbase, xp.base, xbytes, xbar);
-        }
-        if (warp == NW - 1) {
-            // the scalar RMSNorm factor of the input: the producer left one sum of squares per 32 activations
-            double t = 0.0;
-            if (fu.ss_in) {
-                for (int i = lane; i < fu.ss_count; i += 32) {
-                    t += fu.ss_in[i];
-                }
+    uint8_t* xbase = smem + Plan::X_OFF;
+    const uint32_t xbytes = (uint32_t)xpack1_bytes(kc);
+    if (!XF32 && threadIdx.x == 0) {  // the thread that initialised xbar
+        mbar_expect_tx(xbar, xbytes);
+        bulk_copy_g2s(xbase, xp.base, xbytes, xbar);
+    }
+    if (warp == NW - 1) {
+        // the scalar RMSNorm factor of the input: the producer left one sum of squares per 32 activations
+        double t = 0.0;
+        if (fu.ss_in) {
+            for (int i = lane; i < fu.ss_count; i += 32) {
+                t += fu.ss_in[i];
+            }
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
-                }
-            }
-            if (lane == 0) {
-                s_in_sh = fu.ss_in ? (float)(1.0 / sqrt(t / (double)fu.d_in + (double)fu.eps)) : 1.0f;
+            for (int o = 16; o > 0; o >>= 1) {
+                t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
             }
         }
-        if constexpr (EPI == EPI_RESID_PACK) {
-            if (threadIdx.x < 32) {
-                const int64_t row = (int64_t)blockIdx.x * 32 + threadIdx.x;
-                if (row < v.n) {
-                    h_pre = fu.h_in[row];
-                    w_pre = fu.norm_w[row];
-                }
-            }
-        }
-        if constexpr (XF32) {
-            // pack the fp32 activations here: spans of 128, one float4 per lane, all loads of a thread issued
-            // before the first is used.  Every CTA reads the same few KB: each starts at another span, so
-            // that the CTAs do not all ask the same L2 lines at the same moment.
-            const int nspan = (int)(v.k / 128);
-            constexpr int MAXS = 4;
-            const int rot = nspan > 0 ? (int)((blockIdx.x * 13u) % (unsigned)nspan) : 0;
-            const float* xsrc_f = fu.x_f32;
-            for (int s0 = warp; s0 < nspan; s0 += NW * MAXS) {
-                float4 xv[MAXS];
-#pragma unroll
-                for (int i = 0; i < MAXS; ++i) {
-                    const int sq = s0 + i * NW;
-                    if (sq < nspan) {
-                        const int sp = sq + rot < nspan ? sq + rot : sq + rot - nspan;
-                        xv[i] = __ldcg(reinterpret_cast<const float4*>(xsrc_f) + sp * 32 + lane);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < MAXS; ++i) {
-                    const int sq = s0 + i * NW;
-                    if (sq < nspan) {
-                        const int sp = sq + rot < nspan ? sq + rot : sq + rot - nspan;
-                        warp_pack_span128(xv[i], xbase + (size_t)(sp >> 1) * XPK1_REC, (sp & 1) * 4);
-                    }
-                }
-            }
-            for (int blk = nspan * 4 + warp; blk < kc * 8; blk += NW) {  // the ragged end, then zero blocks
-                const int64_t e = (int64_t)blk * 32 + lane;
-                warp_pack_block32(e < v.k ? __ldcg(xsrc_f + e) : 0.0f, xbase + (size_t)(blk >> 3) * XPK1_REC, blk & 7);
-            }
-        }
-        __syncthreads();  // xbar initialised, zero page written, activations packed
-        xsrc.base = xbase;
-        xsrc.zeros = xbase + xbytes;
-        if (!XF32 && !mbar_wait(xbar, 0)) {
-            ok = false;
-            if (lane == 0) {
-                atomicExch(status, 2);
-            }
-        }
-    } else {
-        if (threadIdx.x == 0) {
-            s_in_sh = 1.0f;
-        }
-        xsrc.base = nullptr;
         if (lane == 0) {
-            for (int s = 0; s < DEPTH && s < n_my; ++s) {
-                uint64_t* bar = &my_bars[s];
-                mbar_expect_tx(bar, Plan::XCHUNK);
-                bulk_copy_g2s(my_slots + (size_t)s * Plan::SLOT + TILE, xp.base + (size_t)(wl + s * WARPS) * Plan::XCHUNK,
-                              Plan::XCHUNK, bar);
+            s_in_sh = fu.ss_in ? (float)(1.0 / sqrt(t / (double)fu.d_in + (double)fu.eps)) : 1.0f;
+        }
+    }
+    if constexpr (EPI == EPI_RESID_PACK) {
+        if (threadIdx.x < 32) {
+            const int64_t row = (int64_t)blockIdx.x * 32 + threadIdx.x;
+            if (row < v.n) {
+                h_pre = fu.h_in[row];
+                w_pre = fu.norm_w[row];
             }
+        }
+    }
+    if constexpr (XF32) {
+        // pack the fp32 activations here: spans of 128, one float4 per lane, all loads of a thread issued
+        // before the first is used.  Every CTA reads the same few KB: each starts at another span, so
+        // that the CTAs do not all ask the same L2 lines at the same moment.
+        const int nspan = (int)(v.k / 128);
+        constexpr int MAXS = 4;
+        const int rot = nspan > 0 ? (int)((blockIdx.x * 13u) % (unsigned)nspan) : 0;
+        const float* xsrc_f = fu.x_f32;
+        for (int s0 = warp; s0 < nspan; s0 += NW * MAXS) {
+            float4 xv[MAXS];
+#pragma unroll
+            for (int i = 0; i < MAXS; ++i) {
+                const int sq = s0 + i * NW;
+                if (sq < nspan) {
+                    const int sp = sq + rot < nspan ? sq + rot : sq + rot - nspan;
+                    xv[i] = __ldcg(reinterpret_cast<const float4*>(xsrc_f) + sp * 32 + lane);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < MAXS; ++i) {
+                const int sq = s0 + i * NW;
+                if (sq < nspan) {
+                    const int sp = sq + rot < nspan ? sq + rot : sq + rot - nspan;
+                    warp_pack_span128(xv[i], xbase + (size_t)(sp >> 1) * XPK1_REC, (sp & 1) * 4);
+                }
+            }
+        }
+        for (int blk = nspan * 4 + warp; blk < kc * 8; blk += NW) {  // the ragged end, then zero blocks
+            const int64_t e = (int64_t)blk * 32 + lane;
+            warp_pack_block32(e < v.k ? __ldcg(xsrc_f + e) : 0.0f, xbase + (size_t)(blk >> 3) * XPK1_REC, blk & 7);
+        }
+    }
+    __syncthreads();  // xbar initialised, zero page written, activations packed
+    xsrc.base = xbase;
+    xsrc.zeros = xbase + xbytes;
+    if (!XF32 && !mbar_wait(xbar, 0)) {
+        ok = false;
+        if (lane == 0) {
+            atomicExch(status, 2);
         }
     }
 
-    float acc[NOUT];
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) {
-        acc[o] = 0.0f;
-    }
+    float acc[2] = {0.0f, 0.0f};
 
     // 3. consume tiles as they land; refill each slot right after it has been read
     for (int i = 0; i < n_my; ++i) {
@@ -238,12 +213,7 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
             }
         }
         if (ok) {
-            if constexpr (MC == 1) {
-                compute_chunk_m1<FMT>(my_slots + (size_t)s * Plan::SLOT, xsrc, wl + i * WARPS, lane, acc);
-            } else {
-                xsrc.attach(my_slots + (size_t)s * Plan::SLOT + TILE);
-                compute_chunk<FMT, MC>(my_slots + (size_t)s * Plan::SLOT, xsrc, lane, acc);
-            }
+            compute_chunk_m1<FMT>(my_slots + (size_t)s * Plan::SLOT, xsrc, wl + i * WARPS, lane, acc);
         }
         __syncwarp();
         if (ok && lane == 0 && i + DEPTH < n_my) {
@@ -251,61 +221,44 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<MC, WARPS 
             const int cn = wl + (i + DEPTH) * WARPS;
             mbar_expect_tx(&my_bars[s], TILE);
             bulk_copy_g2s(my_slots + (size_t)s * Plan::SLOT, my_tiles + (size_t)cn * TILE, TILE, &my_bars[s]);
-            if constexpr (MC > 1) {
-                mbar_expect_tx(&my_bars[s], Plan::XCHUNK);
-                bulk_copy_g2s(my_slots + (size_t)s * Plan::SLOT + TILE, xp.base + (size_t)cn * Plan::XCHUNK, Plan::XCHUNK,
-                              &my_bars[s]);
-            }
         }
     }
 
-    // 4. partial sums of the warps meet in shared memory: red[warp][row][activation row]
-    float* red = reinterpret_cast<float*>(smem + Plan::red_off(kc, MC));
+    // 4. partial sums of the warps meet in shared memory: red[warp][row]
+    float* red = reinterpret_cast<float*>(smem + Plan::red_off(kc));
     const int g = lane >> 2;
     const int t = lane & 3;
-    if constexpr (MC == 1) {
-        // lane t folded one block of every group of four
+    // lane t folded one block of every group of four
 #pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-            acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], o);
-            acc[1] += __shfl_xor_sync(0xFFFFFFFFu, acc[1], o);
-        }
-        if (t == 0) {
-            red[warp * 16 + g] = acc[0];
-            red[warp * 16 + g + 8] = acc[1];
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < Cols<MC>::NCP; ++j) {
-            red[(warp * 16 + g) * MC + 4 * j + t] = acc[2 * j + 0];
-            red[(warp * 16 + g + 8) * MC + 4 * j + t] = acc[2 * j + 1];
-        }
+    for (int o = 1; o < 4; o <<= 1) {
+        acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], o);
+        acc[1] += __shfl_xor_sync(0xFFFFFFFFu, acc[1], o);
+    }
+    if (t == 0) {
+        red[warp * 16 + g] = acc[0];
+        red[warp * 16 + g + 8] = acc[1];
     }
     __syncthreads();
     const float s_in = s_in_sh;
 
     if constexpr (EPI == EPI_STORE) {
-        for (int i = threadIdx.x; i < 16 * MC; i += NW * 32) {
-            const int col = i >> 4;
-            const int r = i & 15;
+        if (threadIdx.x < 16) {
             float sum = 0.0f;
 #pragma unroll
             for (int w = 0; w < WARPS; ++w) {
-                sum += red[(w * 16 + r) * MC + col];
+                sum += red[w * 16 + threadIdx.x];
             }
             sum *= s_in;
-            const int64_t row = (int64_t)blockIdx.x * 16 + r;
-            if (row < v.n && col < m) {
-                y[(int64_t)col * v.n + row] = sum;
-                if constexpr (MC == 1) {
-                    if (ps.n_peers > 0) {
+            const int64_t row = (int64_t)blockIdx.x * 16 + threadIdx.x;
+            if (row < v.n) {
+                y[row] = sum;
+                if (ps.n_peers > 0) {
 #pragma unroll
-                        for (int p = 0; p < QMM_MAX_PEERS; ++p) {  // over NVLink into the peer's receive buffer
-                            if (p < ps.n_peers) {
-                                asm volatile("st.relaxed.sys.global.v2.u32 [%0], {%1, %2};" ::"l"(ps.dst[p] + row),
-                                             "r"(__float_as_uint(sum)), "r"(epoch)
-                                             : "memory");
-                            }
+                    for (int p = 0; p < QMM_MAX_PEERS; ++p) {  // over NVLink into the peer's receive buffer
+                        if (p < ps.n_peers) {
+                            asm volatile("st.relaxed.sys.global.v2.u32 [%0], {%1, %2};" ::"l"(ps.dst[p] + row),
+                                         "r"(__float_as_uint(sum)), "r"(epoch)
+                                         : "memory");
                         }
                     }
                 }
@@ -418,14 +371,14 @@ struct Tune {
     static constexpr int DEPTH = FMT == FMT_Q8_0 ? 2 : 3;
 };
 
-template <int FMT, int MC, int WARPS, int DEPTH, int EPI, bool XF32>
-cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
+template <int FMT, int WARPS, int DEPTH, int EPI, bool XF32>
+cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y, int* status,
                              const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
 {
     constexpr int TILES = epi_tiles(EPI);
-    using Plan = SmemPlan<FMT, MC, WARPS, DEPTH, TILES>;
-    auto kernel = gemv_kernel<FMT, MC, WARPS, DEPTH, EPI, TILES, XF32>;
-    int smem = Plan::total(w.kc, MC);
+    using Plan = SmemPlan<FMT, WARPS, DEPTH, TILES>;
+    auto kernel = gemv_kernel<FMT, WARPS, DEPTH, EPI, TILES, XF32>;
+    int smem = Plan::total(w.kc);
     if (smem > 227 * 1024) {
         return cudaErrorInvalidConfiguration;
     }
@@ -479,22 +432,22 @@ cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y,
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 1;
     cfg.attrs = attr;
-    return cudaLaunchKernelEx(&cfg, kernel, w, xp, y, m, status, ps, fu);
+    return cudaLaunchKernelEx(&cfg, kernel, w, xp, y, status, ps, fu);
 }
 
-template <int FMT, int MC, int WARPS, int DEPTH, int EPI>
-cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
+template <int FMT, int WARPS, int DEPTH, int EPI>
+cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float* y, int* status,
                                 const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
 {
-    if constexpr (MC == 1 && EPI != EPI_SWIGLU && EPI != EPI_SWIGLU_PACK) {
+    if constexpr (EPI != EPI_SWIGLU && EPI != EPI_SWIGLU_PACK) {
         if (fu.x_f32 != nullptr) {
-            return launch_gemv_xsrc<FMT, MC, WARPS, DEPTH, EPI, true>(w, xp, y, m, status, ps, fu, stream);
+            return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, true>(w, xp, y, status, ps, fu, stream);
         }
     }
     if (fu.x_f32 != nullptr) {
         return cudaErrorInvalidValue;
     }
-    return launch_gemv_xsrc<FMT, MC, WARPS, DEPTH, EPI, false>(w, xp, y, m, status, ps, fu, stream);
+    return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, false>(w, xp, y, status, ps, fu, stream);
 }
 
 // Batch 1: warps x ring slots by row length.
@@ -531,48 +484,38 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         const int budget = 232448 / per_sm - 1280;
         // 4-bit rows of up to 16 chunks: four warps with four slots, every tile requested at once (7B-shape step with eight
         // blocks 304.9 -> 302.5 us against eight warps with one slot)
-        if (tile_bytes(FMT) == 2304 && w.kc > 8 && w.kc <= 16 && SmemPlan<FMT, 1, 4, 4, 2>::total(w.kc, 1) <= budget) {
-            return launch_gemv_variant<FMT, 1, 4, 4, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        if (tile_bytes(FMT) == 2304 && w.kc > 8 && w.kc <= 16 && SmemPlan<FMT, 4, 4, 2>::total(w.kc) <= budget) {
+            return launch_gemv_variant<FMT, 4, 4, EPI>(w, xp, y, status, ps, fu, stream);
         }
-        if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0 && SmemPlan<FMT, 1, 8, 1, 2>::total(w.kc, 1) <= budget) {
-            return launch_gemv_variant<FMT, 1, 8, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0 && SmemPlan<FMT, 8, 1, 2>::total(w.kc) <= budget) {
+            return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
         }
-        if (w.kc > 16 && SmemPlan<FMT, 1, 8, 3, 2>::total(w.kc, 1) <= budget) {
-            return launch_gemv_variant<FMT, 1, 8, 3, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        if (w.kc > 16 && SmemPlan<FMT, 8, 3, 2>::total(w.kc) <= budget) {
+            return launch_gemv_variant<FMT, 8, 3, EPI>(w, xp, y, status, ps, fu, stream);
         }
-        if (SmemPlan<FMT, 1, 4, 3, 2>::total(w.kc, 1) <= budget) {
-            return launch_gemv_variant<FMT, 1, 4, 3, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        if (SmemPlan<FMT, 4, 3, 2>::total(w.kc) <= budget) {
+            return launch_gemv_variant<FMT, 4, 3, EPI>(w, xp, y, status, ps, fu, stream);
         }
-        if (SmemPlan<FMT, 1, 4, 2, 2>::total(w.kc, 1) <= budget) {
-            return launch_gemv_variant<FMT, 1, 4, 2, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        if (SmemPlan<FMT, 4, 2, 2>::total(w.kc) <= budget) {
+            return launch_gemv_variant<FMT, 4, 2, EPI>(w, xp, y, status, ps, fu, stream);
         }
         // more than one CTA per SM wanted and nothing deeper fits: one slot per warp, the number of CTAs keeps
         // the bytes in flight up
-        return launch_gemv_variant<FMT, 1, 4, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        return launch_gemv_variant<FMT, 4, 1, EPI>(w, xp, y, status, ps, fu, stream);
     }
     if (tile_bytes(FMT) == 2304 && EPI == EPI_STORE && fu.ss_in != nullptr && w.kc > 8 && w.kc <= 16) {
-        return launch_gemv_variant<FMT, 1, 4, 2, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        return launch_gemv_variant<FMT, 4, 2, EPI>(w, xp, y, status, ps, fu, stream);
     }
     if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0) {
-        return launch_gemv_variant<FMT, 1, 8, 1, EPI>(w, xp, y, 1, status, ps, fu, stream);
+        return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
     }
-    if (w.kc > 32 && SmemPlan<FMT, 1, 16, 2, 1>::total(w.kc, 1) <= LIMIT) {
-        return launch_gemv_variant<FMT, 1, 16, 2, EPI>(w, xp, y, 1, status, ps, fu, stream);
+    if (w.kc > 32 && SmemPlan<FMT, 16, 2, 1>::total(w.kc) <= LIMIT) {
+        return launch_gemv_variant<FMT, 16, 2, EPI>(w, xp, y, status, ps, fu, stream);
     }
-    if (w.kc > 16 && SmemPlan<FMT, 1, 8, 3, TILES>::total(w.kc, 1) <= LIMIT) {
-        return launch_gemv_variant<FMT, 1, 8, 3, EPI>(w, xp, y, 1, status, ps, fu, stream);
+    if (w.kc > 16 && SmemPlan<FMT, 8, 3, TILES>::total(w.kc) <= LIMIT) {
+        return launch_gemv_variant<FMT, 8, 3, EPI>(w, xp, y, status, ps, fu, stream);
     }
-    return launch_gemv_variant<FMT, 1, Tune<FMT>::WARPS, Tune<FMT>::DEPTH, EPI>(w, xp, y, 1, status, ps, fu, stream);
-}
-
-template <int FMT, int MC>
-cudaError_t launch_gemv_batch(const WeightView& w, const XPackView& xp, float* y, int m, int* status, cudaStream_t stream)
-{
-    // batches 2..16 carry 3-10 KB of activations per slot: a shallower ring keeps 2-3 CTAs per SM
-    constexpr int DEPTH = MC == 4 && FMT != FMT_Q8_0 ? 3 : 2;
-    const PeerScatter none = {};
-    const GemvFuse plain = {};
-    return launch_gemv_variant<FMT, MC, Tune<FMT>::WARPS, DEPTH, EPI_STORE>(w, xp, y, m, status, none, plain, stream);
+    return launch_gemv_variant<FMT, Tune<FMT>::WARPS, Tune<FMT>::DEPTH, EPI>(w, xp, y, status, ps, fu, stream);
 }
 
 template <int FMT>
@@ -587,7 +530,7 @@ cudaError_t launch_gemv_fmt(const WeightView& w, const XPackView& xp, float* y, 
         // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
         // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
         // 7B-shape step slower)
-        case EPI_SWIGLU_PACK: return launch_gemv_variant<FMT, 1, 2, 2, EPI_SWIGLU_PACK>(w, xp, y, 1, status, ps, fu, stream);
+        case EPI_SWIGLU_PACK: return launch_gemv_variant<FMT, 2, 2, EPI_SWIGLU_PACK>(w, xp, y, status, ps, fu, stream);
         default: return cudaErrorInvalidValue;
         }
     }
@@ -595,15 +538,15 @@ cudaError_t launch_gemv_fmt(const WeightView& w, const XPackView& xp, float* y, 
         return cudaErrorInvalidValue;
     }
     if (m <= 4) {
-        return launch_gemv_batch<FMT, 4>(w, xp, y, m, status, stream);
+        return launch_gemv_batch<FMT, 1>(w, xp, y, m, status, stream);
     }
     if (m <= 8) {
-        return launch_gemv_batch<FMT, 8>(w, xp, y, m, status, stream);
+        return launch_gemv_batch<FMT, 2>(w, xp, y, m, status, stream);
     }
     if (m <= 12) {
-        return launch_gemv_batch<FMT, 12>(w, xp, y, m, status, stream);
+        return launch_gemv_batch<FMT, 3>(w, xp, y, m, status, stream);
     }
-    return launch_gemv_batch<FMT, 16>(w, xp, y, m, status, stream);
+    return launch_gemv_batch<FMT, 4>(w, xp, y, m, status, stream);
 }
 
 }  // namespace

@@ -134,14 +134,20 @@ __device__ __forceinline__ void warp_pack_chunk(const float (&v)[8], uint8_t* re
 // activations half*16 + 4t .. +3 of block b, and the block's meta entry.
 __device__ __forceinline__ uint32_t* xpack_word(uint8_t* rec, int ncp, int row, int b, int digit, int t, int half)
 {
-    const int lane = ncp == 0 ? b * 8 + 4 * digit + t : (b * ncp + (row >> 2)) * 32 + 4 * (2 * (row & 3) + digit) + t;
-    return reinterpret_cast<uint32_t*>(rec) + (lane * 2 + half);
+    return reinterpret_cast<uint32_t*>(rec) +
+           (ncp == 0 ? (b * 8 + 4 * digit + t) * 2 + half : xpack_word_at(ncp, row, b, digit, t, half));
 }
 
 __device__ __forceinline__ void xpack_meta(uint8_t* rec, int ncp, int row, int b, int q, float amax)
 {
-    int4* meta = reinterpret_cast<int4*>(rec + (ncp == 0 ? XPK1_META : xpack_xq_bytes(ncp)));
-    meta[ncp == 0 ? b : b * 16 + row] = make_int4(8 * q, 128 * q, __float_as_int(amax / 32639.0f), 0);
+    if (ncp == 0) {
+        reinterpret_cast<int4*>(rec + XPK1_META)[b] = make_int4(8 * q, 128 * q, __float_as_int(amax / 32639.0f), 0);
+    } else {
+        float* meta = reinterpret_cast<float*>(rec + xpack_xq_bytes(ncp)) + b * 16 + xpack_meta_pos(ncp, row);
+        const float xs = amax / 32639.0f;
+        meta[0] = xs;
+        meta[XPK_META_PLANE / 4] = (float)(8 * q) * xs;
+    }
 }
 
 __device__ __forceinline__ size_t xpack_row_rec_bytes(int ncp)
