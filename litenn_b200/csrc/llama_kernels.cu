@@ -63,10 +63,12 @@ __device__ __forceinline__ double block_sum_double(double v, double* red)
 __global__ void embed_row_kernel(int fmt, const uint8_t* __restrict__ raw, const int* __restrict__ tokens, int n_rows,
                                  int d, float* __restrict__ h)
 {
+    pdl_trigger();
+    pdl_sync();
     const int elems = block_elems(fmt), bytes = block_bytes(fmt);
     const int64_t row_bytes = (int64_t)(d / elems) * bytes;
     for (int r = blockIdx.y; r < n_rows; r += gridDim.y) {
-        const uint8_t* row = raw + (int64_t)tokens[r] * row_bytes;
+        const uint8_t* row = raw + (int64_t)__ldcg(tokens + r) * row_bytes;
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d; i += gridDim.x * blockDim.x) {
             h[(int64_t)r * d + i] = dequant_raw_element(fmt, row + (i / elems) * bytes, i % elems);
         }
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(128) resid_pack_kernel(const float* __restrict
                 pk[r] = ld_sys_v2(pg.recv + (size_t)r * d + e);
             }
         }
-        const float own = add[e];
+        const float own = __ldcg(add + e);
 #pragma unroll
         for (int r = 0; r < MAXR; ++r) {
             if (r < pg.tp_size) {
@@ -194,9 +196,9 @@ __global__ void __launch_bounds__(128) resid_pack_kernel(const float* __restrict
             }
         }
     } else if (add) {
-        a = add[e];
+        a = __ldcg(add + e);
     }
-    emit_block32(h_in[e] + a, group, e, w, h_out, packed, ss_out);
+    emit_block32(__ldcg(h_in + e) + a, group, e, w, h_out, packed, ss_out);
 }
 
 // cos/sin tables [max_seq][rope_dim/2], computed in double and cast (Layer/RoPE.h:22-39).
@@ -726,7 +728,7 @@ __global__ void __launch_bounds__(256) resid_rmsnorm_rows_kernel(float* __restri
         for (int j = 0; j < KEEP; ++j) {
             const int i = threadIdx.x + j * 256;
             if (i < n4) {
-                const float4 a = ar[i];
+                const float4 a = __ldcg(ar + i);
                 keep[j].x += a.x;
                 keep[j].y += a.y;
                 keep[j].z += a.z;
@@ -743,7 +745,7 @@ __global__ void __launch_bounds__(256) resid_rmsnorm_rows_kernel(float* __restri
     for (int i = threadIdx.x + KEEP * 256; i < n4; i += 256) {  // rows longer than 8192
         float4 v = hr[i];
         if (ar) {
-            const float4 a = ar[i];
+            const float4 a = __ldcg(ar + i);
             v = make_float4(v.x + a.x, v.y + a.y, v.z + a.z, v.w + a.w);
             hr[i] = v;
         }
@@ -834,13 +836,15 @@ __device__ __forceinline__ void store_ctx(float* p, float a, float b)  // tests 
     *reinterpret_cast<float2*>(p) = make_float2(a, b);
 }
 
+// (The prefill attention kernels take plain pointers: what they read is written by kernels that may still run when they start,
+// and loads of read-only data need not stay behind the dependency wait.)
 // Causal attention for rows row0..row0+ROWS-1 of one head (those below m) by one warp, fp32 arithmetic throughout: it
 // reuses each loaded batch of eight keys for all of its rows; a row simply ignores the keys beyond its own position.
 // Online softmax per row, one rescale per batch.
 template <int DPL, int ROWS, typename OutT>
-__device__ __forceinline__ void attn_rows(const float* __restrict__ qkv, int row_stride, int m, int pos0, int n_heads,
-                                          int n_kv, int max_seq, const __half* __restrict__ cache_k,
-                                          const __half* __restrict__ cache_v, OutT* __restrict__ ctx, int row0, int head)
+__device__ __forceinline__ void attn_rows(const float* qkv, int row_stride, int m, int pos0, int n_heads,
+                                          int n_kv, int max_seq, const __half* cache_k,
+                                          const __half* cache_v, OutT* ctx, int row0, int head)
 {
     constexpr int hd = 32 * DPL;
     const int lane = threadIdx.x & 31;
@@ -923,10 +927,10 @@ __device__ __noinline__ void attn_rows_again(const float* qkv, int row_stride, i
 // sums, and a warp that finds one does its rows again in fp32, key by key.
 template <int HD, typename OutT>
 __global__ void __launch_bounds__(128, HD == 128 ? 2 : 3)  // what its shared memory lets an SM hold at HD = 128
-    attn_prefill_kernel(const float* __restrict__ qkv, int row_stride, int m,
+    attn_prefill_kernel(const float* qkv, int row_stride, int m,
                                                            int pos0, int n_heads, int n_kv, int max_seq,
-                                                           const __half* __restrict__ cache_k,
-                                                           const __half* __restrict__ cache_v, OutT* __restrict__ ctx)
+                                                           const __half* cache_k,
+                                                           const __half* cache_v, OutT* ctx)
 {
     constexpr int KT = 64;                 // keys per tile
     constexpr int ROW = HD * 2;            // bytes of a key row
@@ -1145,6 +1149,7 @@ __global__ void __launch_bounds__(128, HD == 128 ? 2 : 3)  // what its shared me
         }
         __syncthreads();  // the buffer is refilled two tiles from now
     }
+    pdl_trigger();  // not earlier: the next GEMM's CTAs would take the SMs that this grid leaves free, two to an SM
     bool finite = true;
 #pragma unroll
     for (int rs = 0; rs < 2; ++rs) {
@@ -1174,12 +1179,14 @@ __global__ void __launch_bounds__(128, HD == 128 ? 2 : 3)  // what its shared me
 // A few rows at a time, where a 64-row tile of the kernel above would be mostly padding: one warp per four rows of a
 // head.  Bound by the L2 reads of K and V (every row streams the whole prefix of its head).
 template <int DPL, int ROWS, typename OutT>
-__global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __restrict__ qkv, int row_stride, int m,
+__global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* qkv, int row_stride, int m,
                                                                 int pos0, int n_heads, int n_kv, int max_seq,
-                                                                const __half* __restrict__ cache_k,
-                                                                const __half* __restrict__ cache_v,
-                                                                OutT* __restrict__ ctx)
+                                                                const __half* cache_k,
+                                                                const __half* cache_v,
+                                                                OutT* ctx)
 {
+    pdl_trigger();
+    pdl_sync();
     const int groups = (m + ROWS - 1) / ROWS;
     const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (wid < (int64_t)groups * n_heads) {
@@ -1187,6 +1194,22 @@ __global__ void __launch_bounds__(128) attn_prefill_rows_kernel(const float* __r
         attn_rows<DPL, ROWS>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx,
                              (groups - 1 - (int)(wid / n_heads)) * ROWS, (int)(wid % n_heads));
     }
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 template <typename OutT>
@@ -1198,8 +1221,8 @@ cudaError_t attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_k
         constexpr int ROWS = 4;
         const unsigned ctas = (unsigned)(((m + ROWS - 1) / ROWS * n_heads + 3) / 4);
         auto kernel = hd == 64 ? attn_prefill_rows_kernel<2, ROWS, OutT> : attn_prefill_rows_kernel<4, ROWS, OutT>;
-        kernel<<<ctas, 128, 0, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
-        return cudaGetLastError();
+        return launch_pdl(kernel, dim3(ctas), dim3(128), 0, st, qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v,
+                          ctx);
     }
     const dim3 grid((unsigned)((m + 63) / 64), (unsigned)n_heads);
     auto launch = [&](auto kernel) -> cudaError_t {
@@ -1208,6 +1231,8 @@ cudaError_t attn_prefill(const float* qkv, int m, int pos0, int n_heads, int n_k
         if (e != cudaSuccess) {
             return e;
         }
+        // not ahead of the kernel before: its 112 KB per CTA would keep that kernel's own CTAs waiting (128 tokens, four 7B-shape
+        // blocks 733 us against 762)
         kernel<<<grid, 128, smem, st>>>(qkv, row_stride, m, pos0, n_heads, n_kv, max_seq, cache_k, cache_v, ctx);
         return cudaGetLastError();
     };
@@ -1233,22 +1258,6 @@ __global__ void __launch_bounds__(256) silu_mul_rows_kernel(const float* __restr
                         (g.z * (1.0f / (1.0f + expf(-g.z)))) * u.z, (g.w * (1.0f / (1.0f + expf(-g.w)))) * u.w);
     }
     out.put(blockIdx.y, i4, o, ok);
-}
-
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 template <typename... KArgs, typename... Args>
@@ -1282,8 +1291,8 @@ cudaError_t ll_rope_tables(int max_seq, int rope_dim, double theta, float* rope_
 
 cudaError_t ll_embed_rows(int fmt, const uint8_t* raw, const int* tokens, int n_rows, int d, float* h, cudaStream_t st)
 {
-    embed_row_kernel<<<dim3((d + 255) / 256, n_rows < 1024 ? n_rows : 1024), 256, 0, st>>>(fmt, raw, tokens, n_rows, d, h);
-    return cudaGetLastError();
+    return launch_pdl(embed_row_kernel, dim3((d + 255) / 256, n_rows < 1024 ? n_rows : 1024), dim3(256), 0, st, fmt, raw, tokens,
+                      n_rows, d, h);
 }
 
 cudaError_t ll_embed_pack(int fmt, const uint8_t* raw, const int* token, int d, const float* w, float* h,

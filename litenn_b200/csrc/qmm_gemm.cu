@@ -159,8 +159,10 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == DW) {
-        // ---- TMA producer: tokens ----
+        // ---- TMA producer: tokens.  Only they come from an earlier kernel; the first weights are dequantized while it drains,
+        // and what is stored in the end depends on the tokens ----
         if (lane == 0) {
+            g_pdl_wait();
             int slot = 0;
             uint32_t phase = 1;
             for (int s = 0; s < n_steps; ++s) {
@@ -217,6 +219,10 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         if (ok && elect_one()) {
             umma_commit(accum);
         }
+        // The next kernel may start while this one stores its results.  Not earlier: its CTAs would take the places that this
+        // kernel's grid leaves free, two to an SM, and leave others without (128 tokens, eight 7B-shape blocks: 1488 us without
+        // overlap, 1591 with the start of this kernel as the trigger)
+        g_pdl_launch_dependents();
         __syncwarp();
     } else {
         // ---- dequant producers: weights -> TMEM ----
@@ -404,7 +410,7 @@ cudaError_t launch_gemm_nb(const CUtensorMap& xmap, const GemmArgs& args, const 
 {
     auto kernel = gemm_ts_kernel<FMT, NB>;
     static bool configured[64] = {};
-    constexpr int LIMIT = NB == 2 ? 204 * 1024 : 113 * 1024;
+    constexpr int LIMIT = 204 * 1024;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
@@ -427,13 +433,15 @@ cudaError_t launch_gemm_nb(const CUtensorMap& xmap, const GemmArgs& args, const 
     cfg.blockDim = dim3((8 * NB + 2) * 32);
     cfg.dynamicSmemBytes = (size_t)plan.smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)plan.splits;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, xmap, args);
 }
 
@@ -463,6 +471,9 @@ GemmPlan gemm_form(const WeightView& w, int64_t m, int sm_count, int nb, int tok
     p.ring = std::min(GEMM_MAX_RING, room / (tokens * 128));
     const int part_bytes = splits > 1 ? tokens * 128 * 4 : 0;
     p.smem = 1024 /*alignment*/ + GEMM_BAR_BYTES + std::max(p.ring * tokens * 128, part_bytes);
+    if (nb == 1 && p.grid <= sm_count) {
+        p.smem = std::max(p.smem, 116 * 1024);  // one CTA per SM, also where the kernel before still holds some SMs
+    }
     return p;
 }
 

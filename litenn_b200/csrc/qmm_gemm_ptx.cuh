@@ -66,6 +66,17 @@ __device__ __forceinline__ bool g_mbar_wait_warp(uint64_t* bar, uint32_t parity)
     return __all_sync(0xFFFFFFFFu, g_mbar_wait(bar, parity));
 }
 
+// Programmatic dependent launch: the next kernel of the stream may start its prologue; everything that earlier kernels of
+// the stream wrote is visible.
+__device__ __forceinline__ void g_pdl_launch_dependents()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void g_pdl_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // True in one lane of a converged warp.  MMAs are issued under this and not under a lane comparison: the compiler then
 // knows that their operands are uniform.
 __device__ __forceinline__ bool elect_one()

@@ -185,8 +185,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        // ---- TMA producer: activations ----
+        // ---- TMA producer: activations.  Only they come from an earlier kernel; the first weights are dequantized while it
+        // drains, and what is stored in the end depends on the activations ----
         if (lane == 0) {
+            g_pdl_wait();
             for (int s = 0; s < n_stages; ++s) {
                 const int slot = s % GEMM_STAGES;
                 if (s >= GEMM_STAGES && !g_mbar_poll(&empty[slot], (uint32_t)(s / GEMM_STAGES - 1) & 1u)) {
@@ -235,6 +237,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         if (ok && elect_one()) {
             umma_commit(accum);
         }
+        g_pdl_launch_dependents();  // the next kernel may start while this one stores its results
         __syncwarp();
     } else {
         // ---- dequant producers: weights -> bf16 B tile ----
@@ -411,8 +414,17 @@ cudaError_t launch_smem_exact(const CUtensorMap& xmap, const GemmArgs& args, int
             configured[dev] = true;
         }
     }
-    kernel<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(xmap, args);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, xmap, args);
 }
 
 template <int FMT>

@@ -94,16 +94,18 @@ template <bool VEC>
 __global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ x, int64_t count,
                                                           unsigned short* __restrict__ out)
 {
+    pdl_launch_dependents();
+    pdl_wait();  // x may come from the previous kernel; the buffer may still be read by it
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     if constexpr (VEC) {
         for (int64_t i = first; i < count / 4; i += step) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(x) + i);
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(x) + i);
             reinterpret_cast<uint2*>(out)[i] =
                 make_uint2(bf16_bits(v.x) | (bf16_bits(v.y) << 16), bf16_bits(v.z) | (bf16_bits(v.w) << 16));
         }
     } else {
         for (int64_t i = first; i < count; i += step) {
-            out[i] = (unsigned short)bf16_bits(x[i]);
+            out[i] = (unsigned short)bf16_bits(__ldcg(x + i));
         }
     }
 }
@@ -117,12 +119,16 @@ cudaError_t launch_f32_to_bf16(const float* x, int64_t count, void* out_bf16, cu
                      (reinterpret_cast<uintptr_t>(out_bf16) & 7u) == 0;
     const int64_t blocks = ((vec ? count / 4 : count) + 255) / 256;
     const unsigned grid = (unsigned)(blocks < 4096 ? blocks : 4096);
-    if (vec) {
-        f32_to_bf16_kernel<true><<<grid, 256, 0, stream>>>(x, count, out);
-    } else {
-        f32_to_bf16_kernel<false><<<grid, 256, 0, stream>>>(x, count, out);
-    }
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, vec ? f32_to_bf16_kernel<true> : f32_to_bf16_kernel<false>, x, count, out);
 }
 
 cudaError_t launch_pack_x(const float* x, int m, int64_t k, int kc, uint8_t* out, cudaStream_t stream)
