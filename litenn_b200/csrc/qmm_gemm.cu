@@ -471,8 +471,11 @@ GemmPlan gemm_form(const WeightView& w, int64_t m, int sm_count, int nb, int tok
     p.ring = std::min(GEMM_MAX_RING, room / (tokens * 128));
     const int part_bytes = splits > 1 ? tokens * 128 * 4 : 0;
     p.smem = 1024 /*alignment*/ + GEMM_BAR_BYTES + std::max(p.ring * tokens * 128, part_bytes);
-    if (nb == 1 && p.grid <= sm_count) {
-        p.smem = std::max(p.smem, 116 * 1024);  // one CTA per SM, also where the kernel before still holds some SMs
+    // One CTA per SM, also where the kernel before still holds some SMs.  Clusters of four and eight leave SMs of a GPC
+    // over: 15 clusters of eight fit a B200 this way (Q4_0, K = 4096, 48 rows: 9.0 us for 120 CTAs, 15.2 for 128 and 9.5 for
+    // 136 at two to an SM), so beyond 13/16 of the SMs they may share.
+    if (nb == 1 && p.grid <= (splits >= 4 ? sm_count * 13 / 16 : sm_count)) {
+        p.smem = std::max(p.smem, 116 * 1024);
     }
     return p;
 }
