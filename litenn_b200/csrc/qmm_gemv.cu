@@ -152,6 +152,26 @@ cudaError_t launch_unpack_x(const uint8_t* packed, int64_t k, float* x, cudaStre
     return cudaGetLastError();
 }
 
+// One launch instead of two while every SM's copy of the vector costs less than the packing kernel and its boundary (1.1 us
+// of a stream, 2.6 us of a host loop, where 1024 x 4096 falls from 7.0 to 5.2 us).  Up to 32 chunks it does, the one wave
+// being also the better matvec; above, packing 11008 values takes 256 rows of Q4_0 5.5 us and not 4.4, and only Q8_0
+// on one row tile per SM gains (7.5 -> 5.9).  Q8_0 beyond 16 chunks is bound by its bytes either way (28672 x 8192: 39.7
+// us, 40.5 in one launch).  Of many tiles per SM only the 4-bit formats have room for enough slots.
+bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count)
+{
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || w.k % 32 != 0 || sm_count < 1) {  // x is read 16 bytes at a time
+        return false;
+    }
+    const int tiles = (w.rt + sm_count - 1) / sm_count;
+    if (w.kc > 32) {
+        return w.fmt == FMT_Q8_0 && tiles == 1 && w.kc <= 112;
+    }
+    if (w.fmt == FMT_Q8_0) {
+        return tiles <= (w.kc > 16 ? 2 : 16);
+    }
+    return tiles <= (w.fmt == FMT_Q6_K ? 16 : 28);
+}
+
 cudaError_t launch_gemv_fused(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                               const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
 {

@@ -29,7 +29,7 @@
 // norm weights folded in) or silu(gate) * up from its epilogue.
 #pragma once
 
-#include <cstdlib>
+#include <atomic>
 #include <mutex>
 
 #include "qmm_gemv_batch.cuh"
@@ -62,21 +62,21 @@ struct SmemPlan {
 // 256 threads on every SM at once (42 registers at most): the bound keeps the fp32-packing prologue
 // and the fused epilogues from costing a second wave.  Plain CTAs of 128 threads are held to 64 registers, eight to an SM:
 // one row of Q6_K 11008 x 2048 takes 7.29 us, 7.70 with six to an SM; Q4_0 and Q8_0 differ by 1 % at most, either way.
-template <int THREADS, int EPI>
+template <int THREADS, int EPI, int TILES, bool XF32>
 constexpr int gemv_min_blocks()
 {
-    return EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
+    return TILES > epi_tiles(EPI) || (XF32 && EPI == EPI_STORE) || EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
 }
 
 template <int FMT, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
-__global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TILES * 32, EPI>())
+__global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TILES * 32, EPI, TILES, XF32>())
     gemv_kernel(WeightView v, XPackView xp, float* __restrict__ y, int* __restrict__ status, PeerScatter ps,
                 GemvFuse fu)
 {
     using Plan = SmemPlan<FMT, WARPS, DEPTH, TILES>;
     constexpr int NW = WARPS * TILES;
     constexpr uint32_t TILE = tile_bytes(FMT);
-    static_assert(TILES == epi_tiles(EPI), "row tiles per CTA follow from the fused form");
+    static_assert(TILES % epi_tiles(EPI) == 0, "a fused form's group of row tiles stays in one CTA");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float s_in_sh;  // 1/rms factor of the input activations
 
@@ -150,8 +150,8 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
         }
     }
     if constexpr (EPI == EPI_RESID_PACK) {
-        if (threadIdx.x < 32) {
-            const int64_t row = (int64_t)blockIdx.x * 32 + threadIdx.x;
+        if (threadIdx.x < 16 * TILES) {
+            const int64_t row = (int64_t)blockIdx.x * (16 * TILES) + threadIdx.x;
             if (row < v.n) {
                 h_pre = fu.h_in[row];
                 w_pre = fu.norm_w[row];
@@ -242,14 +242,15 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
     const float s_in = s_in_sh;
 
     if constexpr (EPI == EPI_STORE) {
-        if (threadIdx.x < 16) {
+        if (threadIdx.x < 16 * TILES) {
             float sum = 0.0f;
+            const int w0 = ((int)threadIdx.x >> 4) * WARPS, r = threadIdx.x & 15;
 #pragma unroll
             for (int w = 0; w < WARPS; ++w) {
-                sum += red[w * 16 + threadIdx.x];
+                sum += red[(w0 + w) * 16 + r];
             }
             sum *= s_in;
-            const int64_t row = (int64_t)blockIdx.x * 16 + threadIdx.x;
+            const int64_t row = (int64_t)blockIdx.x * (16 * TILES) + threadIdx.x;
             if (row < v.n) {
                 y[row] = sum;
                 if (ps.n_peers > 0) {
@@ -265,15 +266,16 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
             }
         }
     } else if constexpr (EPI == EPI_RESID_PACK) {
-        if (warp == 0) {  // lane = row within the CTA's 32 rows: warps lane/16*WARPS .. +WARPS-1 hold its partial sums
+        const int64_t blk = (int64_t)blockIdx.x * (TILES / 2) + warp;  // block of 32 output rows of this warp
+        if (warp < TILES / 2 && blk * 32 < v.n) {  // lane = row of the block: the warps of its tile hold the partial sums
             float sum = 0.0f;
-            const int w0 = (lane >> 4) * WARPS, r = lane & 15;
+            const int w0 = (2 * warp + (lane >> 4)) * WARPS, r = lane & 15;
 #pragma unroll
             for (int w = 0; w < WARPS; ++w) {
                 sum += red[(w0 + w) * 16 + r];
             }
             sum *= s_in;
-            const int64_t row = (int64_t)blockIdx.x * 32 + lane;
+            const int64_t row = blk * 32 + lane;
             if (ps.n_peers > 0 && row < v.n) {
                 // tensor parallelism: this rank's partial goes to every peer, the peers' partials are awaited
 #pragma unroll
@@ -323,13 +325,15 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
                 sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
             }
             if (lane == 0) {
-                fu.ss_out[blockIdx.x] = sq;
+                fu.ss_out[blk] = sq;
             }
-            warp_pack_block32(hv * w_pre, fu.packed_out + (size_t)(blockIdx.x >> 3) * XPK1_REC, blockIdx.x & 7);
+            warp_pack_block32(hv * w_pre, fu.packed_out + (size_t)(blk >> 3) * XPK1_REC, (int)(blk & 7));
         }
     } else if constexpr (EPI == EPI_SWIGLU_PACK) {
-        if (warp == 0) {  // lane = channel within the CTA's 32: row tile lane / 8, tile rows lane % 8 (gate) and + 8 (up)
-            const int w0 = (lane >> 3) * WARPS, r = lane & 7;
+        const int64_t blk = (int64_t)blockIdx.x * (TILES / 4) + warp;  // block of 32 channels of this warp
+        if (warp < TILES / 4 && blk * 64 < v.n) {
+            // lane = channel of the block: row tile lane / 8, tile rows lane % 8 (gate) and + 8 (up)
+            const int w0 = (4 * warp + (lane >> 3)) * WARPS, r = lane & 7;
             float gate = 0.0f, up = 0.0f;
 #pragma unroll
             for (int w = 0; w < WARPS; ++w) {
@@ -338,12 +342,12 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
             }
             gate *= s_in;
             up *= s_in;
-            const int64_t ch = (int64_t)blockIdx.x * 32 + lane;
+            const int64_t ch = blk * 32 + lane;
             const float act = 2 * ch < v.n ? (gate * (1.0f / (1.0f + expf(-gate)))) * up : 0.0f;
             if (y && 2 * ch < v.n) {
                 y[ch] = act;
             }
-            warp_pack_block32(act, fu.packed_out + (size_t)(blockIdx.x >> 3) * XPK1_REC, blockIdx.x & 7);
+            warp_pack_block32(act, fu.packed_out + (size_t)(blk >> 3) * XPK1_REC, (int)(blk & 7));
         }
     } else {
         if (threadIdx.x < 8) {
@@ -364,6 +368,25 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
     }
 }
 
+// SMs of a device, 0 if it cannot be asked; asked once.
+inline int sm_count_of(int dev)
+{
+    static std::atomic<int> known[64];
+    if (dev >= 0 && dev < 64) {
+        if (const int n = known[dev].load(std::memory_order_relaxed)) {
+            return n;
+        }
+    }
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        return 0;
+    }
+    if (dev >= 0 && dev < 64) {
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // Ring depth per format: 28-37 KB of tiles in flight per CTA.
 template <int FMT>
 struct Tune {
@@ -371,27 +394,25 @@ struct Tune {
     static constexpr int DEPTH = FMT == FMT_Q8_0 ? 2 : 3;
 };
 
-template <int FMT, int WARPS, int DEPTH, int EPI, bool XF32>
+template <int FMT, int WARPS, int DEPTH, int EPI, bool XF32, int TILES = epi_tiles(EPI)>
 cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y, int* status,
                              const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
 {
-    constexpr int TILES = epi_tiles(EPI);
     using Plan = SmemPlan<FMT, WARPS, DEPTH, TILES>;
     auto kernel = gemv_kernel<FMT, WARPS, DEPTH, EPI, TILES, XF32>;
     int smem = Plan::total(w.kc);
     if (smem > 227 * 1024) {
         return cudaErrorInvalidConfiguration;
     }
-    if (w.rt % TILES != 0) {
+    if (w.rt % epi_tiles(EPI) != 0) {
         return cudaErrorInvalidValue;
     }
-    const int grid = w.rt / TILES;
+    const int grid = (w.rt + TILES - 1) / TILES;
     // Residency cap.  The block scheduler fills an SM up to its limit before it is even with the others, so
     // a grid of 688 CTAs that could sit 7 to an SM leaves a third of the SMs with little to do (measured on
     // B200: 6.7 us at a limit of 7, 5.2 us at 5 for W[11008,4096]).  The dynamic shared memory request is
     // padded so that no SM can hold more than its even share, ceil(grid / SMs), of the CTAs.
     static std::mutex mu;
-    static int sm_count[64] = {};
     static int configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -400,13 +421,8 @@ cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y,
     }
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (dev >= 0 && dev < 64 && sm_count[dev] == 0) {
-            cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
-        }
-        int share = dev >= 0 && dev < 64 && sm_count[dev] > 0 ? (grid + sm_count[dev] - 1) / sm_count[dev] : 0;
-        if (const char* env = getenv("QMM_GEMV_CTAS_PER_SM")) {  // tuning aid
-            share = atoi(env);
-        }
+        const int sms = sm_count_of(dev);
+        const int share = sms > 0 ? (grid + sms - 1) / sms : 0;
         if (share >= 1 && share <= 16) {
             const int want = 232448 / share - 1024 - 256;
             smem = want > smem ? want : smem;
@@ -439,7 +455,7 @@ template <int FMT, int WARPS, int DEPTH, int EPI>
 cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float* y, int* status,
                                 const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
 {
-    if constexpr (EPI != EPI_SWIGLU && EPI != EPI_SWIGLU_PACK) {
+    if constexpr (EPI == EPI_RESID_PACK) {
         if (fu.x_f32 != nullptr) {
             return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, true>(w, xp, y, status, ps, fu, stream);
         }
@@ -448,6 +464,124 @@ cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float*
         return cudaErrorInvalidValue;
     }
     return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, false>(w, xp, y, status, ps, fu, stream);
+}
+
+// The one-wave form: a CTA on every SM, each with as many row tiles as that takes (ceil(tiles / SMs), up to the next
+// compiled count), WARPS warps and WARPS x DEPTH slots per tile.  What bounds a matvec of many small CTAs is the last
+// of its waves and, for an fp32 vector, that every CTA packs the vector again; here there is one wave and at most 148
+// copies.  Measured on B200, a stream of different weights, us each, many CTAs -> one wave:
+//   packed vector  Q4_0 8192 x 28672 28.9 -> 22.4, 10240 x 8192 12.4 -> 9.4, 28672 x 8192 27.4 -> 22.7, 4096 x 4096 3.8 -> 3.5;
+//                  Q4_K 28672 x 8192 29.9 -> 22.6, 11008 x 4096 7.4 -> 6.7; Q6_K 28672 x 8192 35.4 -> 31.5, 14336 x 4096
+//                  11.1 -> 9.7; Q8_0 11008 x 4096 11.0 -> 9.5
+//   fp32 vector    (before: a kernel that packs it, then the matvec) Q4_0 1024 x 4096 4.2 -> 3.0, 14336 x 4096 9.5 -> 8.1,
+//                  28672 x 8192 28.2 -> 23.9; Q4_K 14336 x 4096 10.6 -> 9.0; Q6_K 4096 x 2048 4.2 -> 3.4; Q8_0 4096 x 4096 6.0 -> 5.4
+// More warps per tile shorten a short row's chain of tiles; more than about 90 KB of slots gains nothing, so the warps per
+// tile fall as the tiles grow.  The shared-memory request keeps a second CTA of the same kernel off an SM: without
+// it, 4096 x 8192 of Q4_K takes 7.2 us and not 5.6.  LESS: warps and depth to fall back to where long rows leave less room
+// for slots; with at most GEMV_WAVE_KC chunks the last entry always fits.
+constexpr int GEMV_WAVE_KC = 112;
+
+template <int FMT, int EPI, bool XF32>
+struct GemvWave {
+    const WeightView& w;
+    const XPackView& xp;
+    float* y;
+    int* status;
+    const PeerScatter& ps;
+    const GemvFuse& fu;
+    cudaStream_t stream;
+
+    template <int TILES, int WARPS, int DEPTH, int... LESS>
+    cudaError_t go() const
+    {
+        if constexpr (TILES % epi_tiles(EPI) != 0) {
+            return cudaErrorInvalidConfiguration;  // not reached: the caller rounds up to whole groups
+        } else if constexpr (sizeof...(LESS) > 0) {
+            if (SmemPlan<FMT, WARPS, DEPTH, TILES>::total(w.kc) > 227 * 1024) {
+                return go<TILES, LESS...>();
+            }
+            return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, XF32, TILES>(w, xp, y, status, ps, fu, stream);
+        } else {
+            return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, XF32, TILES>(w, xp, y, status, ps, fu, stream);
+        }
+    }
+
+    cudaError_t launch(int sms) const
+    {
+        constexpr int GROUP = epi_tiles(EPI);
+        constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
+        const int share = (w.rt + sms - 1) / sms;
+        const int tiles = (share + GROUP - 1) / GROUP * GROUP;
+        const bool small = w.kc <= 8;  // two tiles per warp at most, whatever the form: fewer warps to add up
+        if (tiles <= 1) {
+            return w.kc <= 4 ? go<1, 8, 1>() : go<1, 16, 2>();
+        }
+        if (tiles == 2) {
+            return go<2, 8, 2>();
+        }
+        if (tiles == 3) {
+            return small && w.kc > 4 ? go<3, 8, 1>() : go<3, 5, 2>();
+        }
+        if (tiles == 4) {
+            return go<4, 4, 3, 4, 2>();
+        }
+        if (tiles == 5) {
+            return go<5, 4, 2, 4, 1>();
+        }
+        if (tiles == 6) {
+            return small ? go<6, 2, 2>() : go<6, 4, 2, 2, 2>();
+        }
+        if (tiles == 7) {
+            if constexpr (NIBBLE) {
+                return small ? go<7, 2, 2>() : go<7, 4, 2>();
+            } else {
+                return small ? go<7, 2, 2>() : go<7, 2, 3, 2, 2>();
+            }
+        }
+        if (tiles == 8) {
+            return small ? go<8, 2, 2>() : go<8, 2, 3, 2, 2>();
+        }
+        if (tiles <= 10) {
+            return go<10, 2, 2, 2, 1>();
+        }
+        if (tiles <= 12) {
+            return go<12, 2, 2, 2, 1>();
+        }
+        if constexpr (NIBBLE) {
+            return tiles <= 14   ? go<14, 2, 2>()
+                   : tiles <= 16 ? go<16, 2, 2>()
+                   : tiles <= 20 ? go<20, 1, 2>()
+                   : tiles <= 25 ? go<25, 1, 2>()
+                   : tiles <= 28 ? go<28, 1, 2>()
+                                 : cudaErrorInvalidConfiguration;
+        } else {
+            // 1-byte and 6-bit tiles leave room for two warps per row tile only with one slot each: one warp with three is 4 % faster
+            return tiles <= 14   ? go<14, 1, 3, 1, 2>()
+                   : tiles <= 16 ? go<16, 1, 3, 1, 2>()
+                                 : cudaErrorInvalidConfiguration;
+        }
+    }
+};
+
+// Where the one-wave form takes a packed vector: not while the small CTAs of the forms below are all resident at once and
+// even (up to six per SM for 8 <= kc <= 16, which the larger tiles of Q8_0 and Q4_K's arithmetic stop earlier, three
+// above), except for two tiles per SM, where the small CTAs are either one or two to an SM (4096 x 4096: 7 % for every format).
+// Inside a chain (ss_in) small CTAs also start while the kernel before drains, which a CTA that fills its SM cannot: the
+// line lies at nine tiles (the vocabulary: 70B-shape token 562.3 -> 558.1 us; with the QKV matvec in it 564.5).
+template <int FMT>
+bool gemv_one_wave(const WeightView& w, bool chained, int sms)
+{
+    const int tiles = (w.rt + sms - 1) / sms;
+    if (w.kc > GEMV_WAVE_KC || tiles > (tile_bytes(FMT) == 2304 ? 28 : 16)) {
+        return false;
+    }
+    if (chained) {
+        return tiles >= 9;
+    }
+    if (w.kc > 16) {
+        return tiles >= (FMT == FMT_Q8_0 ? 4 : 3);
+    }
+    return tiles == 2 || tiles >= (FMT == FMT_Q4_0 ? 7 : FMT == FMT_Q6_K ? 6 : FMT == FMT_Q8_0 ? 5 : 4);
 }
 
 // Batch 1: warps x ring slots by row length.
@@ -468,17 +602,29 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
 {
     constexpr int TILES = epi_tiles(EPI);
     constexpr int LIMIT = 113 * 1024;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    const int sms = sm_count_of(dev);
+    if (sms < 1) {
+        return cudaErrorInvalidDevice;
+    }
+    if constexpr (EPI == EPI_STORE) {
+        if (fu.x_f32 != nullptr) {  // gemv_packs_itself says which
+            return GemvWave<FMT, EPI, true>{w, xp, y, status, ps, fu, stream}.launch(sms);
+        }
+        if (gemv_one_wave<FMT>(w, fu.ss_in != nullptr, sms)) {
+            return GemvWave<FMT, EPI, false>{w, xp, y, status, ps, fu, stream}.launch(sms);
+        }
+    }
     if constexpr (TILES == 2) {
         // The residual form has two row tiles per CTA and n / 32 CTAs: 128 for a 4096-wide model, 256 for an
         // 8192-wide one.  All of them should be resident at once (a second wave of a few CTAs doubles the
         // kernel's time), so the variant is the deepest one whose shared memory lets ceil(CTAs / SMs) CTAs
         // share an SM.  8 warps per tile with three slots each walk a long row with 110 KB in flight per CTA
         // (ffn_down of the 7B shape, K = 11008: 7.1 us against 8.1 us with 16 warps x 2 slots).
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
-            return cudaErrorInvalidDevice;
-        }
         const int ctas = w.rt / 2;
         const int per_sm = (ctas + sms - 1) / sms;
         const int budget = 232448 / per_sm - 1280;

@@ -24,6 +24,8 @@ cudaError_t launch_gemv(const WeightView& w, const XPackView& xp, float* y, int 
 // `fu` asks for an input RMSNorm factor or a fused epilogue (GemvFuse); both in qmm_common.cuh.
 cudaError_t launch_gemv_fused(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                               const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream);
+// Whether the matvec of one fp32 vector is one launch that packs x itself (launch_gemv_fused with fu.x_f32 and EPI_STORE).
+bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count);
 // per-format instantiations (qmm_gemv_<format>.cu)
 cudaError_t launch_gemv_q4_0(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                              const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream);
