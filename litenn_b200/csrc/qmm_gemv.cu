@@ -164,7 +164,7 @@ bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count)
     }
     const int tiles = (w.rt + sm_count - 1) / sm_count;
     if (w.kc > 32) {
-        return w.fmt == FMT_Q8_0 && tiles == 1 && w.kc <= 112;
+        return w.fmt == FMT_Q8_0 && tiles == 1 && w.kc <= GEMV_WAVE_KC;
     }
     if (w.fmt == FMT_Q8_0) {
         return tiles <= (w.kc > 16 ? 2 : 16);

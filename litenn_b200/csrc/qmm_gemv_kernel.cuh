@@ -479,8 +479,6 @@ cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float*
 // tile fall as the tiles grow.  The shared-memory request keeps a second CTA of the same kernel off an SM: without
 // it, 4096 x 8192 of Q4_K takes 7.2 us and not 5.6.  LESS: warps and depth to fall back to where long rows leave less room
 // for slots; with at most GEMV_WAVE_KC chunks the last entry always fits.
-constexpr int GEMV_WAVE_KC = 112;
-
 template <int FMT, int EPI, bool XF32>
 struct GemvWave {
     const WeightView& w;
@@ -490,6 +488,7 @@ struct GemvWave {
     const PeerScatter& ps;
     const GemvFuse& fu;
     cudaStream_t stream;
+    static constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
 
     template <int TILES, int WARPS, int DEPTH, int... LESS>
     cudaError_t go() const
@@ -508,19 +507,30 @@ struct GemvWave {
 
     cudaError_t launch(int sms) const
     {
-        constexpr int GROUP = epi_tiles(EPI);
-        constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
-        const int share = (w.rt + sms - 1) / sms;
-        const int tiles = (share + GROUP - 1) / GROUP * GROUP;
+        const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms);
+        if constexpr (EPI == EPI_SWIGLU_PACK) {
+            if (tiles > 12) {
+                return launch_many(tiles);
+            }
+            return go<12, 2, 2, 2, 1>();  // nine tiles at least
+        } else {
+            return launch_few(tiles);
+        }
+    }
+
+    cudaError_t launch_few(int tiles) const
+    {
         const bool small = w.kc <= 8;  // two tiles per warp at most, whatever the form: fewer warps to add up
-        if (tiles <= 1) {
-            return w.kc <= 4 ? go<1, 8, 1>() : go<1, 16, 2>();
-        }
-        if (tiles == 2) {
-            return go<2, 8, 2>();
-        }
-        if (tiles == 3) {
-            return small && w.kc > 4 ? go<3, 8, 1>() : go<3, 5, 2>();
+        if constexpr (EPI == EPI_STORE) {
+            if (tiles <= 1) {
+                return w.kc <= 4 ? go<1, 8, 1>() : go<1, 16, 2>();
+            }
+            if (tiles == 2) {
+                return go<2, 8, 2>();
+            }
+            if (tiles == 3) {
+                return small && w.kc > 4 ? go<3, 8, 1>() : go<3, 5, 2>();
+            }
         }
         if (tiles == 4) {
             return go<4, 4, 3, 4, 2>();
@@ -547,19 +557,34 @@ struct GemvWave {
         if (tiles <= 12) {
             return go<12, 2, 2, 2, 1>();
         }
-        if constexpr (NIBBLE) {
-            return tiles <= 14   ? go<14, 2, 2>()
-                   : tiles <= 16 ? go<16, 2, 2>()
-                   : tiles <= 20 ? go<20, 1, 2>()
+        return launch_many(tiles);
+    }
+
+    cudaError_t launch_many(int tiles) const
+    {
+        // Q6_K and Q8_0 leave room for two warps per row tile only with one slot each: one warp with three is 4 % faster.
+        // So it is inside a chain for every format, as 32 warps of 64 registers leave the next kernel none (28672 x 7168
+        // and three blocks, Q4_0: 227 us a token with two warps, 200 with one).
+        if (tiles <= 16) {
+            if constexpr (NIBBLE && EPI == EPI_STORE) {
+                return tiles <= 14 ? go<14, 2, 2>() : go<16, 2, 2>();
+            } else {
+                return tiles <= 14 ? go<14, 1, 3, 1, 2>() : go<16, 1, 3, 1, 2>();
+            }
+        }
+        if constexpr (EPI == EPI_SWIGLU_PACK) {
+            return tiles <= 20   ? go<20, 1, 2, 1, 1>()
+                   : tiles <= 24 ? go<24, 1, 2, 1, 1>()
+                   : tiles <= 28 ? go<28, 1, 2, 1, 1>()
+                                 : cudaErrorInvalidConfiguration;
+        }
+        if constexpr (EPI == EPI_STORE && NIBBLE) {
+            return tiles <= 20   ? go<20, 1, 2>()
                    : tiles <= 25 ? go<25, 1, 2>()
                    : tiles <= 28 ? go<28, 1, 2>()
                                  : cudaErrorInvalidConfiguration;
-        } else {
-            // 1-byte and 6-bit tiles leave room for two warps per row tile only with one slot each: one warp with three is 4 % faster
-            return tiles <= 14   ? go<14, 1, 3, 1, 2>()
-                   : tiles <= 16 ? go<16, 1, 3, 1, 2>()
-                                 : cudaErrorInvalidConfiguration;
         }
+        return cudaErrorInvalidConfiguration;
     }
 };
 
@@ -568,12 +593,23 @@ struct GemvWave {
 // above), except for two tiles per SM, where the small CTAs are either one or two to an SM (4096 x 4096: 7 % for every format).
 // Inside a chain (ss_in) small CTAs also start while the kernel before drains, which a CTA that fills its SM cannot: the
 // line lies at nine tiles (the vocabulary: 70B-shape token 562.3 -> 558.1 us; with the QKV matvec in it 564.5).
-template <int FMT>
+// The residual form takes it from three tiles on, the packed gate|up form from nine on, as its groups of four tiles sit
+// three to an SM otherwise.  Tokens with three blocks, us: gate|up of 14336 x 4096 Q4_0 145.6 -> 135.8 and Q4_K 146.1 -> 140.5
+// (448 groups, 444 places), 11008 x 4096 Q8_0 226 -> 211 (four blocks); 6912 x 2560 and 8192 x 3072, below nine, move by
+// 1 % either way.  Residual of the 70B shape (8192 rows, four blocks): 550 -> 528.  A grid that the rounding to whole
+// groups leaves on fewer than four fifths of the SMs gains nothing there (5120 rows 205 -> 209, 7168 rows 215 -> 216).
+template <int FMT, int EPI>
 bool gemv_one_wave(const WeightView& w, bool chained, int sms)
 {
-    const int tiles = (w.rt + sms - 1) / sms;
-    if (w.kc > GEMV_WAVE_KC || tiles > (tile_bytes(FMT) == 2304 ? 28 : 16)) {
+    const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms);
+    if (w.kc > GEMV_WAVE_KC || tiles > (EPI == EPI_SWIGLU_PACK || (EPI == EPI_STORE && tile_bytes(FMT) == 2304) ? 28 : 16)) {
         return false;
+    }
+    if constexpr (EPI == EPI_SWIGLU_PACK) {
+        return w.rt > 8 * sms;
+    }
+    if constexpr (EPI == EPI_RESID_PACK) {
+        return w.rt > 2 * sms && gemv_wave_fills(w.rt, epi_tiles(EPI), sms);
     }
     if (chained) {
         return tiles >= 9;
@@ -615,9 +651,19 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         if (fu.x_f32 != nullptr) {  // gemv_packs_itself says which
             return GemvWave<FMT, EPI, true>{w, xp, y, status, ps, fu, stream}.launch(sms);
         }
-        if (gemv_one_wave<FMT>(w, fu.ss_in != nullptr, sms)) {
+    }
+    if constexpr (EPI != EPI_SWIGLU) {
+        // (a tensor-parallel rank keeps the residual form that waits for its peers in small CTAs)
+        if (fu.x_f32 == nullptr && !(EPI == EPI_RESID_PACK && ps.n_peers > 0) &&
+            gemv_one_wave<FMT, EPI>(w, fu.ss_in != nullptr, sms)) {
             return GemvWave<FMT, EPI, false>{w, xp, y, status, ps, fu, stream}.launch(sms);
         }
+    }
+    if constexpr (EPI == EPI_SWIGLU_PACK) {
+        // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
+        // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
+        // 7B-shape step slower)
+        return launch_gemv_variant<FMT, 2, 2, EPI>(w, xp, y, status, ps, fu, stream);
     }
     if constexpr (TILES == 2) {
         // The residual form has two row tiles per CTA and n / 32 CTAs: 128 for a 4096-wide model, 256 for an
@@ -673,10 +719,7 @@ cudaError_t launch_gemv_fmt(const WeightView& w, const XPackView& xp, float* y, 
         case EPI_STORE: return launch_gemv_m1<FMT, EPI_STORE>(w, xp, y, status, ps, fu, stream);
         case EPI_RESID_PACK: return launch_gemv_m1<FMT, EPI_RESID_PACK>(w, xp, y, status, ps, fu, stream);
         case EPI_SWIGLU: return launch_gemv_m1<FMT, EPI_SWIGLU>(w, xp, y, status, ps, fu, stream);
-        // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
-        // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
-        // 7B-shape step slower)
-        case EPI_SWIGLU_PACK: return launch_gemv_variant<FMT, 2, 2, EPI_SWIGLU_PACK>(w, xp, y, status, ps, fu, stream);
+        case EPI_SWIGLU_PACK: return launch_gemv_m1<FMT, EPI_SWIGLU_PACK>(w, xp, y, status, ps, fu, stream);
         default: return cudaErrorInvalidValue;
         }
     }

@@ -24,6 +24,18 @@ cudaError_t launch_gemv(const WeightView& w, const XPackView& xp, float* y, int 
 // `fu` asks for an input RMSNorm factor or a fused epilogue (GemvFuse); both in qmm_common.cuh.
 cudaError_t launch_gemv_fused(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                               const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream);
+// The one-wave matvec: row tiles per CTA, in whole groups of a fused form (epi_tiles), that put every tile on the chip at
+// once, and whether such CTAs sit on at least four fifths of the SMs.  Rows of more than GEMV_WAVE_KC chunks do not leave it
+// the shared memory.
+constexpr int GEMV_WAVE_KC = 112;
+constexpr int gemv_wave_tiles(int rt, int group, int sms)
+{
+    return ((rt + sms - 1) / sms + group - 1) / group * group;
+}
+constexpr bool gemv_wave_fills(int rt, int group, int sms)
+{
+    return 5LL * rt >= 4LL * sms * gemv_wave_tiles(rt, group, sms);
+}
 // Whether the matvec of one fp32 vector is one launch that packs x itself (launch_gemv_fused with fu.x_f32 and EPI_STORE).
 bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count);
 // per-format instantiations (qmm_gemv_<format>.cu)
