@@ -142,9 +142,11 @@ int qmm_dequantize_raw(int device, int fmt, const void* payload_dev, int64_t n, 
  * DequantizeNode{Block,[n,k],Float32} -> Transpose -> MatMul(x, ·)
  * (src/LiteNN/Graph.h:66-70,115-120; Layer/Linear.h:64-90) and stands where
  * DeviceTraits<CUDA>::DoBinaryOp(MatMul) (src/LiteNN/Device/CUDA.cpp:1914-1940)
- * is called today.  A packing kernel quantizes the activations first; its scratch memory
+ * is called today.  The activations are quantized first: by a packing kernel, whose scratch memory
  * (the packed activations) comes from a per-(device,stream) workspace the library allocates
- * on first use.
+ * on first use, or for many shapes of one 16-byte aligned row by the product's own kernel.
+ * y may lie over x, wholly or in part: such a call always takes the packing kernel, which has read
+ * all of x before the product stores.
  */
 int qmm_gemv_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int m, void* stream);
 

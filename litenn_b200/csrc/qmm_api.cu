@@ -623,7 +623,7 @@ int qmm_gemv_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int m, v
         return fail(QMM_E_INVALID, "qmm_gemv_f32: batch %d outside 1..%d (use qmm_gemm_bf16 for prefill)", m,
                     QMM_GEMV_MAX_BATCH);
     }
-    if (m == 1 && gemv_packs_itself(view_of(w), x_dev, w->sm_count)) {
+    if (m == 1 && gemv_packs_itself(view_of(w), x_dev, y_dev, w->sm_count)) {
         GemvFuse fu = {};
         fu.x_f32 = x_dev;
         return gemv_packed_impl("qmm_gemv_f32", w, nullptr, y_dev, 1, nullptr, &fu, stream_v);

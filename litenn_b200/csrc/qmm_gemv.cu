@@ -157,8 +157,14 @@ cudaError_t launch_unpack_x(const uint8_t* packed, int64_t k, float* x, cudaStre
 // being also the better matvec; above, packing 11008 values takes 256 rows of Q4_0 5.5 us and not 4.4, and only Q8_0
 // on one row tile per SM gains (7.5 -> 5.9).  Q8_0 beyond 16 chunks is bound by its bytes either way (28672 x 8192: 39.7
 // us, 40.5 in one launch).  Of many tiles per SM only the 4-bit formats have room for enough slots.
-bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count)
+// Never where y lies over x: CTAs that are done store y while others still read x.  The packing kernel reads all of x first.
+bool gemv_packs_itself(const WeightView& w, const float* x, const float* y, int sm_count)
 {
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), x1 = x0 + (uintptr_t)w.k * sizeof(float);
+    const uintptr_t y0 = reinterpret_cast<uintptr_t>(y), y1 = y0 + (uintptr_t)w.n * sizeof(float);
+    if (x0 < y1 && y0 < x1) {
+        return false;
+    }
     if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || w.k % 32 != 0 || sm_count < 1) {  // x is read 16 bytes at a time
         return false;
     }

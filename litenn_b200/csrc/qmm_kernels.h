@@ -37,7 +37,7 @@ constexpr bool gemv_wave_fills(int rt, int group, int sms)
     return 5LL * rt >= 4LL * sms * gemv_wave_tiles(rt, group, sms);
 }
 // Whether the matvec of one fp32 vector is one launch that packs x itself (launch_gemv_fused with fu.x_f32 and EPI_STORE).
-bool gemv_packs_itself(const WeightView& w, const float* x, int sm_count);
+bool gemv_packs_itself(const WeightView& w, const float* x, const float* y, int sm_count);
 // per-format instantiations (qmm_gemv_<format>.cu)
 cudaError_t launch_gemv_q4_0(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                              const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream);
