@@ -59,12 +59,13 @@ __device__ __forceinline__ double block_sum_double(double v, double* red)
 
 // ---- decode (one token) -------------------------------------------------------------------------
 
-// h[d] = dequantized row `token` of the raw (not repacked) embedding payload.
+// h[d] = dequantized row `token` of the raw (not repacked) embedding payload.  First kernel of a prompt and of a batched step:
+// like embed_pack_kernel it waits before it lets its dependents launch.
 __global__ void embed_row_kernel(int fmt, const uint8_t* __restrict__ raw, const int* __restrict__ tokens, int n_rows,
                                  int d, float* __restrict__ h)
 {
-    pdl_trigger();
     pdl_sync();
+    pdl_trigger();
     const int elems = block_elems(fmt), bytes = block_bytes(fmt);
     const int64_t row_bytes = (int64_t)(d / elems) * bytes;
     for (int r = blockIdx.y; r < n_rows; r += gridDim.y) {
@@ -305,7 +306,8 @@ __global__ void __launch_bounds__(256) attn_fused_kernel(const float* __restrict
     __shared__ float vals[256];
     pdl_trigger();
     // Everything up to pdl_sync() reads only what earlier tokens left behind (the position, the
-    // rotation tables, the cached keys and values), so it runs while the qkv GEMV is finishing.
+    // rotation tables, the cached keys and values), so it runs while the qkv GEMV is finishing.  All of that is in place
+    // because the first kernel of a step waits for the step before and only then releases what follows it.
     const int rank = (int)cluster.block_rank();
     const int chunk = blockIdx.x / ATTN_CLUSTER;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
