@@ -160,7 +160,8 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
 
     if (warp == DW) {
         // ---- TMA producer: tokens.  Only they come from an earlier kernel; the first weights are dequantized while it drains,
-        // and what is stored in the end depends on the tokens ----
+        // and what is stored in the end depends on the tokens.  Every warp waits for that kernel before its first bounded wait,
+        // whose limit is for this kernel's own steps ----
         if (lane == 0) {
             g_pdl_wait();
             int slot = 0;
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         int slot = 0;
         uint32_t phase = 0;
         bool ok = true;
+        g_pdl_wait();
         for (int s = 0; s < n_steps; ++s) {
             const int as = s % GEMM_A_STAGES;
             ok = g_mbar_wait(&full_b[slot], phase) && g_mbar_wait(&full_a[as], (uint32_t)(s / GEMM_A_STAGES) & 1u);
@@ -265,6 +267,9 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
                         load_quarter<FMT>(P, next, q, lane);
                     }
                     const int as = s % GEMM_A_STAGES;
+                    if (s == GEMM_A_STAGES) {
+                        g_pdl_wait();
+                    }
                     if (s >= GEMM_A_STAGES && !g_mbar_wait_warp(&empty_a[as], (uint32_t)(s / GEMM_A_STAGES - 1) & 1u)) {
                         if (lane == 0) {
                             atomicExch(args.status, 13);
@@ -290,6 +295,7 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         }
 
         // ---- epilogue: D has one weight row per lane, one token per column ----
+        g_pdl_wait();
         if (!g_mbar_wait_warp(accum, 0)) {
             if (lane == 0) {
                 atomicExch(args.status, 14);

@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 
     if (warp == 0) {
         // ---- TMA producer: activations.  Only they come from an earlier kernel; the first weights are dequantized while it
-        // drains, and what is stored in the end depends on the activations ----
+        // drains, and what is stored in the end depends on the activations.  Every warp waits for that kernel before its first
+        // bounded wait, whose limit is for this kernel's own steps ----
         if (lane == 0) {
             g_pdl_wait();
             for (int s = 0; s < n_stages; ++s) {
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         // ---- MMA issuer: the whole warp walks the stages, one lane issues ----
         const uint32_t idesc = umma_idesc_bf16(n);
         bool ok = true;
+        g_pdl_wait();
         for (int s = 0; s < n_stages; ++s) {
             const int slot = s % GEMM_STAGES;
             const uint32_t parity = (uint32_t)(s / GEMM_STAGES) & 1u;
@@ -276,6 +278,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     uint32_t r[16];
                     dequant_quarter<FMT>(P, S, q, r);
                     const int slot = s % GEMM_STAGES;
+                    if (s == GEMM_STAGES) {
+                        g_pdl_wait();
+                    }
                     if (ok && s >= GEMM_STAGES) {
                         // lane 0 probes, the others wait for it at the warp barrier
                         bool landed = true;
@@ -308,6 +313,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
 
         // ---- epilogue: a warp reaches TMEM lanes 32*(warp%4).., four warps share them by columns ----
+        g_pdl_wait();
         if (!g_mbar_wait_warp(accum, 0)) {
             if (lane == 0) {
                 atomicExch(args.status, 14);

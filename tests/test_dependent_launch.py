@@ -26,3 +26,17 @@ def test_the_first_kernel_of_a_step_waits_before_it_releases_the_next(name):
     body = kernel_body("llama_kernels.cu", name)
     assert body.index("pdl_sync()") < body.index("pdl_trigger()")
     assert body.count("pdl_trigger()") == 1
+
+
+@pytest.mark.parametrize("file,name", [("qmm_gemm.cu", "gemm_ts_kernel"), ("qmm_gemm_smem.cu", "gemm_tcgen05_kernel")])
+def test_every_warp_of_a_gemm_waits_for_the_kernel_before_ahead_of_a_bounded_wait(file, name):
+    """A limit that ran while an earlier kernel still works would fail a healthy product."""
+    body = kernel_body(file, name)
+    roles = re.split(r"\bif \(warp == |\} else if \(warp == |\} else \{\n(?=\s+const int (?:quad|dw) )", body)
+    waiting = [r for r in roles if re.search(r"g_mbar_(?:wait|poll)", r)]
+    assert len(waiting) >= 3  # tokens, tensor core, weights
+    for role in waiting:
+        # the wait ahead of a stage's first reuse stands inside that loop, and one before the epilogue serves short products
+        assert role.index("g_pdl_wait()") < re.search(r"g_mbar_(?:wait|poll)", role).start(), role[:200]
+    weights = waiting[2]
+    assert weights.rindex("g_pdl_wait()") < weights.index("g_mbar_wait_warp(accum")
