@@ -144,7 +144,8 @@ int qmm_dequantize_raw(int device, int fmt, const void* payload_dev, int64_t n, 
  * DeviceTraits<CUDA>::DoBinaryOp(MatMul) (src/LiteNN/Device/CUDA.cpp:1914-1940)
  * is called today.  The activations are quantized first: by a packing kernel, whose scratch memory
  * (the packed activations) comes from a per-(device,stream) workspace the library allocates
- * on first use, or for many shapes of one 16-byte aligned row by the product's own kernel.
+ * on first use, or for many shapes of one 16-byte aligned row by the product's own kernel (a call outside a
+ * stream capture makes the workspace all the same, so that it is there for a captured call that needs it).
  * y may lie over x, wholly or in part: such a call always takes the packing kernel, which has read
  * all of x before the product stores.
  */

@@ -116,12 +116,8 @@ int get_status_word(int device, int** out)
     return QMM_OK;
 }
 
-// Two activation buffers of `one` bytes per (device, stream), handed out alternately.
-int get_workspace_half(int device, void* stream, size_t one, uint8_t** out)
+int grow_workspace(Workspace& ws, void* stream, size_t bytes)
 {
-    std::lock_guard<std::mutex> lock(g_ws_mutex);
-    Workspace& ws = g_workspaces[std::make_pair(device, stream)];
-    const size_t bytes = 2 * one;
     if (ws.bytes < bytes) {
         if (ws.base) {
             // the old buffer may still be read by work queued on the stream
@@ -134,9 +130,43 @@ int get_workspace_half(int device, void* stream, size_t one, uint8_t** out)
         QMM_CUDA(cudaMalloc(&ws.base, want));
         ws.bytes = want;
     }
+    return QMM_OK;
+}
+
+// Two activation buffers of `one` bytes per (device, stream), handed out alternately.
+int get_workspace_half(int device, void* stream, size_t one, uint8_t** out)
+{
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    Workspace& ws = g_workspaces[std::make_pair(device, stream)];
+    if (int rc = grow_workspace(ws, stream, 2 * one)) {
+        return rc;
+    }
     *out = ws.base + (ws.flip ? ws.bytes / 2 : 0);
     ws.flip ^= 1;
     return QMM_OK;
+}
+
+// The same buffers for a call that does without them: a later call of the same size on the stream may need them while it is
+// captured, when nothing can be allocated.  A captured call leaves them as they are, and nothing fails here.
+void reserve_workspace(int device, void* stream, size_t one)
+{
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    Workspace& ws = g_workspaces[std::make_pair(device, stream)];
+    if (ws.bytes >= 2 * one) {
+        return;
+    }
+    DeviceGuard guard(device);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+    if (guard.ok && cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone) {
+        // another stream may be in a capture, which an allocation would end unless it is declared harmless
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess) {
+            grow_workspace(ws, stream, 2 * one);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+        }
+    }
+    cudaGetLastError();
 }
 
 int create_impl(int device, int fmt, const void* payload, size_t payload_bytes, int payload_on_device, int64_t n,
@@ -623,15 +653,16 @@ int qmm_gemv_f32(const qmm_weight* w, const float* x_dev, float* y_dev, int m, v
         return fail(QMM_E_INVALID, "qmm_gemv_f32: batch %d outside 1..%d (use qmm_gemm_bf16 for prefill)", m,
                     QMM_GEMV_MAX_BATCH);
     }
-    if (m == 1 && gemv_packs_itself(view_of(w), x_dev, y_dev, w->sm_count)) {
-        GemvFuse fu = {};
-        fu.x_f32 = x_dev;
-        return gemv_packed_impl("qmm_gemv_f32", w, nullptr, y_dev, 1, nullptr, &fu, stream_v);
-    }
     // Two activation buffers per (device, stream), used alternately.
     size_t one = 0;
     if (int rc = qmm_packed_activation_bytes(w->k, m, &one)) {
         return rc;
+    }
+    if (m == 1 && gemv_packs_itself(view_of(w), x_dev, y_dev, w->sm_count)) {
+        reserve_workspace(w->device, stream_v, one);
+        GemvFuse fu = {};
+        fu.x_f32 = x_dev;
+        return gemv_packed_impl("qmm_gemv_f32", w, nullptr, y_dev, 1, nullptr, &fu, stream_v);
     }
     uint8_t* buf = nullptr;
     {
