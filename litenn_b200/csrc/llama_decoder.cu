@@ -9,9 +9,10 @@
 //                       previous kernel; multiplies its row sums by 1/rms
 //   attention           RoPE, KV append, attention over the cache, packs the context
 //   attn_output matvec  epilogue: h += result; packs (h * ffn_norm), sums of squares
-//   gate|up matvec      rows interleaved gate/up; epilogue: silu(gate) * up, packed for ffn_down.  An fp32 product that
-//                       ffn_down (or a kernel of its own) packs was slower for every width: 5120 wide with an FFN of
-//                       13824 185 -> 168 us a token of three blocks, 70B shape (four blocks) 528 -> 459
+//   gate|up matvec      rows interleaved gate/up; epilogue: silu(gate) * up, packed for ffn_down (fp32 where a wide model
+//                       has few channels, which ffn_down packs itself: gemv_swiglu_packs in qmm_kernels.h.  Elsewhere
+//                       an fp32 product was slower: 5120 wide with an FFN of 13824 185 us a token of three blocks,
+//                       packed 168; 70B shape, four blocks, 528 and 459)
 //   ffn_down matvec     epilogue: h += result; packs (h * next norm), sums of squares
 // (RMSNorm(h) * w = (h * w) / rms(h): packing needs no statistic of the whole row, and the scalar
 // 1/rms commutes with the matvec.)  With tensor parallelism the two K-split matvecs also exchange their
@@ -105,7 +106,10 @@ struct qmm_llama {
     // decode buffers
     float *h = nullptr, *y = nullptr, *qkv = nullptr, *logits = nullptr;
     uint8_t *pk_d = nullptr, *pk_ctx = nullptr;
-    uint8_t* pk_act = nullptr;  // [ffn of this rank] silu(gate) * up as packed activations
+    float* act_f = nullptr;     // [ffn of this rank] silu(gate) * up, fp32; the ffn_down matvec packs it itself
+    uint8_t* pk_act = nullptr;  // the same as packed activations, written by the gate|up matvec (glu_packed)
+    bool glu_packed = false;    // gemv_swiglu_packs
+    int sm_count = 0;
     double* ss_d = nullptr;  // [d_model / 32] sums of squares of the residual stream
     float *rope_cos = nullptr, *rope_sin = nullptr;
     int *pos = nullptr, *token = nullptr, *out_tokens = nullptr, *out_count = nullptr, *pair = nullptr, *pairs = nullptr;
@@ -296,12 +300,14 @@ GemvFuse with_rms(const qmm_llama* m, int mode)
 }
 
 // h += W * x summed over the ranks; leaves pk_d = pack(h * norm_w) and ss_d for the matvec that follows.
-int linear_resid(qmm_llama* m, const qmm_weight* w, const uint8_t* packed_in, const float* norm_w, int site,
-                 cudaStream_t st)
+int linear_resid(qmm_llama* m, const qmm_weight* w, const uint8_t* packed_in, const float* x_f32, const float* norm_w,
+                 int site, cudaStream_t st)
 {
     const qmm_llama_config& c = m->cfg;
+    GemvFuse in = {};  // input side only: fp32 activations are packed by the matvec itself
+    in.x_f32 = x_f32;
     if (c.tp_size == 1) {
-        GemvFuse fu = {};
+        GemvFuse fu = in;
         fu.mode = EPI_RESID_PACK;
         fu.h_in = m->h;
         fu.h_out = m->h;
@@ -313,7 +319,7 @@ int linear_resid(qmm_llama* m, const qmm_weight* w, const uint8_t* packed_in, co
     if (m->xchg_ready) {
         // one kernel: partial sums, their exchange over peer memory, the sum over the ranks, residual, packing
         const PeerScatter ps = scatter_for(m, site);
-        GemvFuse fu = {};
+        GemvFuse fu = in;
         fu.mode = EPI_RESID_PACK;
         fu.h_in = m->h;
         fu.h_out = m->h;
@@ -323,7 +329,16 @@ int linear_resid(qmm_llama* m, const qmm_weight* w, const uint8_t* packed_in, co
         return qmm_internal_gemv_fused(w, packed_in, nullptr, &ps, &fu, st);
     }
     const PeerGather off = {};
-    LL_QMM(qmm_internal_gemv_fused(w, packed_in, m->y, nullptr, nullptr, st));
+    if (x_f32) {
+        WeightView view;
+        LL_QMM(qmm_internal_weight_view(w, &view));
+        if (!gemv_packs_itself(view, x_f32, m->y, m->sm_count)) {  // more row tiles than a plain matvec that packs can hold
+            LL_QMM(qmm_pack_activations(m->device, x_f32, 1, m->ffl, m->pk_act, st));
+            packed_in = m->pk_act;
+            in.x_f32 = nullptr;
+        }
+    }
+    LL_QMM(qmm_internal_gemv_fused(w, packed_in, m->y, nullptr, &in, st));
     LL_QMM(all_reduce(m, m->y, c.d_model, st));
     LL_CUDA(ll_resid_pack(m->h, m->y, norm_w, c.d_model, m->h, m->pk_d, m->ss_d, off, st));
     return QMM_OK;
@@ -379,12 +394,18 @@ int enqueue_decode_step(qmm_llama* m, cudaStream_t st)
         LL_QMM(qmm_internal_gemv_fused(L.w[QMM_LL_QKV], m->pk_d, m->qkv, nullptr, &rms, st));
         LL_CUDA(ll_attn_fused(m->qkv, m->pos, m->hl, m->kvl, c.head_dim, c.rope_dim, m->rope_cos, m->rope_sin,
                               c.max_seq, L.cache_k, L.cache_v, m->pk_ctx, 1, AttnBatch{}, st));
-        LL_QMM(linear_resid(m, L.w[QMM_LL_O], m->pk_ctx, L.ffn_norm, 2 * l, st));
+        LL_QMM(linear_resid(m, L.w[QMM_LL_O], m->pk_ctx, nullptr, L.ffn_norm, 2 * l, st));
         const float* next_norm = l + 1 < c.n_layers ? m->layers[l + 1].attn_norm : m->final_norm;
-        GemvFuse glu = with_rms(m, EPI_SWIGLU_PACK);
-        glu.packed_out = m->pk_act;
-        LL_QMM(qmm_internal_gemv_fused(L.w[QMM_LL_GU], m->pk_d, nullptr, nullptr, &glu, st));
-        LL_QMM(linear_resid(m, L.w[QMM_LL_DOWN], m->pk_act, next_norm, 2 * l + 1, st));
+        if (m->glu_packed) {
+            GemvFuse glu = with_rms(m, EPI_SWIGLU_PACK);
+            glu.packed_out = m->pk_act;
+            LL_QMM(qmm_internal_gemv_fused(L.w[QMM_LL_GU], m->pk_d, nullptr, nullptr, &glu, st));
+            LL_QMM(linear_resid(m, L.w[QMM_LL_DOWN], m->pk_act, nullptr, next_norm, 2 * l + 1, st));
+        } else {
+            const GemvFuse glu = with_rms(m, EPI_SWIGLU);
+            LL_QMM(qmm_internal_gemv_fused(L.w[QMM_LL_GU], m->pk_d, m->act_f, nullptr, &glu, st));
+            LL_QMM(linear_resid(m, L.w[QMM_LL_DOWN], nullptr, m->act_f, next_norm, 2 * l + 1, st));
+        }
     }
     return head_and_pick(m, st);
 }
@@ -578,6 +599,11 @@ int qmm_llama_create(int device, const qmm_llama_config* cfg, qmm_llama** out)
     LL_TRY(dev_alloc(m, &m->pk_d, pk));
     LL_TRY(qmm_packed_activation_bytes((int64_t)m->hl * hd, 1, &pk));
     LL_TRY(dev_alloc(m, &m->pk_ctx, pk));
+    LL_TRY(dev_alloc(m, &m->act_f, (size_t)m->ffl));
+    if (cudaDeviceGetAttribute(&m->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        LL_TRY(qmm_internal_fail(QMM_E_CUDA, "the device's SM count cannot be read"));
+    }
+    m->glu_packed = gemv_swiglu_packs(m->ffl / 8, (d + 255) / 256, m->sm_count);
     LL_TRY(dev_alloc(m, &m->pk_act, xpack1_bytes((m->ffl + 255) / 256)));  // zeroed: blocks past ffl stay zero
     LL_TRY(dev_alloc(m, &m->rope_cos, (size_t)c.max_seq * (c.rope_dim / 2)));
     LL_TRY(dev_alloc(m, &m->rope_sin, (size_t)c.max_seq * (c.rope_dim / 2)));

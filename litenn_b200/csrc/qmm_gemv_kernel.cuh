@@ -65,7 +65,7 @@ struct SmemPlan {
 template <int THREADS, int EPI, int TILES, bool XF32>
 constexpr int gemv_min_blocks()
 {
-    return TILES > epi_tiles(EPI) || (XF32 && EPI == EPI_STORE) || EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? 3 : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
+    return TILES > epi_tiles(EPI) || (XF32 && EPI == EPI_STORE) || EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? (THREADS <= 256 ? 3 : 1) : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
 }
 
 template <int FMT, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
@@ -662,8 +662,13 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
     if constexpr (EPI == EPI_SWIGLU_PACK) {
         // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
         // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
-        // 7B-shape step slower)
-        return launch_gemv_variant<FMT, 2, 2, EPI>(w, xp, y, status, ps, fu, stream);
+        // 7B-shape step slower).  Where a long row's CTAs have an SM each, four warps per tile: two keep too few bytes in
+        // flight (8192 wide, eight blocks, FFN 2304 Q4_0 200 -> 182 us a token, 3584 Q4_K 227 -> 209)
+        if (fu.x_f32 != nullptr) {
+            return cudaErrorInvalidValue;
+        }
+        const GemvWave<FMT, EPI, false> form{w, xp, y, status, ps, fu, stream};
+        return w.kc > 16 && w.rt <= TILES * sms ? form.template go<TILES, 4, 2, 2, 2>() : form.template go<TILES, 2, 2>();
     }
     if constexpr (TILES == 2) {
         // The residual form has two row tiles per CTA and n / 32 CTAs: 128 for a 4096-wide model, 256 for an

@@ -36,6 +36,15 @@ constexpr bool gemv_wave_fills(int rt, int group, int sms)
 {
     return 5LL * rt >= 4LL * sms * gemv_wave_tiles(rt, group, sms);
 }
+// Whether gate|up of a decode chain writes its product packed (EPI_SWIGLU_PACK, groups of four row tiles per CTA) or as fp32
+// from CTAs of one tile each (EPI_SWIGLU), which ffn_down then packs itself.  Packed costs less, but a long row (kc > 16) of
+// few tiles is bound by how many SMs read it: eight blocks, us a token, fp32 form and packed: 8192 wide, FFN 1024 Q4_0 154 and
+// 185, 1792 Q4_0 170 and 193, Q6_K 199 and 216; 2304 (288 tiles) Q4_0 180 and 200, with more warps per tile 182; Q6_K 239
+// and 229, with more warps 212; 3584 Q4_0 220 and 213.  12288 wide, FFN 1536 Q4_0 217 and 264, 2304 Q4_K 290 and 304.
+constexpr bool gemv_swiglu_packs(int rt, int kc, int sms)
+{
+    return kc <= 16 || 4LL * rt > 7LL * sms;
+}
 // Whether the matvec of one fp32 vector is one launch that packs x itself (launch_gemv_fused with fu.x_f32 and EPI_STORE).
 bool gemv_packs_itself(const WeightView& w, const float* x, const float* y, int sm_count);
 // per-format instantiations (qmm_gemv_<format>.cu)

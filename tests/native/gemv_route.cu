@@ -18,4 +18,10 @@ int gemv_one_launch(int fmt, int64_t n, int64_t k, uint64_t x, uint64_t y, int s
     return gemv_packs_itself(w, reinterpret_cast<const float*>(x), reinterpret_cast<const float*>(y), sm_count) ? 1 : 0;
 }
 
+// Whether gate|up of `channels` channels writes its product packed
+int swiglu_packs(int channels, int64_t k, int sm_count)
+{
+    return gemv_swiglu_packs((channels + 7) / 8, (int)((k + 255) / 256), sm_count) ? 1 : 0;
+}
+
 }  // extern "C"
