@@ -588,36 +588,84 @@ struct GemvWave {
     }
 };
 
-// Where the one-wave form takes a packed vector: not while the small CTAs of the forms below are all resident at once and
-// even (up to six per SM for 8 <= kc <= 16, which the larger tiles of Q8_0 and Q4_K's arithmetic stop earlier, three
-// above), except for two tiles per SM, where the small CTAs are either one or two to an SM (4096 x 4096: 7 % for every format).
-// Inside a chain (ss_in) small CTAs also start while the kernel before drains, which a CTA that fills its SM cannot: the
-// line lies at nine tiles (the vocabulary: 70B-shape token 562.3 -> 558.1 us; with the QKV matvec in it 564.5).
-// The residual form takes it from three tiles on, the packed gate|up form from nine on, as its groups of four tiles sit
-// three to an SM otherwise.  Tokens with three blocks, us: gate|up of 14336 x 4096 Q4_0 145.6 -> 135.8 and Q4_K 146.1 -> 140.5
-// (448 groups, 444 places), 11008 x 4096 Q8_0 226 -> 211 (four blocks); 6912 x 2560 and 8192 x 3072, below nine, move by
-// 1 % either way.  Residual of the 70B shape (8192 rows, four blocks): 550 -> 528.  A grid that the rounding to whole
-// groups leaves on fewer than four fifths of the SMs gains nothing there (5120 rows 205 -> 209, 7168 rows 215 -> 216).
+// Where the one-wave form takes a packed vector: where it was measured to be faster than the small CTAs of the forms below,
+// over every format, rows of 1..112 chunks and 2..28 tiles per SM.  Small CTAs that are all resident at once and even need no
+// wave of their own; how many an SM holds follows from the format's tiles and the warps that K gives them, so the lines lie
+// elsewhere for each.  Streams of different weights, us each, small CTAs and one wave, on both sides of a line:
+//   plain, K up to 16 chunks   two tiles per SM are one or two CTAs to an SM: 16 chunks 1.35 times, 4 chunks 0.98.
+//                              Q4_0 7 tiles 6 chunks 3.6 and 2.9, 3 chunks 2.6 and 3.0; 14 tiles 16 chunks 15.0 and 15.1,
+//                              16 tiles 16.7 and 18.1 (32 warps).  Q4_K 5 tiles 12 chunks 1.14 times, 7 chunks 3.8 and 4.2;
+//                              5 chunks 12 tiles 1.01 times, 14 tiles 0.94.  Q6_K 6 tiles 8 chunks 1.18 times, 9 chunks 0.95.
+//                              Q8_0 5 tiles 16 chunks 1.15 times, 12 chunks 6.5 and 7.2; 12 tiles 12 chunks 16.9 and 18.6
+//   longer rows                Q6_K 3 tiles and more 1.2..1.5 times; 4-bit rows of up to 30 chunks three CTAs to an SM at 3
+//                              tiles: 24 chunks 1.29 times with all places taken, 4.4 and 5.1 with few.  Q4_0 16 tiles 20
+//                              chunks 1.05 times, 32 chunks 0.94.  Q8_0 5 tiles 1.17 times, 8 tiles 0.98, 12 tiles 0.95
+//   plain, in a chain (ss_in)  small CTAs also start while the kernel before drains, which a CTA that fills its SM cannot: the
+//                              line lies at nine tiles (70B-shape vocabulary 562.3 -> 558.1 us a token; with the QKV matvec in
+//                              it 564.5).  Vocabularies of Q8_0: 12 chunks 1.00..1.05 times, 16..24 chunks 0.97..1.03
+//   residual (n / 32 small CTAs; grids that the rounding to whole groups leaves on fewer than four fifths of the SMs gain
+//                              nothing)  8192 rows, Q6_K 16 chunks 1.30 times, 32 chunks 0.97, 112 chunks 1.20; Q4_K 0.99,
+//                              0.94, 1.08; 9216 rows, Q4_0 16 chunks 1.18, 12 chunks 0.98; 12288 rows, Q4_0 16 chunks 1.17, 32
+//                              chunks 0.94, 80 chunks 1.12; 16384 rows, Q8_0 1.0..1.5 throughout, Q4_0 8 chunks 0.93, 12
+//                              chunks 1.20, 17 chunks 0.90
+//   packed gate|up             its groups of four tiles sit three to an SM: 12 tiles and fewer are one wave already (Q4_0
+//                              22016 x 4096 0.98, Q6_K 0.99; Q4_K 1.06 and with 27648 rows 0.96, Q8_0 1.21 and with 9 chunks
+//                              0.96).  13..16 tiles: Q4_0 16 chunks 1.12, 8 chunks 0.92; Q6_K 1.13, 1.20.  Q6_K 28 tiles 20
+//                              chunks 0.95
 template <int FMT, int EPI>
 bool gemv_one_wave(const WeightView& w, bool chained, int sms)
 {
-    const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms);
-    if (w.kc > GEMV_WAVE_KC || tiles > (EPI == EPI_SWIGLU_PACK || (EPI == EPI_STORE && tile_bytes(FMT) == 2304) ? 28 : 16)) {
+    constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
+    const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms), kc = w.kc;
+    if (kc > GEMV_WAVE_KC || tiles > (EPI == EPI_SWIGLU_PACK || (EPI == EPI_STORE && NIBBLE) ? 28 : 16)) {
         return false;
     }
     if constexpr (EPI == EPI_SWIGLU_PACK) {
-        return w.rt > 8 * sms;
+        if (tiles <= 12) {
+            return w.rt > 8 * sms && kc > 9 && (FMT == FMT_Q8_0 || (FMT == FMT_Q4_K && w.rt <= 11 * sms));
+        }
+        if (tiles <= 16) {
+            return !NIBBLE || kc > (FMT == FMT_Q4_0 ? 10 : 8);
+        }
+        return FMT != FMT_Q6_K || tiles <= 24 || kc <= 12;
+    } else if constexpr (EPI == EPI_RESID_PACK) {
+        if (w.rt <= 2 * sms || !gemv_wave_fills(w.rt, epi_tiles(EPI), sms)) {
+            return false;
+        }
+        if (tiles <= 4) {
+            return kc >= 96 || (FMT == FMT_Q6_K && kc > 8 && kc <= 16) ||
+                   (NIBBLE && kc > 12 && kc <= 16 && 10LL * w.rt >= 9LL * sms * tiles);
+        }
+        if (tiles <= 6) {
+            return kc > 64 || (FMT != FMT_Q8_0 && kc > 8 && kc <= 16);
+        }
+        return !NIBBLE || (kc > 8 && (tiles > 8 || kc <= 16 || kc >= 32));
+    } else {
+        if (FMT == FMT_Q4_0 && tiles > 14 && ((kc > 12 && kc <= 16) || (kc > 20 && tiles <= 16))) {
+            return false;
+        }
+        if (chained) {
+            return tiles >= 9 && (FMT != FMT_Q8_0 || kc <= 12);
+        }
+        if (kc > 16) {
+            return FMT == FMT_Q8_0   ? tiles >= (kc > 32 ? 4 : 5) && tiles <= 6
+                   : FMT == FMT_Q6_K ? tiles >= 3
+                                     : tiles >= 4 || (tiles == 3 && (kc > 30 || 2 * w.rt > 5 * sms));
+        }
+        if (tiles <= 2) {
+            return tiles == 2 && kc >= 5;
+        }
+        if constexpr (FMT == FMT_Q4_0) {
+            return tiles >= (kc >= 3 && kc <= 5 ? 8 : 7);
+        } else if constexpr (FMT == FMT_Q4_K) {
+            return tiles >= (kc <= 2 ? 6 : kc <= 5 ? 8 : kc <= 8 ? 7 : kc < 16 ? 5 : 4) &&
+                   !(kc >= 3 && kc <= 5 && tiles > 12 && tiles <= 14);
+        } else if constexpr (FMT == FMT_Q6_K) {
+            return tiles >= (kc > 8 && kc <= 12 ? 7 : 6);
+        } else {
+            return tiles >= (kc == 16 ? 5 : kc == 2 || kc == 3 ? 7 : 6) && (kc <= 10 || tiles <= 8);
+        }
     }
-    if constexpr (EPI == EPI_RESID_PACK) {
-        return w.rt > 2 * sms && gemv_wave_fills(w.rt, epi_tiles(EPI), sms);
-    }
-    if (chained) {
-        return tiles >= 9;
-    }
-    if (w.kc > 16) {
-        return tiles >= (FMT == FMT_Q8_0 ? 4 : 3);
-    }
-    return tiles == 2 || tiles >= (FMT == FMT_Q4_0 ? 7 : FMT == FMT_Q6_K ? 6 : FMT == FMT_Q8_0 ? 5 : 4);
 }
 
 // Batch 1: warps x ring slots by row length.

@@ -37,3 +37,37 @@ def test_long_rows_of_few_channels_are_read_by_blocks_of_one_row_tile(lib):
         assert not lib.swiglu_packs(channels, k, SMS), (k, channels)
     for k, channels in ((8192, 2304), (8192, 28672), (5120, 3456), (4096, 11008), (4096, 1376), (2048, 512)):
         assert lib.swiglu_packs(channels, k, SMS), (k, channels)
+
+
+STORE, RESIDUAL, GATE_UP = 0, 1, 3
+Q4_0, Q8_0, Q4_K, Q6_K = synth.Q4_0, synth.Q8_0, synth.Q4_K, synth.Q6_K
+
+
+@pytest.mark.parametrize("epi,chained,n,k,wave,small", [
+    # packed vector on its own: short rows of few tiles per SM stay with small blocks
+    (STORE, 0, 16000, 768, (Q8_0, Q6_K), (Q4_0, Q4_K)),
+    (STORE, 0, 10777, 1536, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    (STORE, 0, 11008, 2048, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    (STORE, 0, 16384, 2048, (Q4_0, Q8_0, Q4_K, Q6_K), ()),
+    (STORE, 0, 4096, 4096, (Q4_0, Q8_0, Q4_K, Q6_K), ()),
+    (STORE, 0, 10240, 8192, (Q4_0, Q8_0, Q4_K, Q6_K), ()),
+    (STORE, 0, 5000, 6144, (Q6_K,), (Q4_0, Q8_0, Q4_K)),
+    (STORE, 0, 36000, 8192, (Q4_K, Q6_K), (Q4_0, Q8_0)),
+    # vocabularies
+    (STORE, 1, 32000, 4096, (Q4_0, Q4_K, Q6_K), (Q8_0,)),
+    (STORE, 1, 12288, 4096, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    # residual matvecs
+    (RESIDUAL, 0, 8192, 1024, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    (RESIDUAL, 0, 8192, 4096, (Q6_K,), (Q4_0, Q8_0, Q4_K)),
+    (RESIDUAL, 0, 8192, 28672, (Q4_0, Q8_0, Q4_K, Q6_K), ()),
+    (RESIDUAL, 0, 12288, 8192, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    (RESIDUAL, 0, 16384, 5120, (Q8_0, Q6_K), (Q4_0, Q4_K)),
+    # gate|up
+    (GATE_UP, 1, 22016, 2048, (), (Q4_0, Q8_0, Q4_K, Q6_K)),
+    (GATE_UP, 1, 22016, 4096, (Q8_0, Q4_K), (Q4_0, Q6_K)),
+    (GATE_UP, 1, 28672, 4096, (Q4_0, Q8_0, Q4_K, Q6_K), ()),
+    (GATE_UP, 1, 57344, 8192, (Q4_0, Q8_0, Q4_K), (Q6_K,)),
+])
+def test_one_wave_is_taken_where_it_is_the_faster_form(lib, epi, chained, n, k, wave, small):
+    for fmt in wave + small:
+        assert bool(lib.gemv_takes_one_wave(fmt, epi, ctypes.c_int64(n), ctypes.c_int64(k), chained, SMS)) == (fmt in wave), fmt
