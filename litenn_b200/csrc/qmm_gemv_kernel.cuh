@@ -716,7 +716,9 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
             return cudaErrorInvalidValue;
         }
         const GemvWave<FMT, EPI, false> form{w, xp, y, status, ps, fu, stream};
-        return w.kc > 16 && w.rt <= TILES * sms ? form.template go<TILES, 4, 2, 2, 2>() : form.template go<TILES, 2, 2>();
+        // (one warp per tile where the activations of rows beyond 60000 columns leave no room for more slots)
+        return w.kc > 16 && w.rt <= TILES * sms ? form.template go<TILES, 4, 2, 2, 2, 1, 2>()
+                                                : form.template go<TILES, 2, 2, 1, 2>();
     }
     if constexpr (TILES == 2) {
         // The residual form has two row tiles per CTA and n / 32 CTAs: 128 for a 4096-wide model, 256 for an

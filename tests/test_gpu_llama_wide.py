@@ -19,6 +19,7 @@ def test_decode_matches_oracle(stream, fmt, ffn):  # noqa: F811
 
 
 @pytest.mark.parametrize("fmt", [capi.Q4_0, capi.Q8_0, capi.Q4_K, capi.Q6_K])
-@pytest.mark.parametrize("shape", [(2304, 4352), (64, 36864)])  # the second leaves Q8_0 no room for four warps per row tile
+# (64, 36864): no room for four warps per row tile of Q8_0; (64, 76032): for none of 1-byte and 6-bit tiles but one warp
+@pytest.mark.parametrize("shape", [(2304, 4352), (64, 36864), (64, 76032)])
 def test_gate_up_of_long_rows(torch_cuda, fmt, shape):  # noqa: F811
     check_gate_up(torch_cuda, fmt, shape)
