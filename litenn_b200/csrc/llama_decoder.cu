@@ -600,7 +600,8 @@ int qmm_llama_create(int device, const qmm_llama_config* cfg, qmm_llama** out)
     LL_TRY(qmm_packed_activation_bytes((int64_t)m->hl * hd, 1, &pk));
     LL_TRY(dev_alloc(m, &m->pk_ctx, pk));
     LL_TRY(dev_alloc(m, &m->act_f, (size_t)m->ffl));
-    if (cudaDeviceGetAttribute(&m->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    m->sm_count = sm_count_of(device);
+    if (m->sm_count < 1) {
         LL_TRY(qmm_internal_fail(QMM_E_CUDA, "the device's SM count cannot be read"));
     }
     m->glu_packed = gemv_swiglu_packs(m->ffl / 8, (d + 255) / 256, m->sm_count);

@@ -188,7 +188,7 @@ __host__ __device__ inline size_t xpack_bytes(int kc, int ncp)
 {
     return (size_t)kc * xpack_rec_bytes(ncp);
 }
-__host__ __device__ inline size_t xpack1_bytes(int kc)
+__host__ __device__ constexpr size_t xpack1_bytes(int kc)
 {
     return (size_t)kc * XPK1_REC;
 }
@@ -228,17 +228,17 @@ struct PeerScatter {
 //   EPI_RESID_PACK   h_out[row] = h_in[row] + sum * s_in; the matvec that follows reads
 //                    RMSNorm(h_out) * norm_w, so the epilogue writes h_out * norm_w as packed activations
 //                    (packed_out) and the sum of squares of its 32 rows (ss_out[n / 32], doubles); the
-//                    1/rms factor is a scalar and is applied by the consumer (ss_in above).  A CTA of
-//                    this form owns two row tiles = one 32-wide quantization block of the output.
+//                    1/rms factor is a scalar and is applied by the consumer (ss_in above).  Two row
+//                    tiles = one 32-wide quantization block of the output stay in one CTA.
 //   EPI_SWIGLU       rows are interleaved gate/up: tile rows 0..7 = gate channels 8*tile..8*tile+7, rows
 //                    8..15 = the same channels of up; y[channel] = silu(gate * s_in) * (up * s_in)
 //   EPI_SWIGLU_PACK  the same product written as the packed input of the matvec that follows (packed_out;
-//                    y optional): a CTA of this form owns four row tiles = 32 channels = one quantization block
+//                    y optional): four row tiles = 32 channels = one quantization block stay in one CTA
 constexpr int EPI_STORE = 0;
 constexpr int EPI_RESID_PACK = 1;
 constexpr int EPI_SWIGLU = 2;
 constexpr int EPI_SWIGLU_PACK = 3;
-// Row tiles one CTA owns in each form.
+// The smallest group of row tiles that a form keeps in one CTA; a CTA owns one group or, in the one-wave forms, several.
 __host__ __device__ constexpr int epi_tiles(int epi)
 {
     return epi == EPI_RESID_PACK ? 2 : epi == EPI_SWIGLU_PACK ? 4 : 1;

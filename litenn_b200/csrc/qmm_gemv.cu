@@ -1,6 +1,9 @@
 // Activation packing for the integer-MMA matvec and the dispatch of a matvec to the block
 // format's kernels (qmm_gemv_kernel.cuh, instantiated per format in qmm_gemv_<format>.cu).
+#include <atomic>
+
 #include "qmm_gemv_device.cuh"
+#include "qmm_gemv_forms.cuh"
 #include "qmm_kernels.h"
 #include "qmm_pack.cuh"
 
@@ -152,11 +155,24 @@ cudaError_t launch_unpack_x(const uint8_t* packed, int64_t k, float* x, cudaStre
     return cudaGetLastError();
 }
 
-// One launch instead of two while every SM's copy of the vector costs less than the packing kernel and its boundary (1.1 us
-// of a stream, 2.6 us of a host loop, where 1024 x 4096 falls from 7.0 to 5.2 us).  Up to 32 chunks it does, the one wave
-// being also the better matvec; above, packing 11008 values takes 256 rows of Q4_0 5.5 us and not 4.4, and only Q8_0
-// on one row tile per SM gains (7.5 -> 5.9).  Q8_0 beyond 16 chunks is bound by its bytes either way (28672 x 8192: 39.7
-// us, 40.5 in one launch).  Of many tiles per SM only the 4-bit formats have room for enough slots.
+int sm_count_of(int dev)
+{
+    static std::atomic<int> known[64];
+    if (dev >= 0 && dev < 64) {
+        if (const int n = known[dev].load(std::memory_order_relaxed)) {
+            return n;
+        }
+    }
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        return 0;
+    }
+    if (dev >= 0 && dev < 64) {
+        known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // Never where y lies over x: CTAs that are done store y while others still read x.  The packing kernel reads all of x first.
 bool gemv_packs_itself(const WeightView& w, const float* x, const float* y, int sm_count)
 {
@@ -165,17 +181,10 @@ bool gemv_packs_itself(const WeightView& w, const float* x, const float* y, int 
     if (x0 < y1 && y0 < x1) {
         return false;
     }
-    if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || w.k % 32 != 0 || sm_count < 1) {  // x is read 16 bytes at a time
+    if ((x0 & 15u) != 0 || w.k % 32 != 0 || sm_count < 1) {  // x is read 16 bytes at a time
         return false;
     }
-    const int tiles = (w.rt + sm_count - 1) / sm_count;
-    if (w.kc > 32) {
-        return w.fmt == FMT_Q8_0 && tiles == 1 && w.kc <= GEMV_WAVE_KC;
-    }
-    if (w.fmt == FMT_Q8_0) {
-        return tiles <= (w.kc > 16 ? 2 : 16);
-    }
-    return tiles <= (w.fmt == FMT_Q6_K ? 16 : 28);
+    return gemv_packs_itself_shape(w.fmt, w.rt, w.kc, sm_count);
 }
 
 cudaError_t launch_gemv_fused(const WeightView& w, const XPackView& xp, float* y, int m, int* status,

@@ -472,26 +472,19 @@ cudaError_t launch_gemv_batch(const WeightView& w, const XPackView& xp, float* y
     using Plan = BatchPlan<FMT, NM>;
     auto kernel = gemv_batch_kernel<FMT, NM>;
     static std::mutex mu;
-    static int sm_count[64] = {};
     static int configured[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
         return e;
     }
+    const int sms = sm_count_of(dev);
+    if (sms < 1) {
+        return cudaErrorInvalidDevice;
+    }
     int smem = Plan::TOTAL;
     {
         std::lock_guard<std::mutex> lock(mu);
-        int sms = dev < 64 ? sm_count[dev] : 0;
-        if (sms == 0) {
-            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e != cudaSuccess) {
-                return e;
-            }
-            if (dev < 64) {
-                sm_count[dev] = sms;
-            }
-        }
         // Residency cap.  The block scheduler fills an SM up to its limit before it is even with the others, so a grid that
         // could sit 7 to an SM leaves a third of the SMs with little to do (688 CTAs of the one-row kernel: 6.7 us at a limit
         // of 7, 5.2 us at 5).  The dynamic shared memory request is padded so that no SM can hold more than its even share,

@@ -3,7 +3,8 @@
 // unit of its own (qmm_gemv_q4_0.cu, ...), so the formats compile in parallel.  2..16 rows are qmm_gemv_batch.cuh.
 //
 // The weights never become floats in memory.  One CTA owns one 16-row tile of the
-// output; its warps take the 256-column K chunks of that row tile round-robin.
+// output, or several (TILES: the fused forms' groups, and the one-wave forms of qmm_gemv_forms.cuh, which also choose
+// among the small ones of gate|up); WARPS warps take the 256-column K chunks of each row tile round-robin.
 // Every chunk is one contiguous packed tile (qmm_common.cuh) that a single TMA bulk
 // copy (cp.async.bulk, completion counted on an mbarrier) lands in a shared-memory
 // slot.  Each warp owns DEPTH slots and refills a slot itself as soon as it has
@@ -29,11 +30,11 @@
 // norm weights folded in) or silu(gate) * up from its epilogue.
 #pragma once
 
-#include <atomic>
 #include <mutex>
 
 #include "qmm_gemv_batch.cuh"
 #include "qmm_gemv_device.cuh"
+#include "qmm_gemv_forms.cuh"
 #include "qmm_kernels.h"
 #include "qmm_pack.cuh"
 
@@ -41,22 +42,7 @@ namespace qmm {
 
 namespace {
 
-// Shared memory of one CTA, carved from the dynamic allocation:
-//   slots  TILES*WARPS*DEPTH x tile | mbarriers (+1 for the activations) | all activation records + 512 zero bytes |
-//   cross-warp reduction
-template <int FMT, int WARPS, int DEPTH, int TILES>
-struct SmemPlan {
-    static constexpr int NW = WARPS * TILES;
-    static constexpr int SLOT = tile_bytes(FMT);
-    static constexpr int SLOTS_BYTES = NW * DEPTH * SLOT;
-    static constexpr int BAR_OFF = SLOTS_BYTES;
-    static constexpr int BAR_BYTES = (((NW * DEPTH + 1) * 8 + 15) / 16) * 16;
-    static constexpr int X_OFF = BAR_OFF + BAR_BYTES;
-    __host__ __device__ static int red_off(int kc) { return X_OFF + (int)xpack1_bytes(kc) + 512; }
-    __host__ __device__ static int total(int kc) { return red_off(kc) + NW * 16 * 4; }
-};
-
-// WARPS warps share one row tile; a CTA holds TILES row tiles (2 for EPI_RESID_PACK: the 32 rows of
+// WARPS warps share one row tile; a CTA holds TILES row tiles (at least 2 for EPI_RESID_PACK: the 32 rows of
 // one quantization block of the output, so the epilogue can quantize them without leaving the CTA).
 // Registers decide how many CTAs an SM holds, and a batch-1 grid of 768 row tiles wants six CTAs of
 // 256 threads on every SM at once (42 registers at most): the bound keeps the fp32-packing prologue
@@ -65,7 +51,13 @@ struct SmemPlan {
 template <int THREADS, int EPI, int TILES, bool XF32>
 constexpr int gemv_min_blocks()
 {
-    return TILES > epi_tiles(EPI) || (XF32 && EPI == EPI_STORE) || EPI == EPI_RESID_PACK ? 1 : EPI == EPI_SWIGLU_PACK ? (THREADS <= 256 ? 3 : 1) : (THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3);
+    if (TILES > epi_tiles(EPI) || (XF32 && EPI == EPI_STORE) || EPI == EPI_RESID_PACK) {  // the one-wave forms, and few CTAs
+        return 1;
+    }
+    if (EPI == EPI_SWIGLU_PACK) {
+        return THREADS <= 256 ? 3 : 1;
+    }
+    return THREADS <= 128 ? 8 : THREADS <= 256 ? 6 : 3;
 }
 
 template <int FMT, int WARPS, int DEPTH, int EPI, int TILES, bool XF32>
@@ -368,25 +360,6 @@ __global__ void __launch_bounds__(WARPS * TILES * 32, gemv_min_blocks<WARPS * TI
     }
 }
 
-// SMs of a device, 0 if it cannot be asked; asked once.
-inline int sm_count_of(int dev)
-{
-    static std::atomic<int> known[64];
-    if (dev >= 0 && dev < 64) {
-        if (const int n = known[dev].load(std::memory_order_relaxed)) {
-            return n;
-        }
-    }
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        return 0;
-    }
-    if (dev >= 0 && dev < 64) {
-        known[dev].store(n, std::memory_order_relaxed);
-    }
-    return n;
-}
-
 // Ring depth per format: 28-37 KB of tiles in flight per CTA.
 template <int FMT>
 struct Tune {
@@ -451,6 +424,24 @@ cudaError_t launch_gemv_xsrc(const WeightView& w, const XPackView& xp, float* y,
     return cudaLaunchKernelEx(&cfg, kernel, w, xp, y, status, ps, fu);
 }
 
+// Launches the form that gemv_wave_form or gemv_small_glu_form chooses.
+template <int FMT, int EPI, bool XF32>
+struct GemvLaunch {
+    const WeightView& w;
+    const XPackView& xp;
+    float* y;
+    int* status;
+    const PeerScatter& ps;
+    const GemvFuse& fu;
+    cudaStream_t stream;
+
+    template <int TILES, int WARPS, int DEPTH>
+    cudaError_t form() const
+    {
+        return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, XF32, TILES>(w, xp, y, status, ps, fu, stream);
+    }
+};
+
 template <int FMT, int WARPS, int DEPTH, int EPI>
 cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float* y, int* status,
                                 const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream)
@@ -464,208 +455,6 @@ cudaError_t launch_gemv_variant(const WeightView& w, const XPackView& xp, float*
         return cudaErrorInvalidValue;
     }
     return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, false>(w, xp, y, status, ps, fu, stream);
-}
-
-// The one-wave form: a CTA on every SM, each with as many row tiles as that takes (ceil(tiles / SMs), up to the next
-// compiled count), WARPS warps and WARPS x DEPTH slots per tile.  What bounds a matvec of many small CTAs is the last
-// of its waves and, for an fp32 vector, that every CTA packs the vector again; here there is one wave and at most 148
-// copies.  Measured on B200, a stream of different weights, us each, many CTAs -> one wave:
-//   packed vector  Q4_0 8192 x 28672 28.9 -> 22.4, 10240 x 8192 12.4 -> 9.4, 28672 x 8192 27.4 -> 22.7, 4096 x 4096 3.8 -> 3.5;
-//                  Q4_K 28672 x 8192 29.9 -> 22.6, 11008 x 4096 7.4 -> 6.7; Q6_K 28672 x 8192 35.4 -> 31.5, 14336 x 4096
-//                  11.1 -> 9.7; Q8_0 11008 x 4096 11.0 -> 9.5
-//   fp32 vector    (before: a kernel that packs it, then the matvec) Q4_0 1024 x 4096 4.2 -> 3.0, 14336 x 4096 9.5 -> 8.1,
-//                  28672 x 8192 28.2 -> 23.9; Q4_K 14336 x 4096 10.6 -> 9.0; Q6_K 4096 x 2048 4.2 -> 3.4; Q8_0 4096 x 4096 6.0 -> 5.4
-// More warps per tile shorten a short row's chain of tiles; more than about 90 KB of slots gains nothing, so the warps per
-// tile fall as the tiles grow.  The shared-memory request keeps a second CTA of the same kernel off an SM: without
-// it, 4096 x 8192 of Q4_K takes 7.2 us and not 5.6.  LESS: warps and depth to fall back to where long rows leave less room
-// for slots; with at most GEMV_WAVE_KC chunks the last entry always fits.
-template <int FMT, int EPI, bool XF32>
-struct GemvWave {
-    const WeightView& w;
-    const XPackView& xp;
-    float* y;
-    int* status;
-    const PeerScatter& ps;
-    const GemvFuse& fu;
-    cudaStream_t stream;
-    static constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
-
-    template <int TILES, int WARPS, int DEPTH, int... LESS>
-    cudaError_t go() const
-    {
-        if constexpr (TILES % epi_tiles(EPI) != 0) {
-            return cudaErrorInvalidConfiguration;  // not reached: the caller rounds up to whole groups
-        } else if constexpr (sizeof...(LESS) > 0) {
-            if (SmemPlan<FMT, WARPS, DEPTH, TILES>::total(w.kc) > 227 * 1024) {
-                return go<TILES, LESS...>();
-            }
-            return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, XF32, TILES>(w, xp, y, status, ps, fu, stream);
-        } else {
-            return launch_gemv_xsrc<FMT, WARPS, DEPTH, EPI, XF32, TILES>(w, xp, y, status, ps, fu, stream);
-        }
-    }
-
-    cudaError_t launch(int sms) const
-    {
-        const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms);
-        if constexpr (EPI == EPI_SWIGLU_PACK) {
-            if (tiles > 12) {
-                return launch_many(tiles);
-            }
-            return go<12, 2, 2, 2, 1>();  // nine tiles at least
-        } else {
-            return launch_few(tiles);
-        }
-    }
-
-    cudaError_t launch_few(int tiles) const
-    {
-        const bool small = w.kc <= 8;  // two tiles per warp at most, whatever the form: fewer warps to add up
-        if constexpr (EPI == EPI_STORE) {
-            if (tiles <= 1) {
-                return w.kc <= 4 ? go<1, 8, 1>() : go<1, 16, 2>();
-            }
-            if (tiles == 2) {
-                return go<2, 8, 2>();
-            }
-            if (tiles == 3) {
-                return small && w.kc > 4 ? go<3, 8, 1>() : go<3, 5, 2>();
-            }
-        }
-        if (tiles == 4) {
-            return go<4, 4, 3, 4, 2>();
-        }
-        if (tiles == 5) {
-            return go<5, 4, 2, 4, 1>();
-        }
-        if (tiles == 6) {
-            return small ? go<6, 2, 2>() : go<6, 4, 2, 2, 2>();
-        }
-        if (tiles == 7) {
-            if constexpr (NIBBLE) {
-                return small ? go<7, 2, 2>() : go<7, 4, 2>();
-            } else {
-                return small ? go<7, 2, 2>() : go<7, 2, 3, 2, 2>();
-            }
-        }
-        if (tiles == 8) {
-            return small ? go<8, 2, 2>() : go<8, 2, 3, 2, 2>();
-        }
-        if (tiles <= 10) {
-            return go<10, 2, 2, 2, 1>();
-        }
-        if (tiles <= 12) {
-            return go<12, 2, 2, 2, 1>();
-        }
-        return launch_many(tiles);
-    }
-
-    cudaError_t launch_many(int tiles) const
-    {
-        // Q6_K and Q8_0 leave room for two warps per row tile only with one slot each: one warp with three is 4 % faster.
-        // So it is inside a chain for every format, as 32 warps of 64 registers leave the next kernel none (28672 x 7168
-        // and three blocks, Q4_0: 227 us a token with two warps, 200 with one).
-        if (tiles <= 16) {
-            if constexpr (NIBBLE && EPI == EPI_STORE) {
-                return tiles <= 14 ? go<14, 2, 2>() : go<16, 2, 2>();
-            } else {
-                return tiles <= 14 ? go<14, 1, 3, 1, 2>() : go<16, 1, 3, 1, 2>();
-            }
-        }
-        if constexpr (EPI == EPI_SWIGLU_PACK) {
-            return tiles <= 20   ? go<20, 1, 2, 1, 1>()
-                   : tiles <= 24 ? go<24, 1, 2, 1, 1>()
-                   : tiles <= 28 ? go<28, 1, 2, 1, 1>()
-                                 : cudaErrorInvalidConfiguration;
-        }
-        if constexpr (EPI == EPI_STORE && NIBBLE) {
-            return tiles <= 20   ? go<20, 1, 2>()
-                   : tiles <= 25 ? go<25, 1, 2>()
-                   : tiles <= 28 ? go<28, 1, 2>()
-                                 : cudaErrorInvalidConfiguration;
-        }
-        return cudaErrorInvalidConfiguration;
-    }
-};
-
-// Where the one-wave form takes a packed vector: where it was measured to be faster than the small CTAs of the forms below,
-// over every format, rows of 1..112 chunks and 2..28 tiles per SM.  Small CTAs that are all resident at once and even need no
-// wave of their own; how many an SM holds follows from the format's tiles and the warps that K gives them, so the lines lie
-// elsewhere for each.  Streams of different weights, us each, small CTAs and one wave, on both sides of a line:
-//   plain, K up to 16 chunks   two tiles per SM are one or two CTAs to an SM: 16 chunks 1.35 times, 4 chunks 0.98.
-//                              Q4_0 7 tiles 6 chunks 3.6 and 2.9, 3 chunks 2.6 and 3.0; 14 tiles 16 chunks 15.0 and 15.1,
-//                              16 tiles 16.7 and 18.1 (32 warps).  Q4_K 5 tiles 12 chunks 1.14 times, 7 chunks 3.8 and 4.2;
-//                              5 chunks 12 tiles 1.01 times, 14 tiles 0.94.  Q6_K 6 tiles 8 chunks 1.18 times, 9 chunks 0.95.
-//                              Q8_0 5 tiles 16 chunks 1.15 times, 12 chunks 6.5 and 7.2; 12 tiles 12 chunks 16.9 and 18.6
-//   longer rows                Q6_K 3 tiles and more 1.2..1.5 times; 4-bit rows of up to 30 chunks three CTAs to an SM at 3
-//                              tiles: 24 chunks 1.29 times with all places taken, 4.4 and 5.1 with few.  Q4_0 16 tiles 20
-//                              chunks 1.05 times, 32 chunks 0.94.  Q8_0 5 tiles 1.17 times, 8 tiles 0.98, 12 tiles 0.95
-//   plain, in a chain (ss_in)  small CTAs also start while the kernel before drains, which a CTA that fills its SM cannot: the
-//                              line lies at nine tiles (70B-shape vocabulary 562.3 -> 558.1 us a token; with the QKV matvec in
-//                              it 564.5).  Vocabularies of Q8_0: 12 chunks 1.00..1.05 times, 16..24 chunks 0.97..1.03
-//   residual (n / 32 small CTAs; grids that the rounding to whole groups leaves on fewer than four fifths of the SMs gain
-//                              nothing)  8192 rows, Q6_K 16 chunks 1.30 times, 32 chunks 0.97, 112 chunks 1.20; Q4_K 0.99,
-//                              0.94, 1.08; 9216 rows, Q4_0 16 chunks 1.18, 12 chunks 0.98; 12288 rows, Q4_0 16 chunks 1.17, 32
-//                              chunks 0.94, 80 chunks 1.12; 16384 rows, Q8_0 1.0..1.5 throughout, Q4_0 8 chunks 0.93, 12
-//                              chunks 1.20, 17 chunks 0.90
-//   packed gate|up             its groups of four tiles sit three to an SM: 12 tiles and fewer are one wave already (Q4_0
-//                              22016 x 4096 0.98, Q6_K 0.99; Q4_K 1.06 and with 27648 rows 0.96, Q8_0 1.21 and with 9 chunks
-//                              0.96).  13..16 tiles: Q4_0 16 chunks 1.12, 8 chunks 0.92; Q6_K 1.13, 1.20.  Q6_K 28 tiles 20
-//                              chunks 0.95
-template <int FMT, int EPI>
-bool gemv_one_wave(const WeightView& w, bool chained, int sms)
-{
-    constexpr bool NIBBLE = tile_bytes(FMT) == 2304;
-    const int tiles = gemv_wave_tiles(w.rt, epi_tiles(EPI), sms), kc = w.kc;
-    if (kc > GEMV_WAVE_KC || tiles > (EPI == EPI_SWIGLU_PACK || (EPI == EPI_STORE && NIBBLE) ? 28 : 16)) {
-        return false;
-    }
-    if constexpr (EPI == EPI_SWIGLU_PACK) {
-        if (tiles <= 12) {
-            return w.rt > 8 * sms && kc > 9 && (FMT == FMT_Q8_0 || (FMT == FMT_Q4_K && w.rt <= 11 * sms));
-        }
-        if (tiles <= 16) {
-            return !NIBBLE || kc > (FMT == FMT_Q4_0 ? 10 : 8);
-        }
-        return FMT != FMT_Q6_K || tiles <= 24 || kc <= 12;
-    } else if constexpr (EPI == EPI_RESID_PACK) {
-        if (w.rt <= 2 * sms || !gemv_wave_fills(w.rt, epi_tiles(EPI), sms)) {
-            return false;
-        }
-        if (tiles <= 4) {
-            return kc >= 96 || (FMT == FMT_Q6_K && kc > 8 && kc <= 16) ||
-                   (NIBBLE && kc > 12 && kc <= 16 && 10LL * w.rt >= 9LL * sms * tiles);
-        }
-        if (tiles <= 6) {
-            return kc > 64 || (FMT != FMT_Q8_0 && kc > 8 && kc <= 16);
-        }
-        return !NIBBLE || (kc > 8 && (tiles > 8 || kc <= 16 || kc >= 32));
-    } else {
-        if (FMT == FMT_Q4_0 && tiles > 14 && ((kc > 12 && kc <= 16) || (kc > 20 && tiles <= 16))) {
-            return false;
-        }
-        if (chained) {
-            return tiles >= 9 && (FMT != FMT_Q8_0 || kc <= 12);
-        }
-        if (kc > 16) {
-            return FMT == FMT_Q8_0   ? tiles >= (kc > 32 ? 4 : 5) && tiles <= 6
-                   : FMT == FMT_Q6_K ? tiles >= 3
-                                     : tiles >= 4 || (tiles == 3 && (kc > 30 || 2 * w.rt > 5 * sms));
-        }
-        if (tiles <= 2) {
-            return tiles == 2 && kc >= 5;
-        }
-        if constexpr (FMT == FMT_Q4_0) {
-            return tiles >= (kc >= 3 && kc <= 5 ? 8 : 7);
-        } else if constexpr (FMT == FMT_Q4_K) {
-            return tiles >= (kc <= 2 ? 6 : kc <= 5 ? 8 : kc <= 8 ? 7 : kc < 16 ? 5 : 4) &&
-                   !(kc >= 3 && kc <= 5 && tiles > 12 && tiles <= 14);
-        } else if constexpr (FMT == FMT_Q6_K) {
-            return tiles >= (kc > 8 && kc <= 12 ? 7 : 6);
-        } else {
-            return tiles >= (kc == 16 ? 5 : kc == 2 || kc == 3 ? 7 : 6) && (kc <= 10 || tiles <= 8);
-        }
-    }
 }
 
 // Batch 1: warps x ring slots by row length.
@@ -684,8 +473,7 @@ template <int FMT, int EPI>
 cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, int* status, const PeerScatter& ps,
                            const GemvFuse& fu, cudaStream_t stream)
 {
-    constexpr int TILES = epi_tiles(EPI);
-    constexpr int LIMIT = 113 * 1024;
+    [[maybe_unused]] constexpr int LIMIT = 113 * 1024;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) {
@@ -697,30 +485,22 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
     }
     if constexpr (EPI == EPI_STORE) {
         if (fu.x_f32 != nullptr) {  // gemv_packs_itself says which
-            return GemvWave<FMT, EPI, true>{w, xp, y, status, ps, fu, stream}.launch(sms);
+            return gemv_wave_form<FMT, EPI, true>(w.rt, w.kc, sms, GemvLaunch<FMT, EPI, true>{w, xp, y, status, ps, fu, stream});
         }
     }
     if constexpr (EPI != EPI_SWIGLU) {
         // (a tensor-parallel rank keeps the residual form that waits for its peers in small CTAs)
         if (fu.x_f32 == nullptr && !(EPI == EPI_RESID_PACK && ps.n_peers > 0) &&
-            gemv_one_wave<FMT, EPI>(w, fu.ss_in != nullptr, sms)) {
-            return GemvWave<FMT, EPI, false>{w, xp, y, status, ps, fu, stream}.launch(sms);
+            gemv_one_wave<FMT, EPI>(w.rt, w.kc, fu.ss_in != nullptr, sms)) {
+            return gemv_wave_form<FMT, EPI, false>(w.rt, w.kc, sms, GemvLaunch<FMT, EPI, false>{w, xp, y, status, ps, fu, stream});
         }
     }
     if constexpr (EPI == EPI_SWIGLU_PACK) {
-        // four row tiles per CTA, two warps per tile with two slots each: 8 warps walk kc / 2 tiles apiece
-        // (8 for K = 4096) and a third of a 1376-tile gate|up weight's CTAs fit an SM together (three slots: 1 % of a
-        // 7B-shape step slower).  Where a long row's CTAs have an SM each, four warps per tile: two keep too few bytes in
-        // flight (8192 wide, eight blocks, FFN 2304 Q4_0 200 -> 182 us a token, 3584 Q4_K 227 -> 209)
         if (fu.x_f32 != nullptr) {
             return cudaErrorInvalidValue;
         }
-        const GemvWave<FMT, EPI, false> form{w, xp, y, status, ps, fu, stream};
-        // (one warp per tile where the activations of rows beyond 60000 columns leave no room for more slots)
-        return w.kc > 16 && w.rt <= TILES * sms ? form.template go<TILES, 4, 2, 2, 2, 1, 2>()
-                                                : form.template go<TILES, 2, 2, 1, 2>();
-    }
-    if constexpr (TILES == 2) {
+        return gemv_small_glu_form<FMT>(w.rt, w.kc, sms, GemvLaunch<FMT, EPI, false>{w, xp, y, status, ps, fu, stream});
+    } else if constexpr (EPI == EPI_RESID_PACK) {
         // The residual form has two row tiles per CTA and n / 32 CTAs: 128 for a 4096-wide model, 256 for an
         // 8192-wide one.  All of them should be resident at once (a second wave of a few CTAs doubles the
         // kernel's time), so the variant is the deepest one whose shared memory lets ceil(CTAs / SMs) CTAs
@@ -729,13 +509,19 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         const int ctas = w.rt / 2;
         const int per_sm = (ctas + sms - 1) / sms;
         const int budget = 232448 / per_sm - 1280;
-        // 4-bit rows of up to 16 chunks: four warps with four slots, every tile requested at once (7B-shape step with eight
-        // blocks 304.9 -> 302.5 us against eight warps with one slot)
-        if (tile_bytes(FMT) == 2304 && w.kc > 8 && w.kc <= 16 && SmemPlan<FMT, 4, 4, 2>::total(w.kc) <= budget) {
-            return launch_gemv_variant<FMT, 4, 4, EPI>(w, xp, y, status, ps, fu, stream);
-        }
-        if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0 && SmemPlan<FMT, 8, 1, 2>::total(w.kc) <= budget) {
-            return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
+        if (w.kc > 8 && w.kc <= 16) {
+            // 4-bit rows of up to 16 chunks: four warps with four slots, every tile requested at once (7B-shape step with
+            // eight blocks 304.9 -> 302.5 us against eight warps with one slot)
+            if constexpr (tile_bytes(FMT) == 2304) {
+                if (SmemPlan<FMT, 4, 4, 2>::total(w.kc) <= budget) {
+                    return launch_gemv_variant<FMT, 4, 4, EPI>(w, xp, y, status, ps, fu, stream);
+                }
+            }
+            if constexpr (FMT != FMT_Q8_0) {
+                if (SmemPlan<FMT, 8, 1, 2>::total(w.kc) <= budget) {
+                    return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
+                }
+            }
         }
         if (w.kc > 16 && SmemPlan<FMT, 8, 3, 2>::total(w.kc) <= budget) {
             return launch_gemv_variant<FMT, 8, 3, EPI>(w, xp, y, status, ps, fu, stream);
@@ -749,20 +535,25 @@ cudaError_t launch_gemv_m1(const WeightView& w, const XPackView& xp, float* y, i
         // more than one CTA per SM wanted and nothing deeper fits: one slot per warp, the number of CTAs keeps
         // the bytes in flight up
         return launch_gemv_variant<FMT, 4, 1, EPI>(w, xp, y, status, ps, fu, stream);
+    } else {
+        if (w.kc > 8 && w.kc <= 16) {
+            if constexpr (tile_bytes(FMT) == 2304 && EPI == EPI_STORE) {
+                if (fu.ss_in != nullptr) {
+                    return launch_gemv_variant<FMT, 4, 2, EPI>(w, xp, y, status, ps, fu, stream);
+                }
+            }
+            if constexpr (FMT != FMT_Q8_0) {
+                return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
+            }
+        }
+        if (w.kc > 32 && SmemPlan<FMT, 16, 2, 1>::total(w.kc) <= LIMIT) {
+            return launch_gemv_variant<FMT, 16, 2, EPI>(w, xp, y, status, ps, fu, stream);
+        }
+        if (w.kc > 16 && SmemPlan<FMT, 8, 3, 1>::total(w.kc) <= LIMIT) {
+            return launch_gemv_variant<FMT, 8, 3, EPI>(w, xp, y, status, ps, fu, stream);
+        }
+        return launch_gemv_variant<FMT, Tune<FMT>::WARPS, Tune<FMT>::DEPTH, EPI>(w, xp, y, status, ps, fu, stream);
     }
-    if (tile_bytes(FMT) == 2304 && EPI == EPI_STORE && fu.ss_in != nullptr && w.kc > 8 && w.kc <= 16) {
-        return launch_gemv_variant<FMT, 4, 2, EPI>(w, xp, y, status, ps, fu, stream);
-    }
-    if (w.kc > 8 && w.kc <= 16 && FMT != FMT_Q8_0) {
-        return launch_gemv_variant<FMT, 8, 1, EPI>(w, xp, y, status, ps, fu, stream);
-    }
-    if (w.kc > 32 && SmemPlan<FMT, 16, 2, 1>::total(w.kc) <= LIMIT) {
-        return launch_gemv_variant<FMT, 16, 2, EPI>(w, xp, y, status, ps, fu, stream);
-    }
-    if (w.kc > 16 && SmemPlan<FMT, 8, 3, TILES>::total(w.kc) <= LIMIT) {
-        return launch_gemv_variant<FMT, 8, 3, EPI>(w, xp, y, status, ps, fu, stream);
-    }
-    return launch_gemv_variant<FMT, Tune<FMT>::WARPS, Tune<FMT>::DEPTH, EPI>(w, xp, y, status, ps, fu, stream);
 }
 
 template <int FMT>

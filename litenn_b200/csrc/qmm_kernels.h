@@ -24,18 +24,8 @@ cudaError_t launch_gemv(const WeightView& w, const XPackView& xp, float* y, int 
 // `fu` asks for an input RMSNorm factor or a fused epilogue (GemvFuse); both in qmm_common.cuh.
 cudaError_t launch_gemv_fused(const WeightView& w, const XPackView& xp, float* y, int m, int* status,
                               const PeerScatter& ps, const GemvFuse& fu, cudaStream_t stream);
-// The one-wave matvec: row tiles per CTA, in whole groups of a fused form (epi_tiles), that put every tile on the chip at
-// once, and whether such CTAs sit on at least four fifths of the SMs.  Rows of more than GEMV_WAVE_KC chunks do not leave it
-// the shared memory.
-constexpr int GEMV_WAVE_KC = 112;
-constexpr int gemv_wave_tiles(int rt, int group, int sms)
-{
-    return ((rt + sms - 1) / sms + group - 1) / group * group;
-}
-constexpr bool gemv_wave_fills(int rt, int group, int sms)
-{
-    return 5LL * rt >= 4LL * sms * gemv_wave_tiles(rt, group, sms);
-}
+// SMs of a device, 0 if it cannot be asked; asked once.
+int sm_count_of(int dev);
 // Whether gate|up of a decode chain writes its product packed (EPI_SWIGLU_PACK, groups of four row tiles per CTA) or as fp32
 // from CTAs of one tile each (EPI_SWIGLU), which ffn_down then packs itself.  Packed costs less, but a long row (kc > 16) of
 // few tiles is bound by how many SMs read it: eight blocks, us a token, fp32 form and packed: 8192 wide, FFN 1024 Q4_0 154 and

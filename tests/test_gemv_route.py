@@ -71,3 +71,10 @@ Q4_0, Q8_0, Q4_K, Q6_K = synth.Q4_0, synth.Q8_0, synth.Q4_K, synth.Q6_K
 def test_one_wave_is_taken_where_it_is_the_faster_form(lib, epi, chained, n, k, wave, small):
     for fmt in wave + small:
         assert bool(lib.gemv_takes_one_wave(fmt, epi, ctypes.c_int64(n), ctypes.c_int64(k), chained, SMS)) == (fmt in wave), fmt
+
+
+@pytest.mark.parametrize("epi,xf32", [(STORE, 1), (STORE, 0), (RESIDUAL, 0), (GATE_UP, 0)])
+@pytest.mark.parametrize("fmt", [Q4_0, Q8_0, Q4_K, Q6_K])
+def test_every_shape_has_a_form_that_fits_and_every_compiled_form_a_shape(lib, fmt, epi, xf32):
+    assert lib.gemv_wave_forms_unreached(fmt, epi, xf32, SMS) == 0
+    assert lib.gemv_wave_forms_unreached(fmt, epi, xf32, 74) >= 0  # a part of the chip: the rules scale with it

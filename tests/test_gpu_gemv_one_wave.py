@@ -1,7 +1,8 @@
-"""The matvec of one row at the edges of its one-wave form, for an fp32 vector (16-byte aligned and not) and a packed one.
+"""The matvec of one row over tiles per SM and chunks, for an fp32 vector (16-byte aligned and not) and a packed one.
 
-Each size is the first row count whose tiles need `tiles` to an SM, with a ragged last tile, so every compiled number of
-tiles per CTA runs with most of its CTAs partly or wholly empty, beside the forms on the other side of each line.
+Each size is the first row count whose tiles need `tiles` to an SM, with a ragged last tile, so that for an fp32 vector every
+compiled number of tiles per CTA runs with most of its CTAs partly or wholly empty.  A packed vector takes small blocks for many
+of these sizes; its one-wave forms are in test_gpu_gemv_wave_forms.py.
 """
 import numpy as np
 import pytest

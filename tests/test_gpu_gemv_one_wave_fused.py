@@ -1,6 +1,8 @@
-"""The one-wave form of the residual and the packed gate|up matvec: every number of row tiles per CTA that a chain can take.
+"""The residual and the packed gate|up matvec over row counts of 4..16 and 8..29 tiles per SM, two chunks to a row.
 
-The checks are those of the small forms (sums against the oracle, packed output against its own quantization step)."""
+The checks are those of the small forms (sums against the oracle, packed output against its own quantization step).  Which of
+these shapes take a one-wave form is the rules' choice; every such form over rows of any length is in
+test_gpu_gemv_wave_forms.py."""
 import pytest
 
 from test_gpu_parity import FORMATS, test_fused_residual_norm_chain as check_residual
