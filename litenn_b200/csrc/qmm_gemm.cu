@@ -249,6 +249,7 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
         SN = S;
         bool ok = true;
         int s = 0;
+        static_assert(GEMM_A_STAGES == 4, "a chunk's four K steps fill the stages");
         for (int c = c0; c < c1 && ok; ++c) {
             const bool more = c + 1 < c1;
             const uint8_t* next = wt + tile_stride;
@@ -267,8 +268,8 @@ __global__ void __launch_bounds__((8 * NB + 2) * 32, 3 - NB)
                         load_quarter<FMT>(P, next, q, lane);
                     }
                     const int as = s % GEMM_A_STAGES;
-                    if (s == GEMM_A_STAGES) {
-                        g_pdl_wait();
+                    if (q == 0 && c == c0 + 1) {  // s == GEMM_A_STAGES: stages are reused from here on
+                        g_pdl_wait_only();
                     }
                     if (s >= GEMM_A_STAGES && !g_mbar_wait_warp(&empty_a[as], (uint32_t)(s / GEMM_A_STAGES - 1) & 1u)) {
                         if (lane == 0) {

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     dequant_quarter<FMT>(P, S, q, r);
                     const int slot = s % GEMM_STAGES;
                     if (s == GEMM_STAGES) {
-                        g_pdl_wait();
+                        g_pdl_wait_only();
                     }
                     if (ok && s >= GEMM_STAGES) {
                         // lane 0 probes, the others wait for it at the warp barrier
