@@ -256,7 +256,7 @@ def run_reference(args):
 
 
 def gemv_micro(torch, capi, local, side, stream, steps, warmup):
-    """The Q4_0 FFN GEMV at batch 1 over 12 weight copies, in us per call: the public call (pack + matvec),
+    """The Q4_0 FFN GEMV at batch 1 over 12 weight copies, in us per call: the public call (one launch that packs and multiplies),
     the matvec kernel alone back to back (consecutive launches overlap through programmatic dependent
     launch), and the matvec kernel isolated (an ordinary one-element fill kernel between launches
     serializes them; its own time is measured separately and subtracted)."""
@@ -548,7 +548,7 @@ def run_ours(args):
             "gemv": {"metric": "Q4_0 GEMV achieved HBM GB/s", "workload": "q4_0_gemv_4096x11008_b1",
                      "value": ALGO_BYTES / (full_us * 1e-6) / 1e9, "unit": "GB/s", "us_per_call": full_us,
                      "copies": COPIES, "algorithmic_bytes": ALGO_BYTES,
-                     "note": "public call qmm_gemv_f32 = pack_x + gemv, one CUDA graph of 12 calls"},
+                     "note": "public call qmm_gemv_f32 (packs and multiplies in one launch), one CUDA graph of 12 calls"},
             "batch16": {"workload": "llama7b_q4_0_decode_b16", **b16},
             "gemm": {"workload": "prefill_gemm_m512_k4096_n14336", "q4_k_us": gm["q4_k"]["us"], "q6_k_us": gm["q6_k"]["us"],
                      "q4_k_tflops": gm["q4_k"]["tflops"], "q6_k_tflops": gm["q6_k"]["tflops"],
